@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(192) dense_tc5_kernel(const GemmParams p) {
   const uint32_t tmem = s_tmem;
 
   if (warp == 4) {
-    if (lane == 0) {   // ---- copies ----
+    if (elect_one()) {   // ---- copies ----
       const unsigned char* wsrc = p.w + (size_t)batch * p.w_batch + ((size_t)blockIdx.y * p.kb + kb0) * kTileBytes;
       const unsigned char* xsrc = p.x + (size_t)batch * p.x_batch + (size_t)kb0 * ((size_t)p.mp * 128) + (size_t)row0 * 128;
       const int pre = nkb < STAGES ? nkb : STAGES;
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(192) dense_tc5_kernel(const GemmParams p) {
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {   // ---- MMA issue ----
+    if (elect_one()) {   // ---- MMA issue ----
       // fp32 accumulator, bf16 x bf16, both K-major, N = BN, M = 128
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
       for (int i = 0; i < nkb; ++i) {

@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_tc5_kernel(const FlashArgs 
       asm volatile("cp.async.wait_all;" ::: "memory");
     }
   } else if (warp == 8) {
-    if (lane == 0) {   // ---- MMA issue ----
+    if (elect_one()) {   // ---- MMA issue ----
       constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kKeys >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(a.vpad >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
       const int ksteps = a.dpad >> 4;
