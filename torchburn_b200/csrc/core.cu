@@ -332,11 +332,15 @@ tb_status tb_fused_swiglu_mlp(tb_linear* gate, tb_linear* up, tb_linear* down, c
                 (long long)gate->n, (long long)gate->k, (long long)up->n, (long long)up->k, (long long)down->n, (long long)down->k);
   cudaStream_t st = as_stream(stream);
   const int64_t H = gate->k, I = gate->n, O = down->n;
-  float *d_x = nullptr, *d_h = nullptr, *d_o = nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  TB_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: fused_swiglu_mlp: not while the stream is being captured");
+  WorkspaceLease h;   // the activations between the projections
+  TB_TRY(h.take(st, sizeof(float) * m * I, kWorkspacePlain));
+  float *d_x = nullptr, *d_o = nullptr, *d_h = static_cast<float*>(h.ptr());
   tb_status s = TB_OK;
-  auto cleanup = [&]() { if (io_space == TB_HOST) { cudaFree(d_x); cudaFree(d_o); } cudaFree(d_h); };
-  cudaError_t e = cudaMalloc(&d_h, sizeof(float) * m * I);
-  if (e != cudaSuccess) return fail(TB_ERR_OOM, "fused_swiglu_mlp: %s", cudaGetErrorString(e));
+  cudaError_t e = cudaSuccess;
+  auto cleanup = [&]() { if (io_space == TB_HOST) { cudaFree(d_x); cudaFree(d_o); } };
   if (io_space == TB_HOST) {
     if (cudaMalloc(&d_x, sizeof(float) * m * H) != cudaSuccess || cudaMalloc(&d_o, sizeof(float) * m * O) != cudaSuccess) {
       cleanup();
@@ -350,7 +354,8 @@ tb_status tb_fused_swiglu_mlp(tb_linear* gate, tb_linear* up, tb_linear* down, c
   }
   s = tb_swiglu_gemv_w4a32(d_x, gate->qweight, gate->scales, gate->bias, up->qweight, up->scales, up->bias, d_h, m, I, H, gate->g, stream);
   if (s == TB_OK) s = tb_gemm_w4a32_grouped(d_h, down->qweight, down->scales, down->bias, d_o, m, O, I, down->g, stream);
-  if (s == TB_OK && io_space == TB_HOST) {
+  if (io_space != TB_HOST) return s;   // like every product on device buffers: in the order of the stream
+  if (s == TB_OK) {
     e = cudaMemcpyAsync(out, d_o, sizeof(float) * m * O, cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) s = fail(TB_ERR_CUDA, "fused_swiglu_mlp: %s", cudaGetErrorString(e));
   }

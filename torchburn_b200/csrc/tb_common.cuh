@@ -100,8 +100,25 @@ struct GemvArgs {
 tb_status launch_w4_gemv(const GemvArgs& a, cudaStream_t stream);
 // Kernels that call starts (1, or 2 with the activation pre-pass of the tensor-core kernels).
 int w4_gemv_launches(const GemvArgs& a);
-// Frees the per-stream workspaces that calls with several activation rows and no workspace of their own keep.
-void release_workspaces();
+// Device memory borrowed for the duration of one call's enqueueing and kept between calls (workspace.cu).  Blocks of
+// kind kWorkspaceTickets start with zeroed tickets that every launch leaves zero.
+constexpr int kWorkspaceTickets = 0, kWorkspacePlain = 1;
+constexpr size_t kWorkspaceTicketBytes = 4096;
+class WorkspaceLease {
+ public:
+  WorkspaceLease() = default;
+  WorkspaceLease(const WorkspaceLease&) = delete;
+  WorkspaceLease& operator=(const WorkspaceLease&) = delete;
+  ~WorkspaceLease();
+  tb_status take(cudaStream_t stream, size_t bytes, int kind);
+  void* ptr() const { return ptr_; }
+
+ private:
+  cudaStream_t stream_ = nullptr;
+  void* ptr_ = nullptr;
+  bool own_ = false;   // stream-ordered memory of this call alone
+};
+void release_workspaces();   // gives back every block that no call holds
 // Tuning hook: xmode 0 = fp32 products (M = 1 only), 1 = integer products; rows_per_warp /
 // warps force the launch shape of the M = 1 kernels (0 = automatic).
 void set_gemv_tuning(int xmode, int rows_per_warp, int warps);
@@ -112,6 +129,7 @@ tb_status launch_w4_mma(const GemvArgs& a, void* scratch, cudaStream_t stream);
 // tcgen05 kernel for 16 < M (w4_tc5.cu); its operand images live behind the first 4096 bytes of the same scratch.
 size_t w4_tc5_scratch_bytes(int m, int64_t k);
 bool w4_tc5_supported(const GemvArgs& a);
+int w4_tc5_launches(int m);
 tb_status launch_w4_tc5(const GemvArgs& a, void* scratch, cudaStream_t stream);
 void set_tc5_enabled(int on);
 int tc5_fault_flag();

@@ -10,7 +10,6 @@ tb_status absent() { return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: this build
 
 tb_status launch_w4_gemv(const GemvArgs&, cudaStream_t) { return absent(); }
 int w4_gemv_launches(const GemvArgs&) { return 0; }
-void release_workspaces() {}
 void set_gemv_tuning(int, int, int) {}
 size_t w4_mma_scratch_bytes(int, int64_t) { return 0; }
 int tc5_fault_flag() { return 0; }

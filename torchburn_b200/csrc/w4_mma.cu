@@ -403,7 +403,7 @@ static size_t digit_bytes(int m, int64_t k) {
   return (((size_t)(k / 32) * mt * kTileWords * sizeof(uint32_t)) + 255) & ~(size_t)255;
 }
 size_t w4_mma_scratch_bytes(int m, int64_t k) {
-  const size_t own = digit_bytes(m, k) + kSplitPartBytes, tc5 = w4_tc5_scratch_bytes(m, k);
+  const size_t own = digit_bytes(m < 64 ? m : 64, k) + kSplitPartBytes, tc5 = w4_tc5_scratch_bytes(m, k);
   return kSplitHeader + (own > tc5 ? own : tc5);
 }
 

@@ -1,251 +1,233 @@
-// Batched grouped-INT4 product for more than 16 activation rows on the 5th-generation tensor
-// cores (tcgen05): out[m, j] = sum_g scale[j, g] * sum_{k in g} x[m, k] * code(w[j, k])  (+ bias,
-// + residual, or the SwiGLU of a gate/up pair).  gemm_w4a32_grouped, src/quantization/gemv.rs:
-// 1690-1725; fused_swiglu_mlp_batched, src/quantization/fused_ops.rs:1267-1319.
+// Batched grouped-INT4 product on the 5th-generation tensor cores (tcgen05):
+// out[m, j] = sum_g scale[j, g] * sum_{k in g} x[m, k] * code(w[j, k])  (+ bias, + residual, or the SwiGLU of
+// a gate/up pair).  gemm_w4a32_grouped, src/quantization/gemv.rs:1690-1725; fused_swiglu_mlp_batched,
+// src/quantization/fused_ops.rs:1267-1319.
 //
-// The 4-bit codes are exact in bf16, so the weights enter the tensor core as they are and the
-// scale is applied OUTSIDE it, once per group: every group of K gets a fresh fp32 accumulator
-// in tensor memory, which the epilogue warps read back, multiply by scale[row, group] and add
-// to their registers while the next groups are being multiplied.  The fp32 activations are
-// split once per call (pre-pass, with the fused RMSNorm) into three bf16 pieces x1 + x2 + x3
-// (8 + 8 + 8 mantissa bits); the three products share one accumulator.  Products of a 4-bit
-// code and an 8-bit piece are exact and the tensor core adds them in fp32.
+// The 4-bit codes are exact in fp16, so the weights enter the tensor core as they are and the scale is applied
+// OUTSIDE it, once per group: every group of K gets a fresh fp32 accumulator in tensor memory, which the
+// epilogue warps read back, multiply by scale[row, group] and add to their registers while the next groups are
+// being multiplied.  The fp32 activations are split once per call (pre-pass, with the fused RMSNorm) into two
+// fp16 pieces after a power of two per row has brought the row's largest value to [2^14, 2^15): hi + lo carry
+// 23 bits of a value (fp32: 24), down to 2^-40 of the row's largest.  Products of a 4-bit code and a piece are
+// exact and the tensor core adds them in fp32, the small pieces first.  Two fp16 pieces are a third less
+// arithmetic than the three bf16 pieces that the same accuracy takes.
 //
-// The weights are the M = 128 side of the MMA (a CTA owns 128 weight rows), the activation
-// rows its N = 16..64.  A weight row lives in one LANE of tensor memory: the thread that
-// dequantises row r writes its codes with tcgen05.st straight from registers (A operand from
-// tensor memory), so the weights pass through shared memory only as packed nibbles (the per-thread
-// copy ring), never in operand form.  The activation pieces
-// arrive as ready-made 128-byte-swizzled K-major images by bulk copy.
+// The weights are the M = 128 side of the MMA, the activation rows its N.  A CTA works on NW tiles of 128 weight
+// rows (the gate and the up rows of a pair, or 256 consecutive rows) times MP activation rows; two weight tiles
+// share every activation image, which halves the L2 traffic of the images (2 * MP * 128 bytes per 64 elements of
+// K and SM: the bound at one tile per CTA and long prompts).  A weight row lives in one LANE of tensor memory:
+// the thread that unpacks row r writes its codes with tcgen05.st straight from registers (A operand from tensor
+// memory), so the weights pass through shared memory only as packed nibbles.
 //
-//   unpacking    4 or 8 warps, 128 threads per team (thread = weight row; two teams take every other
-//                stage): the nibbles of the thread's row stream into the thread's own shared-memory
-//                ring with cp.async, eight 64-element chunks ahead; the thread unpacks a chunk into
-//                its stage of tensor memory
-//   epilogue     8 warps: two teams of 128 threads (thread = weight row, a team = half of the activation
-//                rows): per group tcgen05.ld of the accumulator, acc += scale * sum; at the
-//                end bias / residual / SwiGLU and the stores (atomic adds when K is split)
-//   issue        4 warps, one lane each issues MMAs: issuing a tcgen05.mma costs its thread about 50 cycles
-//                whatever its size (measured), six times the arithmetic of a 128 x 16 x 16 MMA, but
-//                several warps issue side by side.  With four accumulator slots issuer i owns slot i and
-//                takes every group of K whose number is i modulo 4; with two slots (a pair at 48 or 64
-//                rows) issuer i owns slot i & 1 and matrix i >> 1.  An issuer commits its MMAs to the
-//                "group done" and "stage free" barriers.  The first of them also allocates tensor memory.
-// The bulk copies of the activation images are issued by the first thread of an unpacking team.
+//   unpacking    4 or 8 warps (thread = weight row) turn the nibbles in the ring into codes in tensor memory
+//   epilogue     8 warps: two teams of 128 threads (thread = weight row, all activation rows) that take every
+//                other VISIT: the accumulators of up to four groups, 128 columns of tensor memory, handed over
+//                at once.  The fixed cost of a hand-over (commit, barrier, tcgen05.ld latency: ~400 cycles) was what
+//                bounded one hand-over per group and both teams at every one of them.
+//   issue        3 warps, one lane each: issuer i owns accumulator slot i and takes visit i, i + 3, ..., so that one
+//                waits for its operands or its slot while another issues
+//   copies       1 warp, one lane: TMA boxes of 128 weight rows x 64 bytes (128 elements of K) and of their scales,
+//                bulk copies of the activation images, each into a ring.  (Copied by the rows' own threads with
+//                cp.async, every 16 bytes of a warp's 32 rows are 32 different lines: the shared-memory pipe was
+//                busy with them half of the time and every read of the ring waited ~500 cycles behind them.)
 //
-// Every wait is bounded.  No cluster features, no multicast.
-#include <cuda_bf16.h>
+// CTAs are persistent: every role walks the CTA's list of tiles by itself, so a tile's prologue and epilogue lie
+// under its neighbours' streaming.  Every wait is bounded.  No cluster features, no multicast.
+#include <cuda_fp16.h>
 
 #include "tb_common.cuh"
 #include "tc5.cuh"
+#include "tma_map.cuh"
 
 namespace tb {
 
 namespace {
 
-constexpr int kTileN = 128;     // weight rows per CTA (the MMA's M)
-constexpr int kKC = 64;         // K elements per stage: one 128-byte row of bf16
-constexpr int kMaxStages = 8;    // one matrix: 8 stages, a pair: 4 (tensor memory: 32 columns of codes per stage and matrix)
-constexpr int kPieces = 3;      // bf16 pieces of an activation
-constexpr int kAhead = 8;       // chunks of nibbles in flight per weight row
+constexpr int kTileN = 128;     // weight rows per MMA (its M)
+constexpr int kKC = 64;         // K elements per stage: one 128-byte row of fp16
+constexpr int kUnit = 128;      // K elements per copy of a weight tile: 64 bytes of nibbles a row
+constexpr int kUnitBytes = kTileN * 64;
+constexpr int kUnitScaleBytes = kTileN * 16;   // 32-element groups: four scales a row
+constexpr int kPieces = 2;      // fp16 pieces of an activation
 constexpr int kTmemCols = 512;
-constexpr int kMinRows = 17;     // up to 16 activation rows the integer mma.sync kernel is as fast or faster (measured)
+constexpr int kSlots = 3;       // accumulator slots of 128 columns; the first 128 columns hold the codes
+// Barriers of the stage rings, by chunk of K.  More of them than stages: a role that runs ahead (three issuers, two unpacking
+// teams) may wait for a chunk while one up to ten chunks older is still open, and a wait on a barrier two phases ahead
+// would pass at once.
+constexpr uint32_t kRing = 16;
+constexpr int kMaxRows = 512;   // activation rows per launch (bounds the workspace)
+constexpr int kMinRows = 9;      // up to 8 activation rows the integer mma.sync kernel is as fast (gate/up pair of 4096 x 14336: 45 against 46 us; at 16 rows 65 against 46)
 
 __device__ int g_tc5_fault = 0;
 
 struct Tc5Params {
-  const uint8_t* w[2];
+  CUtensorMap w[2];          // [n, k / 2] bytes, boxes of 64 x 128 rows
+  CUtensorMap s[2];          // 32-element groups: [n, ng] scales, boxes of 4 x 128 rows
   const float* scales[2];
   const float* bias[2];
   const float* resid;
   float* out;
-  const unsigned char* xq;   // per 64-element chunk of K: kPieces images of [mp rows x 128 B], swizzled
-  int m, mp;                 // activation rows, padded to a multiple of 16
-  int n, k, ng, g;
-  int ksplit, kper;          // CTAs that share a row tile, K elements of each
-  int pair;                  // gate/up pair with the SwiGLU epilogue
-  int slots;                 // accumulator slots in tensor memory
-  int stages;                // stage ring: 8 for one matrix, 4 for a pair
+  const unsigned char* xq;   // [activation tile][64-element chunk of K][piece][MP rows x 128 B], swizzled
+  const float* xinv;         // per activation row: the inverse of its power of two
+  int m;                     // activation rows
+  int n, k, ng;
+  int mtiles, ntiles, ksplit, kper;   // tiles of activation rows and of weight rows, CTAs that share a tile's K, K elements of each
+  int pair;                  // the second weight tile is the up matrix
 };
 
 using namespace tc5;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* s_abort) { return tc5::mbar_wait(bar, parity, s_abort, &g_tc5_fault); }
-__device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* s_abort) { return mbar_wait(bar, parity, s_abort); }
+// Inlined: a call would need registers by the calling convention, which a kernel with split registers cannot give.
 __device__ __forceinline__ bool mbar_wait_fast(uint64_t* bar, uint32_t parity, volatile int* s_abort) {
-  return mbar_ready(bar, parity) ? true : mbar_wait_slow(bar, parity, s_abort);
+  return mbar_ready(bar, parity) ? true : tc5::mbar_wait(bar, parity, s_abort, &g_tc5_fault);
 }
-// The same for a whole warp.  ONE lane polls: hundreds of threads polling the same barriers keep the
-// barrier unit so busy that the arrivals they are waiting for queue up behind their own polls.  The other
-// lanes take the answer (one answer for all lanes keeps warp-wide instructions converged) and the
-// ordering from the warp barrier.
+// The same for a whole converged warp: every lane asks, the warp votes, so that all lanes take the same way (also when
+// the wait is given up) without a branch of one lane in front of every warp-wide instruction.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* s_abort) {
-  bool ok = true;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait_fast(bar, parity, s_abort);
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-}
-
-// D (tensor memory, fp32) (+)= A (tensor memory, bf16) * B (shared memory, bf16)^T
-// b_lo: the lower word of B's shared-memory descriptor (see above); the upper word is the same for every tile.
-// ACC 0: overwrite the accumulator, 1: add to it, 2: decided at run time by `acc`.
-template <int ACC>
-__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t acc = 0) {
-  if (ACC == 2) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        ".reg .b64 bd;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t"
-        "}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(acc)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        ".reg .b64 bd;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t"
-        "}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "n"(ACC)
-        : "memory");
+  long long t0 = 0;
+  for (uint32_t i = 0;; ++i) {
+    if (__all_sync(0xffffffffu, mbar_ready(bar, parity))) return true;
+    if ((i & 127) == 127) {
+      const long long now = __shfl_sync(0xffffffffu, clock64(), 0);
+      if (t0 == 0) t0 = now;
+      const bool late = now - t0 > kWaitCycles;
+      if (late && (threadIdx.x & 31) == 0) {
+        *s_abort = 1;
+        atomicExch(&g_tc5_fault, 1);
+      }
+      if (late || __any_sync(0xffffffffu, *s_abort != 0)) return false;
+    }
   }
 }
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
+// One arrival for the warp, by its lane 0 and without a branch.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar, int lane) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lane) : "memory");
 }
 
-// 8 nibbles -> four bf16 pairs holding the codes (nibble - 8) of elements (0,4) (1,5) (2,6) (3,7):
-// 0x4300 | nibble is the bf16 number 128 + nibble, and 136 is subtracted exactly.  The activation
+// D (tensor memory, fp32) (+)= A (tensor memory, fp16) * B (shared memory, fp16)^T
+// b_lo: the lower word of B's shared-memory descriptor; the upper word is the same for every tile.
+template <int ACC>
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 bd;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 bd, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "n"(ACC)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
+      "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Two fp32 fused multiply-adds in one issue slot: a += x * s.
+__device__ __forceinline__ void fma2(float& a0, float& a1, uint32_t x0, uint32_t x1, float s) {
+  asm("{\n\t.reg .b64 a, x, s;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 x, {%2, %3};\n\tmov.b64 s, {%4, %4};\n\t"
+      "fma.rn.f32x2 a, x, s, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(a0), "+f"(a1)
+      : "r"(x0), "r"(x1), "f"(s));
+}
+
+// 8 nibbles -> four fp16 pairs holding the codes (nibble - 8) of elements (0,4) (1,5) (2,6) (3,7): 0x6400 | n is
+// the fp16 number 1024 + n and 0x6400 | 16 n is 1024 + 16 n; both become n - 8 exactly.  The activation
 // images use the same order of K inside every 8 elements.
 __device__ __forceinline__ void unpack8(uint32_t word, uint32_t* out4) {
-  const __nv_bfloat162 off = __floats2bfloat162_rn(136.f, 136.f);
+  const uint32_t o1 = 0x64086408u, s16 = 0x2C002C00u, o16 = 0xD480D480u;   // 1032, 1/16, -72
+  const uint32_t up = word >> 8;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t v = ((word >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
-    __nv_bfloat162 b = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&v), off);
-    out4[i] = *reinterpret_cast<uint32_t*>(&b);
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t src = i ? up : word;
+    uint32_t a = (src & 0x000F000Fu) | 0x64006400u, b = (src & 0x00F000F0u) | 0x64006400u;
+    const __half2 va = __hsub2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<const __half2*>(&o1));
+    const __half2 vb = __hfma2(*reinterpret_cast<__half2*>(&b), *reinterpret_cast<const __half2*>(&s16), *reinterpret_cast<const __half2*>(&o16));
+    out4[2 * i] = *reinterpret_cast<const uint32_t*>(&va);
+    out4[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&vb);
   }
 }
 
-struct IssueCtx {
-  uint64_t *full_a, *full_b, *empty, *acc_full, *acc_empty, *drained;   // drained: one per issuer
-  volatile int* s_abort;
-  uint32_t tmem, a_cols, acc_base, acc_cols, b_lo0, stage16, piece16, mp, idesc;
-  int nchunks, slots, nw, stages, qsplit;
+constexpr int floor_pow2(int v) { return v >= 4 ? 4 : (v >= 2 ? 2 : 1); }
+
+// Everything that follows from the template parameters.
+template <int MP, int NW, int G>
+struct Shape {
+  static constexpr int kCols = MP * NW;                    // accumulator columns of one group
+  static constexpr int kFit = floor_pow2(128 / kCols);
+  static constexpr int kGps = kFit < kUnit / G ? kFit : kUnit / G;   // groups per visit
+  static constexpr int kVk = kGps * G;                     // K elements per visit: 32, 64 or 128
+  static constexpr int kSteps = kVk / 16;                  // K16 steps per visit
+  static constexpr int kVisitsPerStage = kVk >= kKC ? 1 : kKC / kVk;
+  static constexpr int kDW = kCols <= 96 ? 8 : 4;          // unpacking warps
+  static constexpr int kThreads = (kDW + 12) * 32;
+  // registers: (kDW + 4) warps give back to the 8 epilogue warps; the sum stays at what the block was launched with
+  static constexpr int kRegsLaunch = kDW == 8 ? 96 : 128, kRegsFew = kDW == 8 ? 64 : 56, kRegsMany = kDW == 8 ? 144 : 200;
+  static_assert((kDW + 4) * kRegsFew + 8 * kRegsMany <= (kDW + 12) * kRegsLaunch, "register split");
+  static constexpr int kStagesA = 128 / (32 * NW);
+  static constexpr int kStagesB = MP <= 16 ? 16 : (MP <= 32 ? 12 : (MP <= 48 ? 8 : 6));
+  static constexpr int kUnits = NW == 2 ? (MP <= 48 ? 4 : 3) : 8;   // ring of weight units: 64 KB, 48 KB in the largest shape
+  static constexpr int kScales = G != 32 ? 8 : (kCols <= 64 ? 8 : 4);   // units (32-element groups) or visits of scales in flight
+  static constexpr int kBBytes = kPieces * MP * 128;       // the activation images of a stage
+  static constexpr int kScaleBytes = NW * kGps * 4;        // of one visit and row
+  static constexpr size_t kOffNib = (size_t)kStagesB * kBBytes;
+  static constexpr size_t kOffScale = kOffNib + (size_t)kUnits * NW * kUnitBytes;
+  static constexpr size_t kOffEx = kOffScale + (size_t)kScales * (G == 32 ? NW * kUnitScaleBytes : 256 * kScaleBytes);
+  static constexpr size_t kSmem = kOffEx + (size_t)kCols * 128 * 4 + 1024;
+  static_assert(kSmem <= 226 * 1024, "shared memory");
 };
 
-// One MMA-issuing thread.  With four accumulator slots issuer i owns slot i and takes the groups of K whose
-// number is i modulo 4, both matrices of a pair.  With two slots (a pair at 48 or 64 activation rows) four
-// issuers still work: issuer i owns slot i & 1 and only matrix i >> 1 (QSPLIT); the slot's "group done" barrier
-// then counts two commits.  SPG (K16 steps per group: 2, 4 or 8) is a template parameter so that the unrolled
-// body knows at compile time where a group starts and ends; descriptors are a constant upper word and a lower
-// word that only takes additions.  An issuer skips the stages that hold none of its groups; a stage's "free"
-// barrier counts the issuers that do work in it.
-template <int SPG, int NW, bool QSPLIT>
-__device__ __forceinline__ void issue_loop(const IssueCtx& x, const uint32_t me) {
-  const uint32_t nslots = (uint32_t)x.slots;
-  const uint32_t my_slot = QSPLIT ? (me & 1u) : me;
-  const int q0 = QSPLIT ? (int)(me >> 1) : 0, q1 = QSPLIT ? q0 + 1 : NW;
-  const uint32_t d_base = x.tmem + x.acc_base + my_slot * x.acc_cols;
-  uint64_t* my_full = &x.acc_full[my_slot];
-  uint64_t* my_empty = &x.acc_empty[my_slot];
-  const uint32_t stage_mask = (uint32_t)x.stages - 1, stage_shift = x.stages == 8 ? 3u : 2u;
-  uint32_t visits = 0;   // groups this issuer has started
-  bool ok = true;
-  for (int c = 0; c < x.nchunks && ok; ++c) {
-    {  // first and last group of this stage: is one of them mine?
-      const uint32_t g0 = ((uint32_t)c * (kKC / 16)) / SPG, g1 = ((uint32_t)c * (kKC / 16) + 3) / SPG;
-      if ((g0 & (nslots - 1)) != my_slot && (g1 & (nslots - 1)) != my_slot) continue;
-    }
-    const uint32_t s = (uint32_t)c & stage_mask, par = ((uint32_t)c >> stage_shift) & 1u;
-    ok = mbar_wait_fast(&x.full_a[s], par, x.s_abort) && mbar_wait_fast(&x.full_b[s], par, x.s_abort);
-    if (!ok) break;
-    tc_fence_after();
-    const uint32_t b_lo = x.b_lo0 + s * x.stage16;
-    const uint32_t a_base = x.tmem + s * x.a_cols;
-#pragma unroll
-    for (int ks = 0; ks < kKC / 16; ++ks) {   // 16 bf16 = 32 bytes of a row = 8 columns of tensor memory per MMA
-      const uint32_t t = (uint32_t)c * (kKC / 16) + ks;            // K16 step of this CTA
-      const uint32_t gi = SPG == 2 ? t >> 1 : (SPG == 4 ? t >> 2 : t >> 3);
-      if ((gi & (nslots - 1)) != my_slot) continue;
-      // SPG 2: groups start at ks 0 and 2; SPG 4: at ks 0; SPG 8: at ks 0 of every other chunk
-      const bool starts = SPG == 2 ? (ks % 2 == 0) : (SPG == 4 ? ks == 0 : (ks == 0 && (c & 1) == 0));
-      const bool ends = SPG == 2 ? (ks % 2 == 1) : (SPG == 4 ? ks == 3 : (ks == 3 && (c & 1) == 1));
-      if (starts) {
-        if (visits > 0) {          // the epilogue must have read this slot's previous sums
-          ok = mbar_wait_fast(my_empty, (visits - 1u) & 1u, x.s_abort);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        ++visits;
-      }
-#pragma unroll
-      for (int pc = 0; pc < kPieces; ++pc)
-#pragma unroll
-        for (int q = 0; q < NW; ++q) {
-          if (q < q0 || q >= q1) continue;
-          const uint32_t d = d_base + (uint32_t)q * x.mp, a = a_base + (uint32_t)(q * 32 + ks * 8);
-          const uint32_t b = b_lo + (uint32_t)(ks * 2) + (uint32_t)pc * x.piece16;
-          if (pc > 0) mma_bf16_ts<1>(d, a, b, x.idesc);
-          else if (SPG == 8 && ks == 0) mma_bf16_ts<2>(d, a, b, x.idesc, (uint32_t)(c & 1));
-          else if ((SPG == 2 && ks % 2 == 0) || (SPG == 4 && ks == 0)) mma_bf16_ts<0>(d, a, b, x.idesc);
-          else mma_bf16_ts<1>(d, a, b, x.idesc);
-        }
-      if (ends) mma_commit(my_full);
-    }
-    mma_commit(&x.empty[s]);   // the stage is free once every issuer's MMAs have read it
-  }
-  // nothing may still be running on the tensor core when the tensor memory is given back
-  mma_commit(&x.drained[me]);
-  mbar_wait_fast(&x.drained[me], 0u, x.s_abort);
-}
+__device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-// MP: activation rows padded to a multiple of 16; NW: 1 matrix or a gate/up pair.  Template parameters keep
-// each variant's loops exactly as long as they need to be (the roles' loop bodies must stay in the
-// instruction cache) and its accumulator registers as few.
-// DW: unpacking warps, 4 or 8 (two teams that take every other stage; 20 warps leave 96 registers per thread, which
-// the single-matrix variants fit).
-template <int MP, int NW, int DW>
-__global__ void __launch_bounds__((DW + 12) * 32, 1) w4_tc5_kernel(const Tc5Params p) {
+template <int MP, int NW, int G>
+__global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(const __grid_constant__ Tc5Params p) {
+  using S = Shape<MP, NW, G>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t full_a[kMaxStages], full_b[kMaxStages], empty[kMaxStages], acc_full[4], acc_empty[4], drained[4];
+  __shared__ __align__(8) uint64_t full_a[kRing], full_b[kRing], done[kRing], full_w[8], empty_w[8], full_s[8], empty_s[8], acc_full[2 * kSlots], acc_empty[kSlots], drained[kSlots];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int b_bytes = kPieces * MP * 128;             // the images of the activations per stage
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int n0 = (int)blockIdx.x * kTileN;
-  const int k0 = (int)blockIdx.y * p.kper;
-  const int nchunks = p.kper / kKC;
-  const int ngroups = p.kper / p.g;
-  const int slots = p.slots;
-  constexpr int kStages = NW == 1 ? 8 : 4;
-  const bool qsplit = NW == 2 && slots == 2;   // two slots: the four issuers split by matrix as well
-  // tensor memory columns: [stage][matrix] 32 columns of codes (64 bf16), then [slot][matrix] mp columns of sums
-  const uint32_t a_cols = 32u * NW, acc_base = kStages * a_cols, acc_cols = (uint32_t)(MP * NW);
+  const int total = p.mtiles * p.ksplit * p.ntiles;
+  const int my_tiles = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int nstages = p.kper / kKC, nunits = p.kper / kUnit, nvisits = p.kper / S::kVk;   // of one tile
+  constexpr uint32_t SA = S::kStagesA, SB = S::kStagesB;
 
   if (tid == 0) {
     s_abort = 0;
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&full_a[s], 4);    // one lane of each unpacking warp
+    for (uint32_t s = 0; s < kRing; ++s) {
+      mbar_init(&full_a[s], NW == 2 && S::kDW == 8 ? 8 : 4);   // one lane of each unpacking warp of the stage
       mbar_init(&full_b[s], 1);
-      mbar_init(&empty[s], (p.g == 32 ? 2u : 1u) * (qsplit ? 2u : 1u));   // the issuers of the stage's groups commit to it
+      mbar_init(&done[s], S::kVisitsPerStage);   // the MMAs that read the stage have finished: one commit per visit
     }
-    for (int s = 0; s < 4; ++s) {
-      mbar_init(&acc_full[s], qsplit ? 2u : 1u);
-      mbar_init(&acc_empty[s], 8);  // one lane of each epilogue warp
+    for (int s = 0; s < S::kUnits; ++s) {
+      mbar_init(&full_w[s], 1);
+      mbar_init(&empty_w[s], NW == 2 && S::kDW == 8 ? 8 : 4);   // one lane of each warp that reads the unit
     }
-    for (int s = 0; s < 4; ++s) mbar_init(&drained[s], 1);
+    for (int s = 0; s < S::kScales; ++s) {
+      mbar_init(&full_s[s], 1);
+      mbar_init(&empty_s[s], S::kGps == 4 ? 4 : 8);             // one team reads a unit's scales, or both
+    }
+    for (int s = 0; s < kSlots; ++s) {
+      mbar_init(&acc_empty[s], 4);   // one lane of each warp of the team that read it
+      mbar_init(&drained[s], 1);
+    }
+    // by visit modulo 6: the visits of one barrier belong to one team, which has waited for the one before
+    for (int s = 0; s < 2 * kSlots; ++s) mbar_init(&acc_full[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  constexpr int kIssue0 = DW + 8;   // first issuing warp
+  constexpr int kIssue0 = S::kDW + 8;   // first issuing warp
   if (warp == kIssue0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -256,228 +238,311 @@ __global__ void __launch_bounds__((DW + 12) * 32, 1) w4_tc5_kernel(const Tc5Para
   const uint32_t tmem = s_tmem;
 
   if (warp >= kIssue0) {
-    // ---------------- MMA issue ----------------
-    if (lane == 0 && (warp - kIssue0 < slots || qsplit)) {
-      IssueCtx x;
-      x.full_a = full_a; x.full_b = full_b; x.empty = empty; x.acc_full = acc_full; x.acc_empty = acc_empty; x.drained = drained;
-      x.s_abort = &s_abort;
-      x.tmem = tmem; x.a_cols = a_cols; x.acc_base = acc_base; x.acc_cols = acc_cols;
-      x.b_lo0 = (smem_u32(smem) >> 4) | (1u << 16);
-      x.stage16 = (uint32_t)b_bytes >> 4;
-      x.piece16 = (uint32_t)(MP * 128) >> 4;
-      x.mp = (uint32_t)MP;
-      // instruction descriptor: fp32 accumulator, bf16 x bf16, B K-major, N = mp, M = 128
-      x.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MP >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
-      x.nchunks = nchunks; x.slots = slots; x.nw = NW; x.stages = kStages; x.qsplit = qsplit ? 1 : 0;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kRegsFew));
+    const bool one = elect_one();
+    if (one && warp - kIssue0 < kSlots) {
+      // ---------------- MMA issue ----------------
       const uint32_t me = (uint32_t)(warp - kIssue0);
-      if (NW == 2 && qsplit) {
-        if (p.g == 32) issue_loop<2, NW, NW == 2>(x, me);
-        else if (p.g == 64) issue_loop<4, NW, NW == 2>(x, me);
-        else issue_loop<8, NW, NW == 2>(x, me);
-      } else {
-        if (p.g == 32) issue_loop<2, NW, false>(x, me);
-        else if (p.g == 64) issue_loop<4, NW, false>(x, me);
-        else issue_loop<8, NW, false>(x, me);
-      }
-    }
-  } else if (warp < DW) {
-    // ---------------- unpacking: thread = weight row; with 8 warps two teams take every other stage ----------------
-    constexpr int TS = DW / 4;                 // teams
-    constexpr int PD = kAhead / TS - 1;        // own chunks in flight
-    const int team = warp >> 2, row = tid & 127;
-    const int j = n0 + row;
-    const bool live = j < p.n;
-    const size_t roff = (size_t)(live ? j : 0) * (size_t)(p.k >> 1) + (size_t)(k0 >> 1);
-    const uint8_t* w0 = p.w[0] + roff;
-    const uint8_t* w1 = (NW == 2 ? p.w[1] : p.w[0]) + roff;
-    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    // the thread's ring: [slot][matrix][row][32 bytes], the two 16-byte halves swapped for rows 4..7 of
-    // every 8 so that a quarter warp touches every bank once
-    const uint32_t ring = smem_u32(smem + (size_t)kStages * b_bytes);
-    const uint32_t flip = (uint32_t)((row >> 2) & 1) * 16u;
-    auto slot_addr = [&](int c, int q) { return ring + (uint32_t)(((c % kAhead) * NW + q) * kTileN + row) * 32u; };
-    auto fetch = [&](int c) {
-      if (live && c < nchunks) {
-        for (int q = 0; q < NW; ++q) {
-          const uint8_t* src = (q ? w1 : w0) + (size_t)c * 32;
-          const uint32_t dst = slot_addr(c, q);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + flip), "l"(src) : "memory");
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (flip ^ 16u)), "l"(src + 16) : "memory");
-        }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");   // one group per chunk, empty ones included
-    };
-    for (int i = 0; i < PD; ++i) fetch(team + i * TS);
-    for (int c = team; c < nchunks; c += TS) {
-      fetch(c + PD * TS);
-      asm volatile("cp.async.wait_group %0;" ::"n"(PD) : "memory");   // chunk c has landed
-      const int s = c % kStages;
-      if (c >= kStages && !mbar_wait_warp(&empty[s], (uint32_t)(c / kStages - 1) & 1u, &s_abort)) break;
-      if (row == 0) {   // the stage's activation images: one bulk copy
-        mbar_expect_tx(&full_b[s], (uint32_t)b_bytes);
-        bulk_g2s(smem + (size_t)s * b_bytes, p.xq + (size_t)(k0 / kKC + c) * b_bytes, (uint32_t)b_bytes, &full_b[s]);
-      }
-      tc_fence_after();
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        if (q < NW) {
-          const uint32_t src = slot_addr(c, q);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {   // 32 elements = 16 columns per 16 bytes of nibbles
-            uint32_t wd[4] = {0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u};  // code 0 for rows past n
-            if (live)
-              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wd[0]), "=r"(wd[1]), "=r"(wd[2]), "=r"(wd[3]) : "r"(src + ((uint32_t)h * 16u ^ flip)));
-            uint32_t v[16];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) unpack8(wd[t], &v[4 * t]);
-            const uint32_t col = lane_base + (uint32_t)s * a_cols + (uint32_t)q * 32u + (uint32_t)h * 16u;
-            const uint32_t lo[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
-            const uint32_t hi[8] = {v[8], v[9], v[10], v[11], v[12], v[13], v[14], v[15]};
-            tmem_st8(col, lo);
-            tmem_st8(col + 8, hi);
-          }
-        }
-      }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full_a[s]);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-  } else {
-    // ---------------- per-group scaling and the epilogue: thread = weight row, team = half of the activation rows ----------------
-    const int team = (warp - DW) >> 2, row = tid & 127;
-    const int j = n0 + row;
-    const bool live = j < p.n;
-    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    constexpr int half = MP >> 1;               // 8, 16, 24 or 32 activation rows per team
-    constexpr int units = half >> 3;            // in blocks of 8 columns
-    const int cb = team * half;
-    const float* s0 = p.scales[0] + (size_t)(live ? j : 0) * p.ng + k0 / p.g;
-    const float* s1 = (NW == 2 ? p.scales[1] : p.scales[0]) + (size_t)(live ? j : 0) * p.ng + k0 / p.g;
-    float acc[NW][half];
-#pragma unroll
-    for (int q = 0; q < NW; ++q)
-#pragma unroll
-      for (int i = 0; i < half; ++i) acc[q][i] = 0.f;
-    bool ok = true;
-    // Four slots and 32-element groups: TWO groups (one 64-element stage) per visit - one wait for both slots, all
-    // their loads in flight at once (64 registers at most), one hand-back.  The fixed cost of a visit (barrier,
-    // tcgen05.ld latency, fences, arrival: ~400 cycles whatever the number of activation rows) is what bounds
-    // the kernel at few rows; the groups of a stage finish together anyway.
-    const bool two_per_visit = slots == 4 && p.g == 32;
-    if constexpr (units * NW <= 4) {
-      if (two_per_visit) {
-        float2 sa = live ? __ldg(reinterpret_cast<const float2*>(s0)) : make_float2(0.f, 0.f);
-        float2 sb = (live && NW == 2) ? __ldg(reinterpret_cast<const float2*>(s1)) : make_float2(0.f, 0.f);
-        for (int gi = 0; gi < ngroups && ok; gi += 2) {
-          const float2 ca = sa, cb2 = sb;
-          if (gi + 2 < ngroups) {
-            sa = live ? __ldg(reinterpret_cast<const float2*>(s0 + gi + 2)) : make_float2(0.f, 0.f);
-            if (NW == 2) sb = live ? __ldg(reinterpret_cast<const float2*>(s1 + gi + 2)) : make_float2(0.f, 0.f);
-          }
-          const int slot = gi & 3;   // 0 or 2: this visit takes slots slot and slot + 1
-          const uint32_t par = (uint32_t)(gi >> 2) & 1u;
-          ok = mbar_wait_warp(&acc_full[slot], par, &s_abort) && mbar_wait_warp(&acc_full[slot + 1], par, &s_abort);
+      // instruction descriptor: fp32 accumulator, fp16 x fp16, B K-major, N = MP, M = 128
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(MP >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
+      const uint32_t b_lo0 = (smem_u32(smem) >> 4) | (1u << 16);
+      const uint32_t d_base = tmem + 128u + me * 128u;
+      const uint32_t nv = (uint32_t)(my_tiles * nvisits);
+      bool ok = true;
+      uint32_t turn = 0;   // visits of this slot so far
+      for (uint32_t v = me; v < nv; v += kSlots, ++turn) {
+        if (turn > 0) {          // the epilogue must have read this slot's previous sums
+          ok = mbar_wait_fast(&acc_empty[me], (turn - 1u) & 1u, &s_abort);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t d = lane_base + acc_base + (uint32_t)slot * acc_cols + (uint32_t)cb;
-          uint32_t r[2][NW][units][8];
+        }
+        constexpr int kStagesPerVisit = S::kSteps > 4 ? 2 : 1;
+        constexpr int kStepsHere = S::kSteps > 4 ? 4 : S::kSteps;   // of one stage
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
+        for (int sv = 0; sv < kStagesPerVisit; ++sv) {
+          const uint32_t c = kStagesPerVisit == 2 ? 2 * v + sv : v / S::kVisitsPerStage;
+          const uint32_t ks0 = S::kVisitsPerStage == 2 ? (v & 1u) * 2u : 0u;
+          ok = mbar_wait_fast(&full_a[c % kRing], (c / kRing) & 1u, &s_abort) && mbar_wait_fast(&full_b[c % kRing], (c / kRing) & 1u, &s_abort);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t b_lo = b_lo0 + (c % SB) * (uint32_t)(S::kBBytes >> 4) + ks0 * 2u;
+          const uint32_t a_base = tmem + (c % SA) * (32u * NW) + ks0 * 8u;
+#pragma unroll
+          for (int ks = 0; ks < kStepsHere; ++ks) {   // 16 fp16 = 32 bytes of an image row = 8 columns of codes
+            constexpr int kStepsPerGroup = G / 16;
+            const int t = sv * 4 + ks, gi = t / kStepsPerGroup;    // K16 step and group of this visit
+#pragma unroll
+            for (int pc = kPieces - 1; pc >= 0; --pc)   // the small piece first
+#pragma unroll
+              for (int q = 0; q < NW; ++q) {
+                const uint32_t d = d_base + (uint32_t)(gi * S::kCols + q * MP), a = a_base + (uint32_t)(q * 32 + ks * 8);
+                const uint32_t b = b_lo + (uint32_t)(ks * 2) + (uint32_t)(pc * (MP * 128 >> 4));
+                if (t % kStepsPerGroup == 0 && pc == kPieces - 1) mma_f16_ts<0>(d, a, b, idesc);
+                else mma_f16_ts<1>(d, a, b, idesc);
+              }
+          }
+          if (sv == kStagesPerVisit - 1) mma_commit(&acc_full[v % (2 * kSlots)]);
+          mma_commit(&done[c % kRing]);
+        }
+        if (!ok) break;
+      }
+      // nothing may still be running on the tensor core when the tensor memory is given back
+      mma_commit(&drained[me]);
+      mbar_wait_fast(&drained[me], 0u, &s_abort);
+    } else if (one) {
+      // ---------------- copies ----------------
+      uint32_t c = 0, u = 0;
+      bool ok = true;
+      const int chunks = p.k / kKC;
+      const uint32_t w_at = smem_u32(smem + S::kOffNib), s_at = smem_u32(smem + S::kOffScale);
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        const int mt = t % p.mtiles, kz = (t / p.mtiles) % p.ksplit;
+        const int n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW);
+        const unsigned char* src = p.xq + ((size_t)mt * chunks + (size_t)kz * nstages) * S::kBBytes;
+        for (int i = 0; i < nunits && ok; ++i, ++u) {
+          const uint32_t ws = u % S::kUnits, ss = u % S::kScales;
+          if (u >= S::kUnits) ok = mbar_wait_fast(&empty_w[ws], (u / S::kUnits - 1u) & 1u, &s_abort);
+          if (!ok) break;
+          mbar_expect_tx(&full_w[ws], NW * kUnitBytes);
+#pragma unroll
+          for (int q = 0; q < NW; ++q)
+            tma_box(w_at + (ws * NW + q) * kUnitBytes, &p.w[p.pair ? q : 0], kz * (p.kper >> 1) + i * 64, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
+          if constexpr (G == 32) {
+            if (u >= S::kScales) ok = mbar_wait_fast(&empty_s[ss], (u / S::kScales - 1u) & 1u, &s_abort);
+            if (!ok) break;
+            mbar_expect_tx(&full_s[ss], NW * kUnitScaleBytes);
 #pragma unroll
             for (int q = 0; q < NW; ++q)
-#pragma unroll
-              for (int u = 0; u < units; ++u) tmem_ld8(d + (uint32_t)h * acc_cols + (uint32_t)(q * MP + u * 8), r[h][q][u]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) { mbar_arrive(&acc_empty[slot]); mbar_arrive(&acc_empty[slot + 1]); }
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int q = 0; q < NW; ++q) {
-              const float cq = q ? (h ? cb2.y : cb2.x) : (h ? ca.y : ca.x);
-#pragma unroll
-              for (int u = 0; u < units; ++u)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[q][u * 8 + i] = fmaf(cq, __uint_as_float(r[h][q][u][i]), acc[q][u * 8 + i]);
-            }
+              tma_box(s_at + (ss * NW + q) * kUnitScaleBytes, &p.s[p.pair ? q : 0], kz * (p.kper / G) + i * 4, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_s[ss]));
+          }
+          for (int h = 0; h < 2; ++h, ++c) {
+            if (c >= SB) ok = mbar_wait_fast(&done[(c - SB) % kRing], ((c - SB) / kRing) & 1u, &s_abort);
+            if (!ok) break;
+            mbar_expect_tx(&full_b[c % kRing], S::kBBytes);
+            bulk_g2s(smem + (size_t)(c % SB) * S::kBBytes, src + (size_t)(2 * i + h) * S::kBBytes, S::kBBytes, &full_b[c % kRing]);
+          }
         }
       }
-    }
-    float sc0 = live ? __ldg(s0) : 0.f, sc1 = (live && NW == 2) ? __ldg(s1) : 0.f;
-    for (int gi = 0; gi < ngroups && !(two_per_visit && units * NW <= 4); ++gi) {
-      const float c0 = sc0, c1 = sc1;
-      if (gi + 1 < ngroups) {
-        sc0 = live ? __ldg(s0 + gi + 1) : 0.f;
-        if (NW == 2) sc1 = live ? __ldg(s1 + gi + 1) : 0.f;
+      // copies in flight must have landed before the CTA gives its shared memory back (all have, unless a wait was given up)
+      if (!ok) {
+        int no_abort = 0;
+        for (uint32_t i = c > SB ? c - SB : 0; i < c; ++i) mbar_wait_fast(&full_b[i % kRing], (i / kRing) & 1u, &no_abort);
+        for (uint32_t i = u > S::kUnits ? u - S::kUnits : 0; i < u; ++i) mbar_wait_fast(&full_w[i % S::kUnits], (i / S::kUnits) & 1u, &no_abort);
+        if (G == 32)
+          for (uint32_t i = u > S::kScales ? u - S::kScales : 0; i < u; ++i) mbar_wait_fast(&full_s[i % S::kScales], (i / S::kScales) & 1u, &no_abort);
       }
-      const int slot = gi % slots;
-      ok = mbar_wait_warp(&acc_full[slot], (uint32_t)(gi / slots) & 1u, &s_abort);
+    }
+  } else if (warp < S::kDW) {
+    // ---------------- unpacking: thread = weight row ----------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kRegsFew));
+    // eight warps: a team per weight tile, or (one tile) teams that take every other unit of 128 elements
+    constexpr bool kTeamTile = S::kDW == 8 && NW == 2, kTeamUnit = S::kDW == 8 && NW == 1;
+    constexpr int kTiles = S::kDW == 4 ? NW : 1;       // weight tiles of one thread
+    const int team = warp >> 2, row = tid & 127;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    // the ring: [slot][tile][row][64 bytes]; the copy's swizzle rotates a row's 16-byte pieces so that a quarter warp
+    // touches every bank once
+    const uint32_t ring = smem_u32(smem + S::kOffNib) + (uint32_t)row * 64u;
+    const uint32_t swz = (uint32_t)((row >> 1) & 3);
+    uint32_t u = kTeamUnit ? (uint32_t)team : 0u;   // the CTA's units run through all its tiles
+    const uint32_t nu = (uint32_t)(my_tiles * nunits);
+    bool ok = true;
+    for (; u < nu && ok; u += kTeamUnit ? 2 : 1) {
+      const uint32_t ws = u % S::kUnits;
+      ok = mbar_wait_warp(&full_w[ws], (u / S::kUnits) & 1u, &s_abort);
       if (!ok) break;
-      tc_fence_after();
-      const uint32_t d = lane_base + acc_base + (uint32_t)slot * acc_cols + (uint32_t)cb;
-      if constexpr (units * NW <= 4) {
-        // every load of the group is in flight at once (32 registers at most)
-        uint32_t r[NW][units][8];
 #pragma unroll
-        for (int q = 0; q < NW; ++q)
+      for (uint32_t h = 0; h < 2; ++h) {
+        const uint32_t c = 2 * u + h;
+        const uint32_t a_col = lane_base + (c % SA) * (32u * NW);
 #pragma unroll
-          for (int u = 0; u < units; ++u) tmem_ld8(d + (uint32_t)(q * MP + u * 8), r[q][u]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int i = 0; i < kTiles; ++i) {
+          const int q = kTeamTile ? team : i;
+          const uint32_t src = ring + (ws * NW + (uint32_t)q) * kUnitBytes, col = a_col + (uint32_t)q * 32u;
+          uint32_t v[2][16];
+#pragma unroll
+          for (uint32_t e = 0; e < 2; ++e) {   // 32 elements = 16 columns per 16 bytes of nibbles
+            uint32_t wd[4];
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wd[0]), "=r"(wd[1]), "=r"(wd[2]), "=r"(wd[3]) : "r"(src + (((2 * h + e) ^ swz) * 16u)));
+#pragma unroll
+            for (int w = 0; w < 4; ++w) unpack8(wd[w], &v[e][4 * w]);
+          }
+          if (h == 1 && i == kTiles - 1) {   // the unit has been read
+            __syncwarp();
+            mbar_arrive_warp(&empty_w[ws], lane);
+          }
+          // the codes are ready in registers before the stage is free: from "free" to "full" it is only the store
+          if (i == 0) {
+            if (c >= SA) ok = mbar_wait_warp(&done[(c - SA) % kRing], ((c - SA) / kRing) & 1u, &s_abort);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          tmem_st16(col, v[0]);
+          tmem_st16(col + 16u, v[1]);
+        }
+        if (!ok) break;
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[slot]);   // the slot's sums are in registers: hand it back before the arithmetic
+        mbar_arrive_warp(&full_a[c % kRing], lane);
+      }
+    }
+  } else {
+    // ---------------- per-group scaling and the epilogue: thread = weight row, team = every other visit ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::kRegsMany));
+    const int team = (warp - S::kDW) >> 2, row = tid & 127;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const int et = tid - S::kDW * 32;
+    const uint32_t sring = smem_u32(smem + S::kOffScale) + (G == 32 ? (uint32_t)row * 16u : (uint32_t)et * S::kScaleBytes);
+    float* ex = reinterpret_cast<float*>(smem + S::kOffEx);
+    // 32-element groups: the scales lie in their ring, four a row and unit.  Larger groups: the rows' scales need not start on
+    // 16 bytes, so every thread copies its own with cp.async: tile, visit within it, ring slot
+    int ft = blockIdx.x, fv = team;
+    uint32_t fs = 0;
+    const float* fp[NW];
+    auto open_tile = [&](int t) {
+      const int n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW), kz = (t / p.mtiles) % p.ksplit;
 #pragma unroll
-        for (int q = 0; q < NW; ++q) {
-          const float cq = q ? c1 : c0;
+      for (int q = 0; q < NW; ++q) {
+        const int j = n0 + (p.pair ? 0 : q * kTileN) + row;
+        fp[q] = t < total && j < p.n ? (p.pair && q ? p.scales[1] : p.scales[0]) + (size_t)j * p.ng + (size_t)kz * (p.kper / G) : nullptr;
+      }
+    };
+    open_tile(ft);
+    auto fetch = [&]() {
+      while (ft < total && fv >= nvisits) {
+        fv -= nvisits;
+        ft += gridDim.x;
+        open_tile(ft);
+      }
+      if (ft < total) {
 #pragma unroll
-          for (int u = 0; u < units; ++u)
+        for (int q = 0; q < NW; ++q)
+          if (fp[q] != nullptr)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(sring + fs * (256u * S::kScaleBytes) + (uint32_t)(q * S::kGps * 4)),
+                         "l"(fp[q] + (size_t)fv * S::kGps), "n"(S::kGps * 4)
+                         : "memory");
+        fv += 2;
+      }
+      fs = fs + 1 == S::kScales ? 0 : fs + 1;
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if constexpr (G != 32)
+#pragma unroll 1
+      for (int i = 0; i < S::kScales - 1; ++i) fetch();
+    uint32_t v = (uint32_t)team, tile_end = 0, rs = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+      tile_end += (uint32_t)nvisits;
+      const int mt = t % p.mtiles, kz = (t / p.mtiles) % p.ksplit;
+      const int n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW);
+      float acc[S::kCols];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[q][u * 8 + i] = fmaf(cq, __uint_as_float(r[q][u][i]), acc[q][u * 8 + i]);
+      for (int i = 0; i < S::kCols; ++i) acc[i] = 0.f;
+      for (; v < tile_end && ok; v += 2) {
+        float sc[NW][S::kGps];
+        if constexpr (G == 32) {
+          constexpr uint32_t kPerUnit = 4 / S::kGps;   // visits per unit
+          const uint32_t un = v / kPerUnit, ss = un % S::kScales;
+          ok = mbar_wait_warp(&full_s[ss], (un / S::kScales) & 1u, &s_abort);
+          if (!ok) break;
+#pragma unroll
+          for (int q = 0; q < NW; ++q) {
+            const uint32_t a = sring + (ss * NW + (uint32_t)q) * kUnitScaleBytes + (v % kPerUnit) * (uint32_t)(S::kGps * 4);
+            if constexpr (S::kGps == 4)
+              asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(sc[q][0]), "=f"(sc[q][1]), "=f"(sc[q][S::kGps - 2]), "=f"(sc[q][S::kGps - 1]) : "r"(a));
+            else if constexpr (S::kGps == 2) asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(sc[q][0]), "=f"(sc[q][S::kGps - 1]) : "r"(a));
+            else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc[q][0]) : "r"(a));
+          }
+          if (S::kGps > 1 || (v & 2u)) {   // this team's last look at the unit
+            __syncwarp();
+            mbar_arrive_warp(&empty_s[ss], lane);
+          }
+        } else {
+          asm volatile("cp.async.wait_group %0;" ::"n"(S::kScales - 2) : "memory");
+#pragma unroll
+          for (int q = 0; q < NW; ++q) {
+            const uint32_t a = sring + rs * (256u * S::kScaleBytes) + (uint32_t)(q * S::kGps * 4);
+#pragma unroll
+            for (int g = 0; g < S::kGps; ++g) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc[q][g]) : "r"(a + g * 4));
+          }
+          rs = rs + 1 == S::kScales ? 0 : rs + 1;
+          fetch();
+          __syncwarp();
         }
-      } else {
+        const uint32_t slot = v % kSlots;
+        ok = mbar_wait_warp(&acc_full[v % (2 * kSlots)], (v / (2 * kSlots)) & 1u, &s_abort);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = lane_base + 128u + slot * 128u;
+        constexpr int kN16 = S::kGps * S::kCols / 16;          // 16-column loads of the visit
+        constexpr int kBatch = S::kCols > 64 ? 2 : (kN16 < 4 ? kN16 : (kN16 % 4 == 0 ? 4 : 3));   // in flight at once
+        static_assert(kN16 % kBatch == 0, "loads per visit");
 #pragma unroll
-        for (int q = 0; q < NW; ++q) {
-          uint32_t r[units][8];
+        for (int b = 0; b < kN16 / kBatch; ++b) {
+          uint32_t r[kBatch][16];
 #pragma unroll
-          for (int u = 0; u < units; ++u) tmem_ld8(d + (uint32_t)(q * MP + u * 8), r[u]);
+          for (int i = 0; i < kBatch; ++i) tmem_ld16(d + (uint32_t)((b * kBatch + i) * 16), r[i]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (q == NW - 1) {
+          if (b == kN16 / kBatch - 1) {   // the slot's sums are in registers: hand it back before the arithmetic
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[slot]);
+            mbar_arrive_warp(&acc_empty[slot], lane);
           }
-          const float cq = q ? c1 : c0;
 #pragma unroll
-          for (int u = 0; u < units; ++u)
+          for (int i = 0; i < kBatch; ++i) {
+            const int col = (b * kBatch + i) * 16, g = col / S::kCols, at = col % S::kCols;
+            const float s = sc[at / MP][g];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[q][u * 8 + i] = fmaf(cq, __uint_as_float(r[u][i]), acc[q][u * 8 + i]);
+            for (int e = 0; e < 16; e += 2) fma2(acc[at + e], acc[at + e + 1], r[i][e], r[i][e + 1], s);
+          }
+        }
+      }
+      // ---- the teams' sums: each finishes half of the activation rows ----
+      constexpr int kHalf = MP / 2;
+      epilogue_barrier();   // the last tile's exchange has been read
+#pragma unroll
+      for (int q = 0; q < NW; ++q)
+#pragma unroll
+        for (int i = 0; i < kHalf; ++i) ex[((team * NW + q) * kHalf + i) * 128 + row] = team ? acc[q * MP + i] : acc[q * MP + kHalf + i];
+      epilogue_barrier();
+      float b0 = 0.f, b1 = 0.f;
+      if (kz == 0) {
+        if (p.bias[0] && n0 + row < p.n) b0 = __ldg(p.bias[0] + n0 + row);
+        if (NW == 2 && p.pair) { if (p.bias[1] && n0 + row < p.n) b1 = __ldg(p.bias[1] + n0 + row); }
+        else if (NW == 2 && p.bias[0] && n0 + kTileN + row < p.n) b1 = __ldg(p.bias[0] + n0 + kTileN + row);
+      }
+      float* mine = ex + (team ^ 1) * NW * kHalf * 128 + row;   // what the other team left for this thread; the sums go back there
+#pragma unroll
+      for (int q = 0; q < NW; ++q)
+#pragma unroll
+        for (int i = 0; i < kHalf; ++i) mine[(q * kHalf + i) * 128] += team ? acc[q * MP + kHalf + i] : acc[q * MP + i];
+#pragma unroll 4
+      for (int i = 0; i < kHalf; ++i) {   // from shared memory: the code of this loop must not push the one above out of the instruction cache
+        const int mrow = mt * MP + team * kHalf + i;
+        if (mrow >= p.m || !ok) break;
+        const float inv = __ldg(p.xinv + mrow);
+        float sum[NW];
+#pragma unroll
+        for (int q = 0; q < NW; ++q) sum[q] = fmaf(mine[(q * kHalf + i) * 128], inv, q ? b1 : b0);
+        if (NW == 2 && p.pair) {
+          const int j = n0 + row;
+          if (j < p.n) p.out[(size_t)mrow * p.n + j] = (sum[0] / (1.0f + expf(-sum[0]))) * sum[NW - 1];   // src/llm/decoder.rs:1319-1322
+        } else {
+#pragma unroll
+          for (int q = 0; q < NW; ++q) {
+            const int j = n0 + q * kTileN + row;
+            if (j >= p.n) continue;
+            float* dst = p.out + (size_t)mrow * p.n + j;
+            float val = sum[q];
+            if (p.resid && kz == 0) val += p.resid[(size_t)mrow * p.n + j];
+            if (p.ksplit > 1) atomicAdd(dst, val);
+            else *dst = val;
+          }
         }
       }
     }
-    if (ok && live) {
-      const float b0 = (p.bias[0] && blockIdx.y == 0) ? __ldg(p.bias[0] + j) : 0.f;
-      const float b1 = (NW == 2 && p.bias[1]) ? __ldg(p.bias[1] + j) : 0.f;
-#pragma unroll
-      for (int i = 0; i < half; ++i) {
-        const int mrow = cb + i;
-        if (mrow < p.m) {
-          float v;
-          if (NW == 2) {
-            const float gg = acc[0][i] + b0, uu = acc[NW - 1][i] + b1;
-            v = (gg / (1.0f + expf(-gg))) * uu;   // src/llm/decoder.rs:1319-1322
-          } else {
-            v = acc[0][i] + b0;
-            if (p.resid && blockIdx.y == 0) v += p.resid[(size_t)mrow * p.n + j];
-          }
-          float* dst = p.out + (size_t)mrow * p.n + j;
-          if (p.ksplit > 1) atomicAdd(dst, v);
-          else *dst = v;
-        }
-      }
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -487,70 +552,169 @@ __global__ void __launch_bounds__((DW + 12) * 32, 1) w4_tc5_kernel(const Tc5Para
   }
 }
 
-// Activations -> kPieces bf16 images per 64-element chunk of K (with the fused RMSNorm).  Inside
-// every 8 elements the order is 0 4 1 5 2 6 3 7, the order in which the codes leave a 32-bit
-// word of nibbles.  grid (mp rows, ceil(k / 2048)); rows past m are zero.
-__global__ void __launch_bounds__(256) tc5_prep_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
-                                                       unsigned char* __restrict__ xq, int m, int mp, int k) {
-  __shared__ float s_part[8];
-  const int row = blockIdx.x, tid = threadIdx.x;
-  float inv = 1.f;
-  if (norm_w != nullptr && row < m) {   // fast_rms_norm, src/quantization/fused_ops.rs:1066-1117
-    const float* xr = x + (size_t)row * k;
-    float ss = 0.f;
-    for (int i = tid; i < k; i += 256) ss = fmaf(xr[i], xr[i], ss);
+// One activation row -> kPieces rows of fp16 images (with the fused RMSNorm) and the inverse of the row's power of
+// two.  Inside every 8 elements the order is 0 4 1 5 2 6 3 7, the order in which the codes leave a 32-bit word of
+// nibbles.  One block per row of the padded tiles (rows past m are zero); a thread takes pieces of 8 elements and keeps
+// up to NI of them in registers between the pass that finds the row's largest value and the sum of squares
+// and the pass that writes (NI 0: any length, read twice).  zero_out: rows of the output to clear for a split of K.
+constexpr int kPrepThreads = 512;
+template <int NI>
+__global__ void __launch_bounds__(kPrepThreads) tc5_prep_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
+                                                                unsigned char* __restrict__ xq, float* __restrict__ xinv, int m, int mp,
+                                                                int k, float* __restrict__ zero_out, int n) {
+  __shared__ float s_ss[kPrepThreads / 32], s_mx[kPrepThreads / 32];
+  const int row = blockIdx.x, tid = threadIdx.x, step = (int)blockDim.x * 8;
+  const bool live = row < m;
+  const float* xr = x + (size_t)(live ? row : 0) * k;
+  float v[NI > 0 ? NI : 1][8];
+  auto load = [&](int e, float (&o)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(xr + e), b = *reinterpret_cast<const float4*>(xr + e + 4);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+  };
+  auto weigh = [&](int e, float (&o)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(norm_w + e), b = *reinterpret_cast<const float4*>(norm_w + e + 4);
+    const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((tid & 31) == 0) s_part[tid >> 5] = ss;
-    __syncthreads();
-    float tot = 0.f;
+    for (int i = 0; i < 8; ++i) o[i] *= w[i];
+  };
+  float ss = 0.f, mx = 0.f;
+  auto note = [&](int e, float (&o)[8]) {
+    if (norm_w != nullptr) {   // fast_rms_norm, src/quantization/fused_ops.rs:1066-1117
 #pragma unroll
-    for (int i = 0; i < 8; ++i) tot += s_part[i];
-    inv = 1.0f / sqrtf(tot / (float)k + eps);
-  }
-  // one thread = 8 consecutive elements = one 16-byte piece of an image row
-  const int e = (int)blockIdx.y * 2048 + tid * 8;
-  if (e >= k) return;
-  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (row < m) {
-    const float4 a = *reinterpret_cast<const float4*>(x + (size_t)row * k + e);
-    const float4 b = *reinterpret_cast<const float4*>(x + (size_t)row * k + e + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    if (norm_w != nullptr) {
-      const float4 na = *reinterpret_cast<const float4*>(norm_w + e);
-      const float4 nb = *reinterpret_cast<const float4*>(norm_w + e + 4);
-      const float nw[8] = {na.x, na.y, na.z, na.w, nb.x, nb.y, nb.z, nb.w};
+      for (int i = 0; i < 8; ++i) ss = fmaf(o[i], o[i], ss);
+      weigh(e, o);
+    }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = (v[i] * inv) * nw[i];
+    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(o[i]));
+  };
+  if constexpr (NI > 0) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int e = i * step + tid * 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[i][j] = 0.f;
+      if (live && e < k) load(e, v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int e = i * step + tid * 8;
+      if (live && e < k) note(e, v[i]);
+    }
+  } else if (live) {
+    for (int e = tid * 8; e < k; e += step) {
+      load(e, v[0]);
+      note(e, v[0]);
     }
   }
-  uint32_t img[kPieces][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {   // the pair (i, i + 4)
-    float r0 = v[i], r1 = v[i + 4];
+  for (int o = 16; o > 0; o >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if ((tid & 31) == 0) { s_ss[tid >> 5] = ss; s_mx[tid >> 5] = mx; }
+  __syncthreads();
+  ss = 0.f;
+  mx = 0.f;
+  for (int i = 0; i < (int)blockDim.x / 32; ++i) { ss += s_ss[i]; mx = fmaxf(mx, s_mx[i]); }
+  const float inv = norm_w != nullptr ? 1.0f / sqrtf(ss / (float)k + eps) : 1.f;
+  mx *= inv;
+  // 2^e brings the largest value to [2^14, 2^15); nothing to bring there, or not a number: 2^0
+  const int ex = (int)((__float_as_uint(mx) >> 23) & 255u);
+  int e2 = ex == 0 || ex == 255 ? 0 : 14 - (ex - 127);
+  e2 = e2 > 126 ? 126 : e2;
+  const float up = __uint_as_float((uint32_t)(e2 + 127) << 23);
+  if (tid == 0 && live) xinv[row] = __uint_as_float((uint32_t)(127 - e2) << 23);
+  auto write = [&](int e, const float (&o)[8]) {
+    uint32_t img[kPieces][4];
 #pragma unroll
-    for (int pc = 0; pc < kPieces; ++pc) {
-      uint32_t h0, h1;
-      if (pc + 1 < kPieces) {     // the upper 16 bits are a bf16 number; the remainder is exact
-        h0 = __float_as_uint(r0) & 0xFFFF0000u;
-        h1 = __float_as_uint(r1) & 0xFFFF0000u;
-        r0 -= __uint_as_float(h0);
-        r1 -= __uint_as_float(h1);
-      } else {                    // the last piece is rounded
-        h0 = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(r0)) << 16;
-        h1 = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(r1)) << 16;
+    for (int i = 0; i < 4; ++i) {   // the pair (i, i + 4)
+      const float a = (o[i] * inv) * up, b = (o[i + 4] * inv) * up;
+      const __half2 hi = __floats2half2_rn(a, b);
+      const float2 back = __half22float2(hi);
+      const __half2 lo = __floats2half2_rn(a - back.x, b - back.y);   // the remainder is exact before it is rounded
+      img[0][i] = *reinterpret_cast<const uint32_t*>(&hi);
+      img[1][i] = *reinterpret_cast<const uint32_t*>(&lo);
+    }
+    const int c = e >> 6, jp = (e >> 3) & 7, r = row % mp;
+    unsigned char* dst = xq + ((size_t)(row / mp) * (k / kKC) + c) * (size_t)(kPieces * mp * 128) + r * 128 + ((jp ^ (r & 7)) * 16);
+#pragma unroll
+    for (int pc = 0; pc < kPieces; ++pc)
+      *reinterpret_cast<uint4*>(dst + (size_t)pc * mp * 128) = make_uint4(img[pc][0], img[pc][1], img[pc][2], img[pc][3]);
+  };
+  if constexpr (NI > 0) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int e = i * step + tid * 8;
+      if (e < k) write(e, v[i]);
+    }
+  } else {
+    for (int e = tid * 8; e < k; e += step) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[0][j] = 0.f;
+      if (live) {
+        load(e, v[0]);
+        if (norm_w != nullptr) weigh(e, v[0]);
       }
-      img[pc][i] = (h0 >> 16) | h1;
+      write(e, v[0]);
     }
   }
-  const int c = e >> 6, jp = (e >> 3) & 7;
-  unsigned char* dst = xq + (size_t)c * (kPieces * mp * 128) + row * 128 + ((jp ^ (row & 7)) * 16);
-#pragma unroll
-  for (int pc = 0; pc < kPieces; ++pc)
-    *reinterpret_cast<uint4*>(dst + (size_t)pc * mp * 128) = make_uint4(img[pc][0], img[pc][1], img[pc][2], img[pc][3]);
+  if (zero_out != nullptr && live)
+    for (int j = tid; j < n; j += (int)blockDim.x) zero_out[(size_t)row * n + j] = 0.f;
 }
 
 int g_tc5_enabled = 1;
+
+using Kernel = void (*)(const Tc5Params);
+struct Variant { int mp, nw; Kernel kern[3]; int threads[3]; size_t smem[3]; };
+template <int MP, int NW>
+constexpr Variant variant() {
+  return Variant{MP, NW, {w4_tc5_kernel<MP, NW, 32>, w4_tc5_kernel<MP, NW, 64>, w4_tc5_kernel<MP, NW, 128>},
+                 {Shape<MP, NW, 32>::kThreads, Shape<MP, NW, 64>::kThreads, Shape<MP, NW, 128>::kThreads},
+                 {Shape<MP, NW, 32>::kSmem, Shape<MP, NW, 64>::kSmem, Shape<MP, NW, 128>::kSmem}};
+}
+const Variant kVariants[] = {variant<16, 1>(), variant<32, 1>(), variant<48, 1>(), variant<64, 1>(),
+                             variant<16, 2>(), variant<32, 2>(), variant<48, 2>(), variant<64, 2>()};
+
+// What a launch costs, in cycles of the busiest CTA: tiles one after the other, a stage of 64 elements being bound by the
+// tensor pipe (MP / 2 cycles per MMA and two more, at least 11), by the CTA's share of HBM (23 bytes per cycle and SM when
+// all of them stream, at most twice that when few do) or by the hand-overs.
+struct Plan { const Variant* v; int mtiles, ntiles, ksplit; };
+double plan_cost(const Variant& v, int m, int64_t n, int64_t k, int g, bool pair, int ks, int sms, Plan* plan) {
+  const int rows = pair ? kTileN : kTileN * v.nw;
+  plan->v = &v; plan->ksplit = ks;
+  plan->mtiles = (m + v.mp - 1) / v.mp;
+  plan->ntiles = (int)((n + rows - 1) / rows);
+  const int64_t tiles = (int64_t)plan->mtiles * plan->ntiles * ks;
+  const int64_t waves = (tiles + sms - 1) / sms;
+  const int64_t active = tiles < sms ? tiles : sms;
+  const double mma = 8.0 * v.nw * (v.mp / 2 + 2 > 11 ? v.mp / 2 + 2 : 11);
+  double rate = 23.0 * (double)sms / (double)active;
+  if (rate > 46.0) rate = 46.0;
+  const double hbm = v.nw * kTileN * (32.0 + 256.0 / g) / rate / (plan->mtiles < 4 ? plan->mtiles : 4);
+  const double hand = 64.0 / g * (v.mp * v.nw) * 2.1 + 60.0;   // tensor memory is read at about 64 bytes per cycle and sub-partition
+  const double unpack = v.nw == 2 ? 200.0 : 110.0;
+  double stage = mma > hbm ? mma : hbm;
+  if (hand > stage) stage = hand;
+  if (unpack > stage) stage = unpack;
+  return (double)waves * ((double)(k / ks / kKC) * stage + 600.0 + 12.0 * v.mp * v.nw) + 4000.0;
+}
+Plan choose_plan(int m, int64_t n, int64_t k, int g, bool pair) {
+  const int sms = sm_count();
+  Plan best{}, cur{};
+  double best_cost = 1e30;
+  for (const Variant& v : kVariants) {
+    if (pair && v.nw != 2) continue;
+    for (int ks = 1; ks <= 8; ++ks) {
+      if (ks > 1 && (pair || (k / kUnit) % ks != 0)) continue;   // the SwiGLU needs whole sums: no split
+      const double c = plan_cost(v, m, n, k, g, pair, ks, sms, &cur) + (ks > 1 ? 1500.0 : 0.0);   // partial sums are added in memory
+      if (c < best_cost) { best_cost = c; best = cur; }
+    }
+  }
+  return best;
+}
+
+size_t image_bytes(int rows, int64_t k) { return (size_t)(k / kKC) * kPieces * (size_t)rows * 128; }
+constexpr int kPadRows = 64;   // padding of the last tile: less than the largest tile
 
 }  // namespace
 
@@ -562,69 +726,61 @@ int tc5_fault_flag() {
   return v;
 }
 
+// The inverse powers of two (kMaxRows + kPadRows floats), then the images.
 size_t w4_tc5_scratch_bytes(int m, int64_t k) {
-  const int mp = ((m < 64 ? m : 64) + 15) & ~15;
-  return (size_t)((k + kKC - 1) / kKC) * kPieces * mp * 128;
+  const int rows = (m < kMaxRows ? m : kMaxRows) + kPadRows;
+  return sizeof(float) * (kMaxRows + kPadRows) + image_bytes(rows, (k + kKC - 1) / kKC * kKC);
 }
 
 bool w4_tc5_supported(const GemvArgs& a) {
-  if (!g_tc5_enabled || a.m < kMinRows) return false;
+  if (!g_tc5_enabled || a.m < kMinRows || !tma_encoder()) return false;
   if (a.k % 128 != 0 || a.n < 1 || (a.g != 32 && a.g != 64 && a.g != 128)) return false;
   if (a.x_ss8 || a.out_scaled || a.out_ss8 || a.x_normed_out) return false;
   if ((reinterpret_cast<uintptr_t>(a.w) & 15) || (a.w2 && (reinterpret_cast<uintptr_t>(a.w2) & 15))) return false;
+  if ((reinterpret_cast<uintptr_t>(a.scales) & 15) || (a.w2 && (reinterpret_cast<uintptr_t>(a.scales2) & 15))) return false;   // boxes and copies of up to 16 bytes
   return true;
 }
+
+// Launches of one call: kMaxRows rows at a time, the pre-pass and the product.
+int w4_tc5_launches(int m) { return 2 * ((m + kMaxRows - 1) / kMaxRows); }
 
 tb_status launch_w4_tc5(const GemvArgs& a, void* scratch, cudaStream_t stream) {
   if (!w4_tc5_supported(a)) return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: tcgen05 product: m=%d n=%lld k=%lld", a.m, (long long)a.n, (long long)a.k);
   const bool pair = a.w2 != nullptr;
-  const int tiles = (int)((a.n + kTileN - 1) / kTileN);
-  for (int m0 = 0; m0 < a.m; m0 += 64) {
-    const int mc = a.m - m0 < 64 ? a.m - m0 : 64;
-    const int mp = (mc + 15) & ~15;
+  const int gi = a.g == 32 ? 0 : (a.g == 64 ? 1 : 2);
+  float* xinv = static_cast<float*>(scratch);
+  unsigned char* xq = static_cast<unsigned char*>(scratch) + sizeof(float) * (kMaxRows + kPadRows);
+  const int slabs = (a.m + kMaxRows - 1) / kMaxRows, per = (a.m + slabs - 1) / slabs;
+  for (int m0 = 0; m0 < a.m; m0 += per) {
+    const int mc = a.m - m0 < per ? a.m - m0 : per;
+    const Plan plan = choose_plan(mc, a.n, a.k, a.g, pair);
+    const Variant& v = *plan.v;
     Tc5Params p;
-    p.w[0] = a.w; p.w[1] = a.w2; p.scales[0] = a.scales; p.scales[1] = a.scales2; p.bias[0] = a.bias; p.bias[1] = a.bias2;
+    p.scales[0] = a.scales; p.scales[1] = a.scales2; p.bias[0] = a.bias; p.bias[1] = a.bias2;
     // residual in place (out == resid) with K split: the partial sums are added onto the residual where it lies
-    const bool in_place = a.resid != nullptr && a.resid == a.out;
-    p.resid = a.resid ? a.resid + (size_t)m0 * a.n : nullptr;
+    const bool in_place = a.resid != nullptr && a.resid == a.out && plan.ksplit > 1;
+    p.resid = a.resid && !in_place ? a.resid + (size_t)m0 * a.n : nullptr;
     p.out = a.out + (size_t)m0 * a.n;
-    p.xq = static_cast<const unsigned char*>(scratch);
-    p.m = mc; p.mp = mp; p.n = (int)a.n; p.k = (int)a.k; p.ng = (int)(a.k / a.g); p.g = a.g;
+    p.xq = xq; p.xinv = xinv;
+    p.m = mc; p.n = (int)a.n; p.k = (int)a.k; p.ng = (int)(a.k / a.g);
+    p.mtiles = plan.mtiles; p.ntiles = plan.ntiles; p.ksplit = plan.ksplit; p.kper = (int)(a.k / plan.ksplit);
     p.pair = pair ? 1 : 0;
-    // narrow matrices: several CTAs share a row tile and split K (the SwiGLU needs whole sums: no split)
-    int ksplit = 1;
-    if (!pair) {
-      const int want = sm_count() / tiles;
-      for (int s = want; s >= 2; --s)
-        if ((a.k / 128) % s == 0) { ksplit = s; break; }
+    for (int q = 0; q < (pair ? 2 : 1); ++q) {
+      if (!tma_matrix_map(&p.w[q], CU_TENSOR_MAP_DATA_TYPE_UINT8, q ? a.w2 : a.w, a.k / 2, a.n, a.k / 2, 64, kTileN, CU_TENSOR_MAP_SWIZZLE_64B) ||
+          (a.g == 32 && !tma_matrix_map(&p.s[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, q ? a.scales2 : a.scales, p.ng, a.n, (int64_t)p.ng * 4, 4, kTileN, CU_TENSOR_MAP_SWIZZLE_NONE)))
+        return fail(TB_ERR_CUDA, "tcgen05 product: no TMA description of a %lld x %lld matrix", (long long)a.n, (long long)a.k);
     }
-    p.ksplit = ksplit;
-    p.kper = (int)(a.k / ksplit);
-    const int nw = pair ? 2 : 1;
-    const int stages = nw == 1 ? 8 : 4;
-    p.stages = stages;
-    const int slots = (kTmemCols - stages * 32 * nw) / (mp * nw);
-    p.slots = slots >= 4 ? 4 : 2;   // a power of two (the issuing thread masks and shifts)
-    const size_t smem = (size_t)stages * kPieces * mp * 128 + (size_t)kAhead * nw * kTileN * 32 + 1024;
-    void (*kern)(const Tc5Params) = nullptr;
-    int threads = 16 * 32;
-    switch (mp * 2 + (pair ? 1 : 0)) {
-      case 32: kern = w4_tc5_kernel<16, 1, 8>; threads = 20 * 32; break;
-      case 33: kern = w4_tc5_kernel<16, 2, 8>; threads = 20 * 32; break;
-      case 64: kern = w4_tc5_kernel<32, 1, 8>; threads = 20 * 32; break;
-      case 65: kern = w4_tc5_kernel<32, 2, 4>; break;
-      case 96: kern = w4_tc5_kernel<48, 1, 8>; threads = 20 * 32; break;
-      case 97: kern = w4_tc5_kernel<48, 2, 4>; break;
-      case 128: kern = w4_tc5_kernel<64, 1, 8>; threads = 20 * 32; break;
-      default: kern = w4_tc5_kernel<64, 2, 4>; break;
-    }
-    TB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    tc5_prep_kernel<<<dim3((unsigned)mp, (unsigned)((a.k + 2047) / 2048)), 256, 0, stream>>>(
-        a.x + (size_t)m0 * a.k, a.norm_w, a.eps, static_cast<unsigned char*>(scratch), mc, mp, (int)a.k);
+    const int ni = (int)((a.k + kPrepThreads * 8 - 1) / (kPrepThreads * 8));
+    int threads = (int)((a.k / 8 + 31) / 32 * 32);
+    if (threads > kPrepThreads) threads = kPrepThreads;
+    const auto prep = ni == 1 ? tc5_prep_kernel<1> : ni == 2 ? tc5_prep_kernel<2> : ni <= 4 ? tc5_prep_kernel<4> : tc5_prep_kernel<0>;
+    prep<<<(unsigned)(plan.mtiles * v.mp), threads, 0, stream>>>(a.x + (size_t)m0 * a.k, a.norm_w, a.eps, xq, xinv, mc, v.mp, (int)a.k,
+                                                              plan.ksplit > 1 && !in_place ? p.out : nullptr, (int)a.n);
     TB_CUDA_TRY(cudaGetLastError());
-    if (ksplit > 1 && in_place) p.resid = nullptr;
-    else if (ksplit > 1) TB_CUDA_TRY(cudaMemsetAsync(p.out, 0, sizeof(float) * (size_t)mc * a.n, stream));
-    kern<<<dim3((unsigned)tiles, (unsigned)ksplit), threads, smem, stream>>>(p);
+    TB_CUDA_TRY(cudaFuncSetAttribute(v.kern[gi], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem[gi]));
+    const int64_t tiles = (int64_t)plan.mtiles * plan.ntiles * plan.ksplit;
+    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+    v.kern[gi]<<<grid, v.threads[gi], v.smem[gi], stream>>>(p);
     TB_CUDA_TRY(cudaGetLastError());
   }
   return TB_OK;
