@@ -1,0 +1,318 @@
+// Attention of many positions of ONE sequence over the fp32 KV cache (a portion of a prompt): steps C-E of
+// RustQwenDecoder::step_internal (src/llm/decoder.rs:1127-1213) for rows 0..R-1 at once.  The rows' keys and values are
+// in the cache already (launch_rope_append_rows); row r attends to [0, offsets[r]].
+//
+// The decode kernel (attention.cu) streams the whole cache once per row: 333 rows behind 1024 positions, 8 layers of
+// the 8B widths, took 5.2 ms.  Here a block takes 64 (row, query head) pairs of one key head, so a 64-key tile is
+// loaded once for all of them, and both products are register-tiled fp32 FMAs (4 x 4 scores and 4 rows x D/16 columns a
+// thread): 8 shared-memory reads of 16 bytes per 64 FMAs keep the FMA pipe (128 lanes per SM) the bound.  All of
+// it stays fp32, as in the decode kernel.  K and V of a tile arrive with cp.async; the weights take the place of the
+// keys once the scores are done, so that two blocks fit an SM and one computes while the other loads.  A portion
+// has few blocks (21 x 8 here), so the keys are split as well (`splits`) and a second kernel merges.
+#include "tb_common.cuh"
+
+namespace tb {
+
+namespace {
+
+constexpr int kPairs = 64;     // (row, query head) pairs per block
+constexpr int kKeys = 64;      // keys per tile
+constexpr int kThreads = 256;  // 16 x 16: thread (ty, tx) owns pairs 4 ty .. 4 ty + 3
+
+struct RowsParams {
+  const float* qkv;
+  const float* k_cache;   // [Hkv, max_seq, D] of the sequence
+  const float* v_cache;
+  const float* cos_t;
+  const float* sin_t;
+  const int32_t* offsets;
+  float* out;             // [R, Hq * D]
+  float* part_o;          // [split][R][Hq][D] and (max, sum) pairs when splits > 1
+  float* part_ml;
+  int rows, num_heads, num_kv_heads, gq, rows_per_block, splits;
+  int64_t max_seq_len;
+  float scale;
+};
+
+template <int D>
+constexpr int kStride = D + 4;   // floats per row of Q, K and V in shared memory: rows fall on different banks
+constexpr int kPStride = kKeys + 4;
+
+template <int D>
+constexpr size_t rows_smem() { return sizeof(float) * ((size_t)(kPairs + 2 * kKeys) * kStride<D> + kPairs) + sizeof(int) * kPairs; }
+
+template <int D>
+__global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams p) {
+  extern __shared__ __align__(16) float sm[];
+  float* qs = sm;
+  float* ks = qs + kPairs * kStride<D>;
+  float* vs = ks + kKeys * kStride<D>;
+  int* lim = reinterpret_cast<int*>(vs + kKeys * kStride<D>);
+  constexpr bool kOwnP = kPairs * kPStride > kKeys * kStride<D>;   // narrow heads: the weights do not fit over the keys
+  __shared__ __align__(16) float p_own[kOwnP ? kPairs * kPStride : 4];
+  float* ps = kOwnP ? p_own : ks;
+  __shared__ int s_max, s_min;
+
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int r0 = blockIdx.x * p.rows_per_block, kvh = blockIdx.y, split = blockIdx.z;
+  const int nrows = min(p.rows_per_block, p.rows - r0), npairs = nrows * p.gq;
+  const int64_t qkv_dim = (int64_t)(p.num_heads + 2 * p.num_kv_heads) * D;
+  if (tid == 0) { s_max = 0; s_min = 0x7fffffff; }
+  __syncthreads();
+  if (tid < kPairs) {   // keys that pair tid sees: none for pairs past the block's and for tokens out of range
+    int n = 0;
+    if (tid < npairs) {
+      const int off = p.offsets[r0 + tid / p.gq];
+      if (off >= 0 && (int64_t)off < p.max_seq_len) n = off + 1;
+      atomicMin(&s_min, n);
+    }
+    lim[tid] = n;
+    atomicMax(&s_max, n);
+  }
+  // the rotated queries (rotate-half with separately rounded products, src/llm/decoder.rs:40-66)
+  for (int i = tid; i < kPairs * D; i += kThreads) {
+    const int m = i / D, e = i - m * D;
+    float v = 0.f;
+    if (m < npairs) {
+      const int r = r0 + m / p.gq, off = p.offsets[r];
+      if (off >= 0 && (int64_t)off < p.max_seq_len) {
+        const float* x = p.qkv + (int64_t)r * qkv_dim + (int64_t)(kvh * p.gq + m % p.gq) * D;
+        const float c = p.cos_t[(int64_t)off * D + e], s = p.sin_t[(int64_t)off * D + e];
+        v = e < D / 2 ? __fsub_rn(__fmul_rn(x[e], c), __fmul_rn(x[e + D / 2], s)) : __fadd_rn(__fmul_rn(x[e], c), __fmul_rn(x[e - D / 2], s));
+      }
+    }
+    qs[m * kStride<D> + e] = v;
+  }
+  __syncthreads();
+  const int t_end = s_max, t_all = s_min;   // keys of the block; every pair sees the keys below t_all
+  const int tiles = (t_end + kKeys - 1) / kKeys, per = (tiles + p.splits - 1) / p.splits;
+  const int tile0 = split * per, tile1 = min(tiles, tile0 + per);
+  const float* kc = p.k_cache + (int64_t)kvh * p.max_seq_len * D;
+  const float* vc = p.v_cache + (int64_t)kvh * p.max_seq_len * D;
+
+  auto copy = [&](float* dst, const float* src, int t0) {   // 64 rows, zeros past the last key
+    for (int i = tid; i < kKeys * (D / 4); i += kThreads) {
+      const int r = i / (D / 4), c = i - r * (D / 4);
+      const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + r * kStride<D> + c * 4);
+      const bool in = t0 + r < t_end;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src + (int64_t)(in ? t0 + r : 0) * D + c * 4), "r"(in ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  constexpr int kC = D / 64 > 0 ? D / 64 : 1;      // column blocks of a thread, 64 apart
+  constexpr int kW = D >= 64 ? 4 : D / 16;         // columns of a block (D = 32: 2)
+  float o[4][kC * kW], m_run[4], l_run[4];
+  int lm[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m_run[i] = -INFINITY;
+    l_run[i] = 0.f;
+    lm[i] = lim[ty * 4 + i];
+#pragma unroll
+    for (int c = 0; c < kC * kW; ++c) o[i][c] = 0.f;
+  }
+  if (tile0 < tile1) {
+    copy(ks, kc, tile0 * kKeys);
+    copy(vs, vc, tile0 * kKeys);
+  }
+  for (int t = tile0; t < tile1; ++t) {
+    const int t0 = t * kKeys;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    // ---- scores: pairs 4 ty + i, keys tx + 16 j ----
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+      float4 q[4], k[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * kStride<D> + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * kStride<D> + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(q[i].x, k[j].x, s[i][j]);
+          s[i][j] = fmaf(q[i].y, k[j].y, s[i][j]);
+          s[i][j] = fmaf(q[i].z, k[j].z, s[i][j]);
+          s[i][j] = fmaf(q[i].w, k[j].w, s[i][j]);
+        }
+    }
+    __syncthreads();   // the keys have been read: their place takes the weights
+    const bool whole = t0 + kKeys <= t_all;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = whole || t0 + tx + 16 * j < lm[i] ? s[i][j] * p.scale : -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
+      }
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+      const float m_new = fmaxf(m_run[i], mx), base = m_new == -INFINITY ? 0.f : m_new;
+      const float resc = expf(m_run[i] - base);
+      m_run[i] = m_new;
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = expf(s[i][j] - base);
+        ps[(ty * 4 + i) * kPStride + tx + 16 * j] = e;
+        sum += e;
+      }
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+      l_run[i] = l_run[i] * resc + sum;
+#pragma unroll
+      for (int c = 0; c < kC * kW; ++c) o[i][c] *= resc;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // ---- weights times values: columns 64 c + kW tx + w ----
+    const int keys = min(kKeys, t_end - t0);
+#pragma unroll 2
+    for (int k0 = 0; k0 < kKeys; k0 += 4) {
+      float4 w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (ty * 4 + i) * kPStride + k0);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        float v[kC * kW];
+#pragma unroll
+        for (int c = 0; c < kC; ++c) {
+          const float* src = vs + (k0 + kk) * kStride<D> + 64 * c + kW * tx;
+          if constexpr (kW == 4) {
+            const float4 f = *reinterpret_cast<const float4*>(src);
+            v[4 * c] = f.x; v[4 * c + 1] = f.y; v[4 * c + 2] = f.z; v[4 * c + 3] = f.w;
+          } else {
+            const float2 f = *reinterpret_cast<const float2*>(src);
+            v[0] = f.x; v[1] = f.y;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float wi = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+          if (whole || t0 + k0 + kk < lm[i]) {   // a later position's values, whatever they are, do not touch this pair
+#pragma unroll
+            for (int c = 0; c < kC * kW; ++c) o[i][c] = fmaf(wi, v[c], o[i][c]);
+          }
+        }
+      }
+      if (k0 + 4 >= keys) break;
+    }
+    __syncthreads();   // weights and values have been read
+    if (t + 1 < tile1) {
+      copy(ks, kc, t0 + kKeys);
+      copy(vs, vc, t0 + kKeys);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = ty * 4 + i;
+    if (m >= npairs) continue;
+    const int64_t row = r0 + m / p.gq, head = kvh * p.gq + m % p.gq;
+    float* dst;
+    float f = 1.f;
+    if (p.splits == 1) {
+      dst = p.out + (row * p.num_heads + head) * D;
+      f = 1.0f / fmaxf(l_run[i], 1e-30f);   // src/llm/decoder.rs:1203
+    } else {
+      const int64_t at = ((int64_t)split * p.rows + row) * p.num_heads + head;
+      dst = p.part_o + at * D;
+      if (tx == 0) *reinterpret_cast<float2*>(p.part_ml + at * 2) = make_float2(m_run[i], l_run[i]);
+    }
+#pragma unroll
+    for (int c = 0; c < kC; ++c)
+#pragma unroll
+      for (int w = 0; w < kW; ++w) dst[64 * c + kW * tx + w] = o[i][c * kW + w] * f;
+  }
+}
+
+// One block per row: the splits' sums brought to one maximum and normalised, in the order of the splits.
+__global__ void __launch_bounds__(256) attn_rows_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, float* __restrict__ out,
+                                                              int rows, int num_heads, int d, int splits) {
+  const int64_t row = blockIdx.x;
+  for (int i = threadIdx.x; i < num_heads * d / 4; i += 256) {
+    const int head = i / (d / 4), c = i - head * (d / 4);
+    float mx = -INFINITY;
+    for (int s = 0; s < splits; ++s) mx = fmaxf(mx, part_ml[(((int64_t)s * rows + row) * num_heads + head) * 2]);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
+    for (int s = 0; s < splits; ++s) {
+      const int64_t at = ((int64_t)s * rows + row) * num_heads + head;
+      const float2 ml = *reinterpret_cast<const float2*>(part_ml + at * 2);
+      if (ml.x == -INFINITY && ml.y == 0.f) continue;   // no key of this split
+      const float w = expf(ml.x - mx);
+      const float4 v = *reinterpret_cast<const float4*>(part_o + at * d + c * 4);
+      a.x = fmaf(w, v.x, a.x); a.y = fmaf(w, v.y, a.y); a.z = fmaf(w, v.z, a.z); a.w = fmaf(w, v.w, a.w);
+      l = fmaf(w, ml.y, l);
+    }
+    const float f = 1.0f / fmaxf(l, 1e-30f);
+    *reinterpret_cast<float4*>(out + (row * num_heads + head) * d + c * 4) = make_float4(a.x * f, a.y * f, a.z * f, a.w * f);
+  }
+}
+
+constexpr int kMaxSplits = 8;
+
+// Splits of the keys: the fewest waves of two blocks per SM times tiles per block (and about two tiles' worth of start-up).
+int choose_splits(int blocks, int64_t keys) {
+  const int64_t tiles = (keys + kKeys - 1) / kKeys, slots = 2ll * sm_count();
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int s = 1; s <= kMaxSplits && s <= tiles; ++s) {
+    const int64_t cost = ((int64_t)blocks * s + slots - 1) / slots * ((tiles + s - 1) / s + 2) + (s > 1 ? 1 : 0);
+    if (cost < best_cost) { best_cost = cost; best = s; }
+  }
+  return best;
+}
+
+template <int D>
+tb_status launch_rows(const RowsParams& p, cudaStream_t stream) {
+  TB_CUDA_TRY(cudaFuncSetAttribute(attn_rows_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<D>()));
+  const int blocks = (p.rows + p.rows_per_block - 1) / p.rows_per_block;
+  attn_rows_kernel<D><<<dim3((unsigned)blocks, (unsigned)p.num_kv_heads, (unsigned)p.splits), kThreads, rows_smem<D>(), stream>>>(p);
+  TB_CUDA_TRY(cudaGetLastError());
+  if (p.splits > 1) {
+    attn_rows_merge_kernel<<<(unsigned)p.rows, 256, 0, stream>>>(p.part_o, p.part_ml, p.out, p.rows, p.num_heads, D, p.splits);
+    TB_CUDA_TRY(cudaGetLastError());
+  }
+  return TB_OK;
+}
+
+}  // namespace
+
+size_t attention_rows_scratch_bytes(int rows, int num_heads, int head_dim) {
+  return sizeof(float) * (size_t)kMaxSplits * rows * num_heads * (head_dim + 2);
+}
+
+tb_status launch_attention_rows(const AttnArgs& a, int64_t keys, cudaStream_t stream, int* launches) {
+  if (!a.qkv || !a.k_cache || !a.v_cache || !a.cos_t || !a.sin_t || !a.offsets || !a.out || !a.scratch || a.per_call_tables || !a.shared_cache)
+    return fail(TB_ERR_ARG, "attention rows: null operand, or not the positions of one sequence");
+  if (a.num_kv_heads <= 0 || a.num_heads % a.num_kv_heads != 0 || a.num_heads / a.num_kv_heads > 8 || a.batch < 1)
+    return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: attention rows: %d heads over %d, %d rows", a.num_heads, a.num_kv_heads, a.batch);
+  if ((reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache) | reinterpret_cast<uintptr_t>(a.out)) & 15)
+    return fail(TB_ERR_ARG, "attention rows: caches and output must be 16-byte aligned");
+  RowsParams p;
+  p.qkv = a.qkv; p.k_cache = a.k_cache; p.v_cache = a.v_cache; p.cos_t = a.cos_t; p.sin_t = a.sin_t; p.offsets = a.offsets; p.out = a.out;
+  p.rows = a.batch; p.num_heads = a.num_heads; p.num_kv_heads = a.num_kv_heads; p.gq = a.num_heads / a.num_kv_heads;
+  p.rows_per_block = kPairs / p.gq;
+  p.max_seq_len = a.max_seq_len;
+  p.scale = 1.0f / sqrtf((float)a.head_dim);
+  p.splits = choose_splits((p.rows + p.rows_per_block - 1) / p.rows_per_block * p.num_kv_heads, keys);
+  p.part_o = static_cast<float*>(a.scratch);
+  p.part_ml = p.part_o + (size_t)p.splits * p.rows * p.num_heads * a.head_dim;
+  if (launches) *launches += p.splits > 1 ? 2 : 1;
+  switch (a.head_dim) {
+    case 128: return launch_rows<128>(p, stream);
+    case 64: return launch_rows<64>(p, stream);
+    case 32: return launch_rows<32>(p, stream);
+  }
+  return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: head_dim %d (supported: 32, 64, 128)", a.head_dim);
+}
+
+}  // namespace tb

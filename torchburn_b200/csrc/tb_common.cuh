@@ -170,6 +170,10 @@ void set_attention_tuning(int ctas_per_sm, int stages);
 int attention_fault_flag();
 tb_status launch_attention_decode(const AttnArgs& a, cudaStream_t stream);
 tb_status launch_rope_append_rows(const AttnArgs& a, cudaStream_t stream);
+// Many positions of one sequence, the last of them at `keys` - 1, appended beforehand (attention_rows.cu); a.scratch holds
+// attention_rows_scratch_bytes of the launch's rows.  Adds the kernels it starts to *launches.
+size_t attention_rows_scratch_bytes(int rows, int num_heads, int head_dim);
+tb_status launch_attention_rows(const AttnArgs& a, int64_t keys, cudaStream_t stream, int* launches);
 // The library's built-in scratch block for tb_attention_decode_static (attention.cu).
 size_t static_attention_scratch_capacity();
 tb_status static_attention_scratch(void** ptr);

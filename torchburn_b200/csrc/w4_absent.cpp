@@ -25,6 +25,8 @@ void set_attention_tuning(int, int) {}
 int attention_fault_flag() { return 0; }
 tb_status launch_attention_decode(const AttnArgs&, cudaStream_t) { return absent(); }
 tb_status launch_rope_append_rows(const AttnArgs&, cudaStream_t) { return absent(); }
+size_t attention_rows_scratch_bytes(int, int, int) { return 0; }
+tb_status launch_attention_rows(const AttnArgs&, int64_t, cudaStream_t, int*) { return absent(); }
 size_t static_attention_scratch_capacity() { return 0; }
 tb_status static_attention_scratch(void**) { return absent(); }
 int w4_step_grid() { return 0; }
