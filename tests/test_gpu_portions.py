@@ -1,0 +1,201 @@
+"""The INT4 path at many rows: the tcgen05 product at the edges of its tiles, attention shares of unequal sequences, long
+portions of a prompt, and the feed-forward call's workspace.
+
+The product is compared with float64.  Per output, with A = sum |x| |w|: activations carry 23 bits (2^-23 A); codes and
+their products are exact; a group's sum takes 2 * g / 16 <= 16 accumulating instructions, which may truncate (2^-23 of at
+most A each), and the sum over K / g groups, the pieces of a split and the bias take one fp32 rounding each (2^-24 A): at
+most (17 * 2 + K / g + 10) * 2^-24 * A, an order of magnitude above what random signs leave."""
+import threading
+
+import numpy as np
+import pytest
+
+from helpers import max_rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.fail("no CUDA device: GPU tests need a B200")
+    return torch
+
+
+@pytest.fixture(scope="module")
+def tb(torch):
+    import torchburn_b200 as tb
+
+    return tb
+
+
+def int4(torch, n, k, g, seed):
+    """(packed, scales, the weights in float64), on the GPU."""
+    gen = torch.Generator("cuda").manual_seed(seed)
+    w = torch.randn(n, k // g, g, device="cuda", generator=gen) * 0.02
+    s = (w.abs().amax(-1) / 7).clamp_min(1e-8)
+    c = (w / s[..., None]).round_().clamp_(-8, 7)
+    q = c.add(8).to(torch.uint8).reshape(n, k)
+    return (q[:, 0::2] | (q[:, 1::2] << 4)).contiguous(), s.contiguous(), (c.double() * s.double()[..., None]).reshape(n, k)
+
+
+def rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("m,n,k,g", [
+    (9, 1, 128, 32), (16, 129, 256, 64), (17, 1152, 896, 32), (33, 300, 4864, 64), (48, 257, 1024, 128), (49, 896, 4864, 32), (64, 14336, 4096, 128),
+    (65, 6144, 4096, 32), (128, 255, 128, 128), (301, 1433, 4096, 64), (333, 4096, 14336, 32), (512, 896, 896, 32), (513, 1000, 256, 64), (20, 200, 20480, 64),
+    (301, 14330, 4096, 64), (333, 4096, 14336, 64),   # several tiles per CTA, rings that refill at once
+])
+def test_products_of_many_rows_match_float64(torch, tb, m, n, k, g):
+    """Rows, outputs and K around the tiles (16 to 64 rows, 128 or 256 outputs, 128 elements of K), one and several
+    tiles per CTA, K split and not; rows whose sizes differ by 10^6; bias and none."""
+    p, s, w = int4(torch, n, k, g, m + n + k)
+    gen = torch.Generator("cuda").manual_seed(m)
+    x = torch.randn(m, k, device="cuda", generator=gen) * 10 ** (6 * torch.rand(m, 1, device="cuda", generator=gen) - 3)
+    b = torch.randn(n, device="cuda", generator=gen)
+    want = x.double() @ w.T
+    for bias in (None, b, None, b):
+        got = tb.w4a32_grouped_linear(x, p, s, bias, g)
+        ref = want if bias is None else want + bias.double()
+        bound = (44 + k // g) * 2.0 ** -24 * (x.double().abs() @ w.abs().T + (0 if bias is None else bias.double().abs()))
+        assert bool(((got.double() - ref).abs() <= bound).all())
+        assert n < 100 or rel(got, ref) < 1e-6   # 2-norm over many outputs: what fp32 sums show is 2e-7
+    assert tb.lib().tb_device_fault_flag() == 0
+
+
+@pytest.mark.parametrize("m,n,k,g", [(9, 100, 128, 32), (40, 500, 256, 64), (64, 4864, 896, 32), (100, 300, 512, 128), (333, 1024, 4096, 32)])
+def test_gate_up_pair_of_many_rows_matches_float64(torch, tb, m, n, k, g):
+    a, b = int4(torch, n, k, g, 1), int4(torch, n, k, g, 2)
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    gate, up = x.double() @ a[2].T, x.double() @ b[2].T
+    out = torch.full((m, n), float("nan"), device="cuda")
+    assert tb.lib().tb_swiglu_gemv_w4a32(x.data_ptr(), a[0].data_ptr(), a[1].data_ptr(), None, b[0].data_ptr(), b[1].data_ptr(), None,
+                                         out.data_ptr(), m, n, k, g, torch.cuda.current_stream().cuda_stream) == 0, tb.last_error()
+    assert rel(out, torch.nn.functional.silu(gate) * up) < 1e-6
+
+
+def test_special_rows_of_a_product(torch, tb):
+    """Zeros, numbers at both ends of fp32 and a NaN stay in their rows."""
+    m, n, k, g = 20, 96, 256, 32
+    p, s, w = int4(torch, n, k, g, 5)
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator("cuda").manual_seed(6))
+    x[3] = 0
+    x[4] *= 1e-35
+    x[5] *= 1e33
+    x[6, 7] = float("nan")
+    x[7] = 0
+    x[7, 200] = 2.5e-39   # a denormal
+    got, want = tb.w4a32_grouped_linear(x, p, s, None, g), x.double() @ w.T
+    assert not got[3].any()
+    assert got[6].isnan().all() and not got[[i for i in range(m) if i != 6]].isnan().any()
+    bound = (44 + k // g) * 2.0 ** -24 * (x.double().abs() @ w.abs().T)
+    for i in (0, 4, 5, 19):
+        assert bool(((got[i].double() - want[i]).abs() <= bound[i]).all())
+    assert float((got[7].double() - want[7]).abs().max()) < 2e-39   # denormal sums may come out as zeros
+
+
+@pytest.mark.parametrize("heads,kv,dim,lengths", [
+    (32, 8, 128, [4096 * (i + 1) // 32 - i % 3 for i in range(32)]), (14, 2, 64, [1, 33, 2000, 31, 64, 65]), (8, 8, 32, [5, 0, 700]),
+    (4, 4, 128, [32, 96]), (16, 8, 64, [3000] + [1] * 39), (8, 1, 128, [1500]),
+])
+def test_attention_of_unequal_sequences(torch, tb, heads, kv, dim, lengths):
+    """A batch whose lengths differ by orders of magnitude (0: a sequence that takes no part), against float64."""
+    b, top = len(lengths), max(lengths) + 1
+    gen = torch.Generator("cuda").manual_seed(b)
+    qkv = torch.randn(b, (heads + 2 * kv) * dim, device="cuda", generator=gen)
+    kc, vc = (torch.randn(b, kv, top, dim, device="cuda", generator=gen) for _ in range(2))
+    cos, sin = torch.ones(top, dim, device="cuda"), torch.zeros(top, dim, device="cuda")
+    off = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device="cuda")
+    out = torch.full((b, heads * dim), float("nan"), device="cuda")
+    want = torch.zeros(b, heads, dim, dtype=torch.float64, device="cuda")
+    for i, n in enumerate(lengths):
+        if n == 0:
+            continue
+        q, k, v = qkv[i].double().split([heads * dim, kv * dim, kv * dim])
+        ks = torch.cat([kc[i, :, :n - 1].double(), k.view(kv, 1, dim)], 1).repeat_interleave(heads // kv, 0)
+        vs = torch.cat([vc[i, :, :n - 1].double(), v.view(kv, 1, dim)], 1).repeat_interleave(heads // kv, 0)
+        w = torch.softmax((ks @ q.view(heads, dim, 1)).squeeze(-1) * dim ** -0.5, -1)
+        want[i] = (w[:, None] @ vs).squeeze(1)
+    L = tb.lib()
+    nbytes = L.tb_attention_scratch_bytes(b, heads, kv, dim, top)
+    scratch = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    for _ in range(2):   # the tickets are left as they were found
+        rc = L.tb_attention_decode(qkv.data_ptr(), kc.data_ptr(), vc.data_ptr(), cos.data_ptr(), sin.data_ptr(), off.data_ptr(), out.data_ptr(),
+                                   scratch.data_ptr(), b, heads, kv, dim, top, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, tb.last_error()
+        assert float((out.view(b, heads, dim).double() - want).abs().max()) < 1e-5
+    assert L.tb_device_fault_flag() == 0
+
+
+def small_decoder(torch, tb, heads, kv, dim, rows, group, seed=0, layers=2, vocab=500, top=1400):
+    hidden, inter = 256, 384
+    t = lambda n, k, i: int4(torch, n, k, group, seed + i)[:2]
+    norm = lambda i: torch.randn(hidden, device="cuda", generator=torch.Generator("cuda").manual_seed(seed + i)) * 0.1 + 1
+    data = []
+    for l in range(layers):
+        i = 10 * l
+        data.append([norm(i), *t((heads + 2 * kv) * dim, hidden, i + 1), *t(hidden, heads * dim, i + 2), norm(i + 3), *t(inter, hidden, i + 4),
+                     *t(inter, hidden, i + 5), *t(hidden, inter, i + 6), None])
+    embed = torch.randn(vocab, hidden, device="cuda", generator=torch.Generator("cuda").manual_seed(seed + 99))
+    return tb.B200QwenDecoder(embed, data, norm(98), *t(vocab, hidden, 97), layers, hidden, inter, heads, kv, dim, group, 1e-6, top, 10000.0, max_batch=rows)
+
+
+@pytest.mark.parametrize("heads,kv,dim,rows,n,start", [(8, 2, 64, 4, 5, 0), (4, 4, 32, 2, 130, 7), (14, 2, 64, 8, 333, 100), (8, 1, 128, 32, 700, 0), (6, 2, 128, 3, 1100, 250)])
+def test_long_portions_equal_single_steps(torch, tb, heads, kv, dim, rows, n, start):
+    """A prompt in long portions against a decoder of one row that takes it token by token: wanted logits in any order, the
+    last ones, the cache; a token out of range in the middle; more tokens behind."""
+    many = small_decoder(torch, tb, heads, kv, dim, rows, 32)
+    one = small_decoder(torch, tb, heads, kv, dim, 1, 32)
+    ids = np.random.default_rng(n).integers(0, 500, start + n + 3).tolist()
+    ids[start + n // 2] = 100000 if n > 100 else ids[start + n // 2]
+    steps = [one.step(t, i) for i, t in enumerate(ids)]
+    if start:
+        many.prefill_tokens(ids[:start], 0)
+    want = [0, n - 1, n // 3]
+    got = many.extend(ids[start:start + n], start, want=want)
+    for w, row in zip(want, got):
+        assert max_rel_err(row, steps[start + w]) < 1e-4
+    assert max_rel_err(many.get_logits(), steps[start + n - 1]) < 1e-4
+    for i in range(3):
+        assert max_rel_err(many.step(ids[start + n + i], start + n + i), steps[start + n + i]) < 1e-4
+
+
+def test_feed_forward_calls_of_several_threads(torch, tb):
+    """Threads on one stream and on their own, sizes that grow and shrink: every call has its workspace to itself."""
+    hidden, inter, g = 256, 640, 32
+    mods = []
+    ws = []
+    for i, (n, k) in enumerate(((inter, hidden), (inter, hidden), (hidden, inter))):
+        p, s, w = int4(torch, n, k, g, 40 + i)
+        m = tb.QuantizedLinear(k, n, group_size=g).cuda().requires_grad_(False)
+        m.qweight.copy_(p)
+        m.scales.copy_(s)
+        mods.append(m)
+        ws.append(w)
+    bad = []
+
+    def work(seed, stream):
+        with torch.cuda.stream(stream):
+            for i in range(12):
+                x = torch.randn((seed * 7 + i * 13) % 90 + 1, hidden, device="cuda", generator=torch.Generator("cuda").manual_seed(seed * 100 + i))
+                y = tb.fused_swiglu_mlp(x, *mods)
+                d = x.double()
+                ref = (torch.nn.functional.silu(d @ ws[0].T) * (d @ ws[1].T)) @ ws[2].T
+                if rel(y, ref) > 2e-6:
+                    bad.append((seed, i, rel(y, ref)))
+    tb.fused_swiglu_mlp(torch.zeros(1, hidden, device="cuda"), *mods)   # the modules' handles
+    shared = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ts = [threading.Thread(target=work, args=(i, shared if i < 2 else torch.cuda.Stream())) for i in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    torch.cuda.synchronize()
+    assert not bad
+    tb.lib().tb_release_workspaces()
+    work(9, shared)
+    torch.cuda.synchronize()
+    assert not bad

@@ -193,7 +193,7 @@ template <int MP, int NW, int G>
 __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(const __grid_constant__ Tc5Params p) {
   using S = Shape<MP, NW, G>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t full_a[kRing], full_b[kRing], done[kRing], full_w[8], empty_w[8], full_s[8], empty_s[8], acc_full[2 * kSlots], acc_empty[kSlots], drained[kSlots];
+  __shared__ __align__(8) uint64_t full_a[kRing], full_b[kRing], done[kRing], full_w[8], empty_w[8], empty_s[8], acc_full[2 * kSlots], acc_empty[kSlots], drained[kSlots];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
 
@@ -215,10 +215,7 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       mbar_init(&full_w[s], 1);
       mbar_init(&empty_w[s], NW == 2 && S::kDW == 8 ? 8 : 4);   // one lane of each warp that reads the unit
     }
-    for (int s = 0; s < S::kScales; ++s) {
-      mbar_init(&full_s[s], 1);
-      mbar_init(&empty_s[s], S::kGps == 4 ? 4 : 8);             // one team reads a unit's scales, or both
-    }
+    for (int s = 0; s < S::kScales; ++s) mbar_init(&empty_s[s], S::kGps == 4 ? 4 : 8);   // one team reads a unit's scales, or both
     for (int s = 0; s < kSlots; ++s) {
       mbar_init(&acc_empty[s], 4);   // one lane of each warp of the team that read it
       mbar_init(&drained[s], 1);
@@ -281,7 +278,7 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
                 else mma_f16_ts<1>(d, a, b, idesc);
               }
           }
-          if (sv == kStagesPerVisit - 1) mma_commit(&acc_full[v % (2 * kSlots)]);
+          if (sv == kStagesPerVisit - 1) mma_commit(&acc_full[me + (turn & 1u) * kSlots]);
           mma_commit(&done[c % kRing]);
         }
         if (!ok) break;
@@ -302,18 +299,17 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
         for (int i = 0; i < nunits && ok; ++i, ++u) {
           const uint32_t ws = u % S::kUnits, ss = u % S::kScales;
           if (u >= S::kUnits) ok = mbar_wait_fast(&empty_w[ws], (u / S::kUnits - 1u) & 1u, &s_abort);
+          if (G == 32 && ok && u >= S::kScales) ok = mbar_wait_fast(&empty_s[ss], (u / S::kScales - 1u) & 1u, &s_abort);
           if (!ok) break;
-          mbar_expect_tx(&full_w[ws], NW * kUnitBytes);
+          // the scales arrive with the codes: who has seen sums of the unit has seen its scales
+          mbar_expect_tx(&full_w[ws], NW * (kUnitBytes + (G == 32 ? kUnitScaleBytes : 0)));
 #pragma unroll
           for (int q = 0; q < NW; ++q)
             tma_box(w_at + (ws * NW + q) * kUnitBytes, &p.w[p.pair ? q : 0], kz * (p.kper >> 1) + i * 64, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
           if constexpr (G == 32) {
-            if (u >= S::kScales) ok = mbar_wait_fast(&empty_s[ss], (u / S::kScales - 1u) & 1u, &s_abort);
-            if (!ok) break;
-            mbar_expect_tx(&full_s[ss], NW * kUnitScaleBytes);
 #pragma unroll
             for (int q = 0; q < NW; ++q)
-              tma_box(s_at + (ss * NW + q) * kUnitScaleBytes, &p.s[p.pair ? q : 0], kz * (p.kper / G) + i * 4, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_s[ss]));
+              tma_box(s_at + (ss * NW + q) * kUnitScaleBytes, &p.s[p.pair ? q : 0], kz * (p.kper / G) + i * 4, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
           }
           for (int h = 0; h < 2; ++h, ++c) {
             if (c >= SB) ok = mbar_wait_fast(&done[(c - SB) % kRing], ((c - SB) / kRing) & 1u, &s_abort);
@@ -328,8 +324,6 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
         int no_abort = 0;
         for (uint32_t i = c > SB ? c - SB : 0; i < c; ++i) mbar_wait_fast(&full_b[i % kRing], (i / kRing) & 1u, &no_abort);
         for (uint32_t i = u > S::kUnits ? u - S::kUnits : 0; i < u; ++i) mbar_wait_fast(&full_w[i % S::kUnits], (i / S::kUnits) & 1u, &no_abort);
-        if (G == 32)
-          for (uint32_t i = u > S::kScales ? u - S::kScales : 0; i < u; ++i) mbar_wait_fast(&full_s[i % S::kScales], (i / S::kScales) & 1u, &no_abort);
       }
     }
   } else if (warp < S::kDW) {
@@ -367,10 +361,6 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
 #pragma unroll
             for (int w = 0; w < 4; ++w) unpack8(wd[w], &v[e][4 * w]);
           }
-          if (h == 1 && i == kTiles - 1) {   // the unit has been read
-            __syncwarp();
-            mbar_arrive_warp(&empty_w[ws], lane);
-          }
           // the codes are ready in registers before the stage is free: from "free" to "full" it is only the store
           if (i == 0) {
             if (c >= SA) ok = mbar_wait_warp(&done[(c - SA) % kRing], ((c - SA) / kRing) & 1u, &s_abort);
@@ -381,6 +371,9 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
           tmem_st16(col + 16u, v[1]);
         }
         if (!ok) break;
+        // The unit has been read.  Not before the stores: they need the words in registers, while an arrival right behind the
+        // loads can overtake them.
+        if (h == 1) mbar_arrive_warp(&empty_w[ws], lane);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
@@ -430,7 +423,8 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
     if constexpr (G != 32)
 #pragma unroll 1
       for (int i = 0; i < S::kScales - 1; ++i) fetch();
-    uint32_t v = (uint32_t)team, tile_end = 0, rs = 0;
+    uint32_t v = (uint32_t)team, tile_end = 0, rs = 0, at6 = (uint32_t)team, par6 = 0;   // at6: v modulo 6, par6: its round's parity
+    int read_s = -1;
     bool ok = true;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
       tile_end += (uint32_t)nvisits;
@@ -440,40 +434,29 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
 #pragma unroll
       for (int i = 0; i < S::kCols; ++i) acc[i] = 0.f;
       for (; v < tile_end && ok; v += 2) {
-        float sc[NW][S::kGps];
-        if constexpr (G == 32) {
-          constexpr uint32_t kPerUnit = 4 / S::kGps;   // visits per unit
-          const uint32_t un = v / kPerUnit, ss = un % S::kScales;
-          ok = mbar_wait_warp(&full_s[ss], (un / S::kScales) & 1u, &s_abort);
-          if (!ok) break;
-#pragma unroll
-          for (int q = 0; q < NW; ++q) {
-            const uint32_t a = sring + (ss * NW + (uint32_t)q) * kUnitScaleBytes + (v % kPerUnit) * (uint32_t)(S::kGps * 4);
-            if constexpr (S::kGps == 4)
-              asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(sc[q][0]), "=f"(sc[q][1]), "=f"(sc[q][S::kGps - 2]), "=f"(sc[q][S::kGps - 1]) : "r"(a));
-            else if constexpr (S::kGps == 2) asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(sc[q][0]), "=f"(sc[q][S::kGps - 1]) : "r"(a));
-            else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc[q][0]) : "r"(a));
-          }
-          if (S::kGps > 1 || (v & 2u)) {   // this team's last look at the unit
-            __syncwarp();
-            mbar_arrive_warp(&empty_s[ss], lane);
-          }
-        } else {
+        if constexpr (G != 32) {
           asm volatile("cp.async.wait_group %0;" ::"n"(S::kScales - 2) : "memory");
-#pragma unroll
-          for (int q = 0; q < NW; ++q) {
-            const uint32_t a = sring + rs * (256u * S::kScaleBytes) + (uint32_t)(q * S::kGps * 4);
-#pragma unroll
-            for (int g = 0; g < S::kGps; ++g) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc[q][g]) : "r"(a + g * 4));
-          }
-          rs = rs + 1 == S::kScales ? 0 : rs + 1;
-          fetch();
           __syncwarp();
         }
-        const uint32_t slot = v % kSlots;
-        ok = mbar_wait_warp(&acc_full[v % (2 * kSlots)], (v / (2 * kSlots)) & 1u, &s_abort);
+        ok = mbar_wait_warp(&acc_full[at6], par6, &s_abort);
         if (!ok) break;
         tc_fence_after();
+        if (G == 32 && read_s >= 0) {   // scales that the last visit has used: handed back only now, an arrival can overtake loads
+          mbar_arrive_warp(&empty_s[read_s], lane);
+          read_s = -1;
+        }
+        float sc[NW][S::kGps];
+        constexpr uint32_t kPerUnit = 128 / S::kVk;   // visits per unit
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+          const uint32_t a = G == 32 ? sring + ((v / kPerUnit % S::kScales) * NW + (uint32_t)q) * kUnitScaleBytes + (v % kPerUnit) * (uint32_t)(S::kGps * 4)
+                                     : sring + rs * (256u * S::kScaleBytes) + (uint32_t)(q * S::kGps * 4);
+          if constexpr (S::kGps == 4)
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(sc[q][0]), "=f"(sc[q][1]), "=f"(sc[q][S::kGps - 2]), "=f"(sc[q][S::kGps - 1]) : "r"(a));
+          else if constexpr (S::kGps == 2) asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(sc[q][0]), "=f"(sc[q][S::kGps - 1]) : "r"(a));
+          else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc[q][0]) : "r"(a));
+        }
+        const uint32_t slot = at6 >= kSlots ? at6 - kSlots : at6;
         const uint32_t d = lane_base + 128u + slot * 128u;
         constexpr int kN16 = S::kGps * S::kCols / 16;          // 16-column loads of the visit
         constexpr int kBatch = S::kCols > 64 ? 2 : (kN16 < 4 ? kN16 : (kN16 % 4 == 0 ? 4 : 3));   // in flight at once
@@ -486,7 +469,6 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (b == kN16 / kBatch - 1) {   // the slot's sums are in registers: hand it back before the arithmetic
             tc_fence_before();
-            __syncwarp();
             mbar_arrive_warp(&acc_empty[slot], lane);
           }
 #pragma unroll
@@ -497,6 +479,15 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
             for (int e = 0; e < 16; e += 2) fma2(acc[at + e], acc[at + e + 1], r[i][e], r[i][e + 1], s);
           }
         }
+        if constexpr (G == 32) {
+          if (S::kGps > 1 || (v & 2u)) read_s = (int)(v / kPerUnit % S::kScales);   // this team's last look at the unit's scales
+        } else {
+          rs = rs + 1 == S::kScales ? 0 : rs + 1;
+          fetch();
+          __syncwarp();
+        }
+        at6 += 2;
+        if (at6 >= 2 * kSlots) { at6 -= 2 * kSlots; par6 ^= 1u; }
       }
       // ---- the teams' sums: each finishes half of the activation rows ----
       constexpr int kHalf = MP / 2;
@@ -675,9 +666,10 @@ constexpr Variant variant() {
 const Variant kVariants[] = {variant<16, 1>(), variant<32, 1>(), variant<48, 1>(), variant<64, 1>(),
                              variant<16, 2>(), variant<32, 2>(), variant<48, 2>(), variant<64, 2>()};
 
-// What a launch costs, in cycles of the busiest CTA: tiles one after the other, a stage of 64 elements being bound by the
-// tensor pipe (MP / 2 cycles per MMA and two more, at least 11), by the CTA's share of HBM (23 bytes per cycle and SM when
-// all of them stream, at most twice that when few do) or by the hand-overs.
+// What a launch costs, in microseconds of the busiest CTA, fitted to sweeps of every variant and split over 32 to 333 rows and
+// the projections of the 8B widths: a stage of 64 elements takes 0.25 + 0.003 MP (one weight tile) or 0.37 + 0.0068 MP (two)
+// with 32-element groups - the roles' instruction chains, not HBM or the tensor pipe (0.29 at 64 x 2) - and about 0.85 of
+// that with larger ones; a tile's end about 1, and 0.05 per accumulator column more where partial sums are added in memory.
 struct Plan { const Variant* v; int mtiles, ntiles, ksplit; };
 double plan_cost(const Variant& v, int m, int64_t n, int64_t k, int g, bool pair, int ks, int sms, Plan* plan) {
   const int rows = pair ? kTileN : kTileN * v.nw;
@@ -686,17 +678,8 @@ double plan_cost(const Variant& v, int m, int64_t n, int64_t k, int g, bool pair
   plan->ntiles = (int)((n + rows - 1) / rows);
   const int64_t tiles = (int64_t)plan->mtiles * plan->ntiles * ks;
   const int64_t waves = (tiles + sms - 1) / sms;
-  const int64_t active = tiles < sms ? tiles : sms;
-  const double mma = 8.0 * v.nw * (v.mp / 2 + 2 > 11 ? v.mp / 2 + 2 : 11);
-  double rate = 23.0 * (double)sms / (double)active;
-  if (rate > 46.0) rate = 46.0;
-  const double hbm = v.nw * kTileN * (32.0 + 256.0 / g) / rate / (plan->mtiles < 4 ? plan->mtiles : 4);
-  const double hand = 64.0 / g * (v.mp * v.nw) * 2.1 + 60.0;   // tensor memory is read at about 64 bytes per cycle and sub-partition
-  const double unpack = v.nw == 2 ? 200.0 : 110.0;
-  double stage = mma > hbm ? mma : hbm;
-  if (hand > stage) stage = hand;
-  if (unpack > stage) stage = unpack;
-  return (double)waves * ((double)(k / ks / kKC) * stage + 600.0 + 12.0 * v.mp * v.nw) + 4000.0;
+  const double stage = (v.nw == 2 ? 0.37 + 0.0068 * v.mp : 0.25 + 0.003 * v.mp) * (g > 32 ? 0.85 : 1.0);
+  return (double)waves * ((double)(k / ks / kKC) * stage + 1.0 + (ks > 1 ? 0.05 * v.mp * v.nw : 0.0)) + (ks > 1 ? 1.0 : 0.0);
 }
 Plan choose_plan(int m, int64_t n, int64_t k, int g, bool pair) {
   const int sms = sm_count();
@@ -706,7 +689,7 @@ Plan choose_plan(int m, int64_t n, int64_t k, int g, bool pair) {
     if (pair && v.nw != 2) continue;
     for (int ks = 1; ks <= 8; ++ks) {
       if (ks > 1 && (pair || (k / kUnit) % ks != 0)) continue;   // the SwiGLU needs whole sums: no split
-      const double c = plan_cost(v, m, n, k, g, pair, ks, sms, &cur) + (ks > 1 ? 1500.0 : 0.0);   // partial sums are added in memory
+      const double c = plan_cost(v, m, n, k, g, pair, ks, sms, &cur);
       if (c < best_cost) { best_cost = c; best = cur; }
     }
   }
