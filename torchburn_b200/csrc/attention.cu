@@ -5,9 +5,9 @@
 // rope_apply_head :28-68) and the wgpu shaders rope_append.wgsl / attn_decode.wgsl.
 //
 // The reference walks the sequence serially per q head with a two-pass softmax.
-// Here the positions [0, offset] of every (sequence, kv head) are divided evenly
-// among the CTAs of a grid row, whatever the current length, so that every SM
-// streams its share.  Inside a CTA one producer lane feeds a ring of shared-memory
+// Here the positions [0, offset] of every (sequence, kv head) are cut into shares
+// of one length over all sequences of the batch (plan_share), whatever the current
+// lengths, so that every SM streams as much.  Inside a CTA one producer lane feeds a ring of shared-memory
 // stages with bulk asynchronous copies (32 K rows + 32 V rows per stage, contiguous
 // in the [Hkv, S, d] cache) and the consumer warps score the rows for all q heads
 // that share the kv head, keep an online softmax and accumulate the weighted V -
@@ -38,6 +38,7 @@ constexpr int kMaxGq = 8;              // q heads per kv head
 constexpr int kMaxStages = 8;
 constexpr int kChunkRows = 512;        // positions whose scores are held in shared memory at a time
 constexpr size_t kCounterBytes = 16384;  // 4096 tickets: (sequence, kv head) pairs of a launch
+constexpr int kMaxParts = 48;          // shares of a sequence: more cost more in the merge than they save
 constexpr int kSeqCap = 32768;         // src/llm/decoder.rs:1180
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s: a wait that long means a lost copy
 
@@ -51,15 +52,15 @@ struct AttnParams {
   const float* sin_t;
   const int32_t* offsets;
   float* out;
-  float* part_o;    // [b, Hq, nc, D]
-  float* part_ml;   // [b, Hq, nc, 2]
+  float* part_o;    // [kv head, share, gq, D]: the shares of a (sequence, kv head) are one run
+  float* part_ml;   // [kv head, share, gq, 2]
   int* counters;    // [b, Hkv] tickets
   float* qkv_rot_out;
   int num_heads, num_kv_heads, gq;
   int fixed_per;    // positions per CTA when forced, else 0: divide the current length evenly
-  int nc;           // CTAs per (sequence, kv head) = gridDim.x
+  int batch;
+  int nc;           // most CTAs that share a (sequence, kv head)
   int stages;       // ring depth
-  int max_parts;    // upper bound of CTAs of a (sequence, kv head) that take positions
   int region_floats;  // floats of the ring region (also holds the combine / merge buffers)
   int64_t max_seq_len;
   int per_call_tables;
@@ -277,6 +278,80 @@ __device__ __forceinline__ void weigh_rows(const float* __restrict__ vb, int nr,
   }
 }
 
+// Which share of which sequence a CTA takes.  gridDim.x CTAs per kv head are laid over the sequences in order, `per`
+// positions each (the last share of a sequence is what remains): per is the smallest multiple of 32 with which the
+// grid suffices for the lengths at hand, so that a batch of unequal sequences keeps every SM busy to the end.  The
+// same number of CTAs for every sequence left the longest ones to the end: 32 sequences of 128 to 4096 positions, 8 kv heads
+// of 128, took 176 us where their bytes take 85.  Every warp works the plan out by itself from the offsets.
+struct Share { int b, split, parts, x0, per, len; };   // sequence, share of it, its shares, the first one's CTA; positions per share, of the sequence
+__device__ __forceinline__ Share plan_share(const AttnParams& p, int x, int lane) {
+  const int B = p.batch, X = (int)gridDim.x;
+  auto length = [&](int b) {
+    if (b >= B) return -1;
+    const int off = p.offsets[b];
+    return off >= 0 && (int64_t)off < p.max_seq_len ? min(off + 1, kSeqCap) : 0;
+  };
+  if (B == 1) {   // one sequence: divided evenly, no search
+    const int len = length(0);
+    int per = p.fixed_per;
+    if (per <= 0) per = max(kStageRows, ((len + X - 1) / X + kStageRows - 1) & ~(kStageRows - 1));
+    const int parts = max(1, (len + per - 1) / per);
+    return Share{x < parts ? 0 : -1, x, parts, 0, per, len};
+  }
+  const int len0 = length(lane), len1 = length(lane + 32);
+  auto len_of = [&](int b0) { return b0 == 0 ? len0 : (b0 == 32 ? len1 : length(b0 + lane)); };
+  int u = p.fixed_per / kStageRows;   // positions per share in units of a stage
+  if (u <= 0) {
+    int total = 0, longest = 0;
+    for (int b0 = 0; b0 < B; b0 += 32) {
+      const int t = max(len_of(b0), 0);
+      total += __reduce_add_sync(0xffffffffu, t);
+      longest = max(longest, __reduce_max_sync(0xffffffffu, t));
+    }
+    // at most nc shares of a sequence; X - B whole shares and one remainder per sequence always suffice
+    const int least = max((longest + p.nc - 1) / p.nc, 1);
+    int lo = max(total / X, least), hi = max(longest, 1);
+    if (X > B) hi = min(hi, max((total + X - B - 1) / (X - B), least));
+    lo = (lo + kStageRows - 1) / kStageRows;
+    hi = max((hi + kStageRows - 1) / kStageRows, lo);
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1, per = mid * kStageRows;
+      int n = 0;
+      for (int b0 = 0; b0 < B; b0 += 32) {
+        const int t = len_of(b0);
+        n += __reduce_add_sync(0xffffffffu, t < 0 ? 0 : max(1, (t + per - 1) / per));
+      }
+      if (n <= X) hi = mid;
+      else lo = mid + 1;
+    }
+    u = lo;
+  }
+  Share s{-1, 0, 0, 0, u * kStageRows, 0};
+  int before = 0;
+  for (int b0 = 0; b0 < B; b0 += 32) {
+    const int t = len_of(b0), parts = t < 0 ? 0 : max(1, (t + s.per - 1) / s.per);   // an empty sequence has a CTA that writes its zeros
+    int end = parts;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    const int first = before + end - parts;
+    const unsigned hit = __ballot_sync(0xffffffffu, x >= first && x < first + parts);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      s.b = b0 + src;
+      s.x0 = __shfl_sync(0xffffffffu, first, src);
+      s.parts = __shfl_sync(0xffffffffu, parts, src);
+      s.len = __shfl_sync(0xffffffffu, t, src);
+      s.split = x - s.x0;
+      return s;
+    }
+    before += __shfl_sync(0xffffffffu, end, 31);
+  }
+  return s;
+}
+
 // One CTA = one share of the positions of one (sequence, kv head).  The share is walked in
 // chunks of at most kChunkRows positions; for every chunk the producer lane streams the K
 // rows and then the V rows through the ring (32 rows per stage).  The consumer warps score the
@@ -313,7 +388,7 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
   float* S = kv_new + 2 * D;                             // [(kChunkRows + 1)][GQM]
   float* region = S + up4((size_t)(kChunkRows + 1) * GQM);
 
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int kvh = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int qkv_dim = (p.num_heads + 2 * p.num_kv_heads) * D;
 
@@ -342,16 +417,11 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
   // own wait, so everything older is complete when this code runs.  The plan and the whole
   // K/V stream therefore start while that kernel is still draining; only the q-dependent
   // work waits.
-  const int off = p.offsets[b];
-  const bool seq_ok = off >= 0 && (int64_t)off < p.max_seq_len;
-  const int t_end = seq_ok ? min(off + 1, kSeqCap) : 0;  // attend to [0, t_end)
-  int per = p.fixed_per;
-  if (per <= 0) {
-    const int parts = min(p.nc, p.max_parts);  // more partials than this cost more in the merge than they save
-    per = (t_end + parts - 1) / parts;
-    per = max(kStageRows, (per + kStageRows - 1) & ~(kStageRows - 1));
-  }
-  const int nvalid = (t_end + per - 1) / per;   // CTAs of this grid row that have positions
+  const Share sh = plan_share(p, (int)blockIdx.x, lane);
+  if (sh.b < 0) return;   // more CTAs than shares
+  const int b = sh.b, split = sh.split, per = sh.per, t_end = sh.len;   // attend to [0, t_end)
+  const int off = t_end - 1;   // (a sequence out of range has no positions; max_seq_len is at most kSeqCap)
+  const int nvalid = (t_end + per - 1) / per;   // shares of the sequence that have positions
   const int t0 = split * per;
   const bool active = t0 < t_end;
   const int rows = active ? min(per, t_end - t0) : 0;
@@ -581,10 +651,10 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
       float o = 0.f;
 #pragma unroll
       for (int w = 0; w < kCW; ++w) o += w_acc[((size_t)w * gq + g) * D + e];
-      const int h = kvh * gq + g;
-      p.part_o[(((int64_t)b * p.num_heads + h) * p.nc + split) * D + e] = o;
+      const int64_t at = ((int64_t)kvh * gridDim.x + blockIdx.x) * gq + g;
+      p.part_o[at * D + e] = o;
       if (e == 0) {
-        float* dst = p.part_ml + (((int64_t)b * p.num_heads + h) * p.nc + split) * 2;
+        float* dst = p.part_ml + at * 2;
         dst[0] = s_ml[0][g];
         dst[1] = s_ml[1][g];
       }
@@ -597,7 +667,7 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
   if (tid == 0) {
     if (s_abort) atomicExch(&g_attn_fault, 1);
     const int ticket = atomicAdd(&p.counters[b * p.num_kv_heads + kvh], 1);
-    s_last = (ticket == (int)gridDim.x - 1);
+    s_last = (ticket == sh.parts - 1);
   }
   consumer_barrier();
   if (tid == 0 && !s_last) tl_mark(p.tl, cta_lin, 5);
@@ -611,22 +681,20 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
     for (int i = tid; i < gq * D; i += kCT) p.out[((int64_t)b * p.num_heads + h0) * D + i] = 0.f;
     return;
   }
-  // Layout of the region now: wts [gq][nc] | ml [gq] | tile [gq][cc][D], cc partials at a time.
+  // Layout of the region now: wts [gq][nc] | ml [gq] | tile [cc][gq][D], cc partials at a time.
   float* wts = region;
   float* ml = wts + up4((size_t)gq * p.nc);
   float* tile = ml + up4(gq);
   const int cc = (int)min((int64_t)nvalid, (int64_t)(p.region_floats - (tile - region)) / ((int64_t)gq * D));
-  const float* po = p.part_o + ((int64_t)b * p.num_heads + h0) * p.nc * D;
+  const int64_t run = ((int64_t)kvh * gridDim.x + sh.x0) * gq;
+  const float* po = p.part_o + run * D;
+  const float* pm = p.part_ml + run * 2;
   // Request the first tile of partials (asynchronous copies, no registers held) before the
   // weights are worked out, so that both trips to L2 overlap.
   auto request_tile = [&](int c0, int n) {
-    for (int i = tid; i < gq * n * CPR; i += kCT) {
-      const int g = i / (n * CPR), r = i - g * (n * CPR);  // r = chunk-in-tile * CPR + column
-      const float* src = po + ((int64_t)g * p.nc + c0) * D + (int64_t)r * 4;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tile + ((size_t)g * cc) * D + (size_t)r * 4)),
-                   "l"(src)
-                   : "memory");
-    }
+    const float* src = po + (int64_t)c0 * gq * D;
+    for (int i = tid; i < gq * n * CPR; i += kCT)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tile + (size_t)i * 4)), "l"(src + (int64_t)i * 4) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // The (max, sum) pairs are requested first - they gate the weights - then the tile.
@@ -637,7 +705,7 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
     for (int k = 0; k < 2; ++k) {
       const int g = warp + hs * kCW, c = lane + 32 * k;
       mlv[hs][k] = (g < gq && c < nvalid)
-                       ? __ldcg(reinterpret_cast<const float2*>(p.part_ml + (((int64_t)b * p.num_heads + h0 + g) * p.nc + c) * 2))
+                       ? __ldcg(reinterpret_cast<const float2*>(pm + (c * gq + g) * 2))
                        : make_float2(-INFINITY, 0.f);
     }
   request_tile(0, min(cc, nvalid));
@@ -646,9 +714,10 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
   for (int hs = 0; hs < 2; ++hs) {
     const int g = warp + hs * kCW;
     if (g >= gq) continue;
-    const float* pml = p.part_ml + ((int64_t)b * p.num_heads + h0 + g) * p.nc * 2;
+    const float* pml = pm + g * 2;
+    const int step = 2 * gq;
     float mx = fmaxf(mlv[hs][0].x, mlv[hs][1].x);
-    for (int c = lane + 64; c < nvalid; c += 32) mx = fmaxf(mx, __ldcg(pml + c * 2));
+    for (int c = lane + 64; c < nvalid; c += 32) mx = fmaxf(mx, __ldcg(pml + c * step));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     float tot = 0.f;
@@ -662,9 +731,9 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
       }
     }
     for (int c = lane + 64; c < nvalid; c += 32) {
-      const float w = expf(__ldcg(pml + c * 2) - mx);
+      const float w = expf(__ldcg(pml + c * step) - mx);
       wts[g * p.nc + c] = w;
-      tot = fmaf(__ldcg(pml + c * 2 + 1), w, tot);
+      tot = fmaf(__ldcg(pml + c * step + 1), w, tot);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
@@ -685,10 +754,10 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
       const int o = tid + k * kCT;
       if (o < gq * CPR) {
         const int g = o / CPR, col = o - g * CPR;
-        const float4* t4 = reinterpret_cast<const float4*>(tile + ((size_t)g * cc) * D) + col;
+        const float4* t4 = reinterpret_cast<const float4*>(tile) + g * CPR + col;   // share after share
         const float* w = wts + g * p.nc + c0;
         for (int c = 0; c < n; ++c) {
-          const float4 v = t4[c * CPR];
+          const float4 v = t4[c * gq * CPR];
           const float wc = w[c];
           acc[k].x = fmaf(wc, v.x, acc[k].x);
           acc[k].y = fmaf(wc, v.y, acc[k].y);
@@ -720,8 +789,9 @@ int g_ctas_per_sm = 0;   // 0 = automatic (2)
 int g_ring_stages = 0;   // 0 = automatic
 
 struct AttnLayout {
-  int fixed_per;  // 0 = divide the current length evenly among the nc CTAs
-  int nc;         // CTAs per (sequence, kv head)
+  int fixed_per;  // 0 = shares by the lengths at hand (plan_share)
+  int grid;       // CTAs per kv head
+  int nc;         // most of them that share a sequence
   int stages;
   size_t part_o, part_ml;
 };
@@ -735,7 +805,6 @@ int max_splits(int64_t max_seq_len) {
 AttnLayout attn_layout(int batch, int num_heads, int num_kv_heads, int head_dim, int64_t max_seq_len) {
   AttnLayout L;
   const int64_t cap = max_seq_len < kSeqCap ? max_seq_len : kSeqCap;
-  const int64_t cols = (int64_t)batch * num_kv_heads;
   // Ring depth: 96 KB of stages for head_dim 128 (two CTAs per SM), fewer bytes for narrower heads.
   const int cps = g_ctas_per_sm > 0 ? g_ctas_per_sm : 2;
   L.stages = head_dim == 128 ? 6 : 8;
@@ -745,18 +814,24 @@ AttnLayout attn_layout(int batch, int num_heads, int num_kv_heads, int head_dim,
   if (g_chunk_override > 0) {
     L.fixed_per = g_chunk_override;
     L.nc = (int)((cap + L.fixed_per - 1) / L.fixed_per);
+    L.grid = batch * L.nc;
   } else {
-    // two resident CTAs per SM, all of them busy whatever the current length
+    // Two resident CTAs per SM, all of them busy whatever the current lengths.  With many sequences their remainders
+    // would make a share as long as a sequence: then several rounds of CTAs, four shares per sequence on average.
     L.fixed_per = 0;
-    int64_t nc = ((int64_t)cps * sm_count()) / cols;
-    const int64_t most = (cap + kStageRows - 1) / kStageRows;
-    if (nc > most) nc = most;
-    if (nc < 1) nc = 1;
-    L.nc = (int)nc;
+    int64_t slots = ((int64_t)cps * sm_count()) / num_kv_heads;
+    if (slots < 1) slots = 1;
+    int64_t x = batch == 1 ? slots : slots * ((4ll * batch + slots - 1) / slots);
+    const int64_t most = (int64_t)batch * ((cap + kStageRows - 1) / kStageRows);
+    if (batch == 1 && x > kMaxParts) x = kMaxParts;
+    if (x > most) x = most;
+    if (x < batch) x = batch;
+    L.grid = (int)x;
+    L.nc = (int)(x < kMaxParts ? x : kMaxParts);
   }
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  L.part_o = up((size_t)batch * num_heads * L.nc * head_dim * sizeof(float));
-  L.part_ml = up((size_t)batch * num_heads * L.nc * 2 * sizeof(float));
+  L.part_o = up((size_t)L.grid * num_heads * head_dim * sizeof(float));
+  L.part_ml = up((size_t)L.grid * num_heads * 2 * sizeof(float));
   return L;
 }
 
@@ -861,7 +936,7 @@ tb_status launch_attention_decode(const AttnArgs& a, cudaStream_t stream) {
   AttnLayout L = attn_layout(a.batch, a.num_heads, a.num_kv_heads, a.head_dim, a.max_seq_len);
   if (L.fixed_per && (L.fixed_per < 64 || L.fixed_per > 512 || (L.fixed_per & (L.fixed_per - 1))))
     return fail(TB_ERR_ARG, "attention: chunk %d is not a power of two in [64, 512]", L.fixed_per);
-  if (L.nc > max_splits(a.max_seq_len)) return fail(TB_ERR_SHAPE, "attention: %d splits exceed the scratch layout", L.nc);
+  if ((int64_t)L.grid > (int64_t)a.batch * max_splits(a.max_seq_len)) return fail(TB_ERR_SHAPE, "attention: %d shares exceed the scratch layout", L.grid);
   size_t cbytes = 0;
   const size_t coff = attention_counters_offset(a.batch, a.num_heads, a.num_kv_heads, a.head_dim, a.max_seq_len, &cbytes);
   const int gqm = gq <= 1 ? 1 : (gq <= 2 ? 2 : (gq <= 4 ? 4 : 8));
@@ -877,8 +952,7 @@ tb_status launch_attention_decode(const AttnArgs& a, cudaStream_t stream) {
   p.part_ml = reinterpret_cast<float*>(base + coff + cbytes + L.part_o);
   p.qkv_rot_out = a.q_rot_out;
   p.num_heads = a.num_heads; p.num_kv_heads = a.num_kv_heads; p.gq = gq;
-  p.fixed_per = L.fixed_per; p.nc = L.nc; p.stages = L.stages;
-  p.max_parts = 48;
+  p.fixed_per = L.fixed_per; p.batch = a.batch; p.nc = L.nc; p.stages = L.stages;
   // two CTAs per SM when the ring can be cut to make room (wide heads with many q heads per kv head)
   int stages = L.stages;
   while (stages > 3 && 2 * (sizeof(float) * (attn_fixed_floats(D, gq, gqm) + attn_region_floats(D, gq, L.nc, stages)) + 2048) > 227 * 1024)
@@ -895,7 +969,7 @@ tb_status launch_attention_decode(const AttnArgs& a, cudaStream_t stream) {
   const size_t smem = sizeof(float) * (attn_fixed_floats(D, gq, gqm) + region);
   if (smem > 200 * 1024) return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: attention needs %zu bytes of shared memory", smem);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)L.nc, (unsigned)a.num_kv_heads, (unsigned)a.batch);
+  cfg.gridDim = dim3((unsigned)L.grid, (unsigned)a.num_kv_heads);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
