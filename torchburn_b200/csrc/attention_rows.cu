@@ -34,6 +34,14 @@ struct RowsParams {
   float scale;
 };
 
+// Two fp32 fused multiply-adds in one issue slot: a += x * y.
+__device__ __forceinline__ void fma2(float2& a, float x0, float x1, float y0, float y1) {
+  asm("{\n\t.reg .b64 a, x, y;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "fma.rn.f32x2 a, x, y, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(a.x), "+f"(a.y)
+      : "f"(x0), "f"(x1), "f"(y0), "f"(y1));
+}
+
 template <int D>
 constexpr int kStride = D + 4;   // floats per row of Q, K and V in shared memory: rows fall on different banks
 constexpr int kPStride = kKeys + 4;
@@ -102,7 +110,9 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
 
   constexpr int kC = D / 64 > 0 ? D / 64 : 1;      // column blocks of a thread, 64 apart
   constexpr int kW = D >= 64 ? 4 : D / 16;         // columns of a block (D = 32: 2)
-  float o[4][kC * kW], m_run[4], l_run[4];
+  constexpr int kO = kC * kW / 2;
+  float2 o[4][kO];
+  float m_run[4], l_run[4];
   int lm[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -110,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
     l_run[i] = 0.f;
     lm[i] = lim[ty * 4 + i];
 #pragma unroll
-    for (int c = 0; c < kC * kW; ++c) o[i][c] = 0.f;
+    for (int c = 0; c < kO; ++c) o[i][c] = make_float2(0.f, 0.f);
   }
   if (tile0 < tile1) {
     copy(ks, kc, tile0 * kKeys);
@@ -121,11 +131,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
     // ---- scores: pairs 4 ty + i, keys tx + 16 j ----
-    float s[4][4];
+    float2 s2[4][4];   // sums over even and odd d
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+      for (int j = 0; j < 4; ++j) s2[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 4
     for (int d = 0; d < D; d += 4) {
       float4 q[4], k[4];
@@ -136,15 +146,20 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          s[i][j] = fmaf(q[i].x, k[j].x, s[i][j]);
-          s[i][j] = fmaf(q[i].y, k[j].y, s[i][j]);
-          s[i][j] = fmaf(q[i].z, k[j].z, s[i][j]);
-          s[i][j] = fmaf(q[i].w, k[j].w, s[i][j]);
-        }
+        for (int j = 0; j < 4; ++j) fma2(s2[i][j], q[i].x, q[i].y, k[j].x, k[j].y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) fma2(s2[i][j], q[i].z, q[i].w, k[j].z, k[j].w);
     }
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = s2[i][j].x + s2[i][j].y;
     __syncthreads();   // the keys have been read: their place takes the weights
     const bool whole = t0 + kKeys <= t_all;
+    float resc[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float mx = -INFINITY;
@@ -156,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
 #pragma unroll
       for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
       const float m_new = fmaxf(m_run[i], mx), base = m_new == -INFINITY ? 0.f : m_new;
-      const float resc = expf(m_run[i] - base);
+      resc[i] = expf(m_run[i] - base);
       m_run[i] = m_new;
       float sum = 0.f;
 #pragma unroll
@@ -167,14 +182,17 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
       }
 #pragma unroll
       for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
-      l_run[i] = l_run[i] * resc + sum;
-#pragma unroll
-      for (int c = 0; c < kC * kW; ++c) o[i][c] *= resc;
+      l_run[i] = l_run[i] * resc[i] + sum;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     // ---- weights times values: columns 64 c + kW tx + w ----
     const int keys = min(kKeys, t_end - t0);
+    float2 ot[4][kO];   // of this tile alone: short sums, added to the running ones once
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < kO; ++c) ot[i][c] = make_float2(0.f, 0.f);
 #pragma unroll 2
     for (int k0 = 0; k0 < kKeys; k0 += 4) {
       float4 w[4];
@@ -199,12 +217,19 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
           const float wi = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
           if (whole || t0 + k0 + kk < lm[i]) {   // a later position's values, whatever they are, do not touch this pair
 #pragma unroll
-            for (int c = 0; c < kC * kW; ++c) o[i][c] = fmaf(wi, v[c], o[i][c]);
+            for (int c = 0; c < kO; ++c) fma2(ot[i][c], wi, wi, v[2 * c], v[2 * c + 1]);
           }
         }
       }
       if (k0 + 4 >= keys) break;
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < kO; ++c) {
+        o[i][c].x = fmaf(o[i][c].x, resc[i], ot[i][c].x);
+        o[i][c].y = fmaf(o[i][c].y, resc[i], ot[i][c].y);
+      }
     __syncthreads();   // weights and values have been read
     if (t + 1 < tile1) {
       copy(ks, kc, t0 + kKeys);
@@ -229,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const RowsParams
 #pragma unroll
     for (int c = 0; c < kC; ++c)
 #pragma unroll
-      for (int w = 0; w < kW; ++w) dst[64 * c + kW * tx + w] = o[i][c * kW + w] * f;
+      for (int w = 0; w < kW; ++w) dst[64 * c + kW * tx + w] = ((w & 1) ? o[i][(c * kW + w) / 2].y : o[i][(c * kW + w) / 2].x) * f;
   }
 }
 
@@ -259,13 +284,14 @@ __global__ void __launch_bounds__(256) attn_rows_merge_kernel(const float* __res
 
 constexpr int kMaxSplits = 8;
 
-// Splits of the keys: the fewest waves of two blocks per SM times tiles per block (and about two tiles' worth of start-up).
+// Splits of the keys: the fewest rounds of one block per SM (two share its FMA pipe) times tiles per block, start-up and
+// merge being worth about a tile and a half.
 int choose_splits(int blocks, int64_t keys) {
-  const int64_t tiles = (keys + kKeys - 1) / kKeys, slots = 2ll * sm_count();
+  const int64_t tiles = (keys + kKeys - 1) / kKeys, slots = sm_count();
   int best = 1;
   int64_t best_cost = INT64_MAX;
   for (int s = 1; s <= kMaxSplits && s <= tiles; ++s) {
-    const int64_t cost = ((int64_t)blocks * s + slots - 1) / slots * ((tiles + s - 1) / s + 2) + (s > 1 ? 1 : 0);
+    const int64_t cost = ((int64_t)blocks * s + slots - 1) / slots * (2 * ((tiles + s - 1) / s) + 3) + (s > 1 ? 2 : 0);
     if (cost < best_cost) { best_cost = cost; best = s; }
   }
   return best;
