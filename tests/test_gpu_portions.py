@@ -199,3 +199,31 @@ def test_feed_forward_calls_of_several_threads(torch, tb):
     work(9, shared)
     torch.cuda.synchronize()
     assert not bad
+
+
+@pytest.mark.parametrize("rows,width,ff,latent", [(300, 256, 9000, False), (600, 128, 19001, False), (260, 320, 9728, True)])
+def test_wide_products_of_long_portions(torch, tb, rows, width, ff, latent):
+    """Portions whose products take several waves of 256-row tiles (pairs of CTAs): odd and even numbers of weight tiles, row
+    counts around a tile, K from two blocks up; against the same prompt in portions of 100 rows (single CTAs).  bfloat16
+    activations: 3e-2 of the logits' spread, as everywhere for two orders of the same sums in 16 bits."""
+    gen = torch.Generator("cuda").manual_seed(rows)
+    bf = lambda *s, std=0.05: (torch.randn(*s, device="cuda", generator=gen) * std).to(torch.bfloat16)
+    heads, dim, vocab = 4, 32, 700
+    w = dict(norm1=bf(width), norm2=bf(width), up_w=bf(ff, width), down_w=bf(width, ff, std=0.01), o_w=bf(width, heads * dim))
+    if latent:
+        w.update(dq_w=bf(64, width), dq_norm=1 + bf(64), uq_w=bf(heads * (dim + 16), 64), dkv_w=bf(64 + 16, width), dkv_norm=1 + bf(64), uk_w=bf(heads * dim, 64),
+                 uv_w=bf(heads * dim, 64))
+        spec = tb.LayerSpec(heads, 1, dim, dim, (dim + 16) ** -0.5, q_rank=64, kv_rank=64, rot_dim=16, rot_dims=16, rot_base=10000.0, ff=ff, activation="relu2", tensors=w)
+    else:
+        w.update(q_w=bf(heads * dim, width), k_w=bf(2 * dim, width), v_w=bf(2 * dim, width))
+        spec = tb.LayerSpec(heads, 2, dim, dim, dim ** -0.5, ff=ff, activation="relu2", tensors=w)
+    embed, norm, head = bf(vocab, width, std=1.0), bf(width), bf(vocab, width)
+    ids = torch.randint(vocab, (rows,), generator=torch.Generator().manual_seed(1)).tolist()
+    got = []
+    for portion in (1024, 100):
+        dec = tb.LayeredDecoder([spec, spec], embed, norm, head=head, hidden_size=width, vocab_size=vocab, norm_eps=1e-6, norm_offset=1.0,
+                                max_seq_len=rows + 8, max_batch=1, prefill_rows=portion)
+        got.append(dec.extend(ids, 0, want=[0, rows // 2, rows - 1]))
+    assert np.isfinite(got[0]).all()
+    err = np.sqrt(((got[0] - got[1]) ** 2).mean(1)) / got[1].std(1)
+    assert err.max() < 3e-2, err

@@ -6,7 +6,7 @@
 // warps read the fp32 accumulator back (thread = output feature, so a store is 32 consecutive floats).
 // From one decode row to a whole prompt portion it is the same kernel: with few rows it streams the
 // weights (several CTAs per SM, K split over CTAs when there are fewer tiles than SMs), with many rows it
-// is bound by the tensor core.  A K split writes partial sums which the consuming row kernel adds in a
+// is bound by the tensor core; launches of several waves of wide tiles go to persistent pairs of CTAs.  A K split writes partial sums which the consuming row kernel adds in a
 // fixed order; without one the epilogue can also write the next kernel's input itself (rows of the activation
 // type, or an activated operand image).  A batch of matrices (one per head) is one launch.  The weight copies of the first stages are issued before the grid dependency wait: weights
 // depend on nothing, so with programmatic launch they overlap the previous kernel's tail.
@@ -23,7 +23,6 @@ using namespace tc5;
 
 constexpr int kTile = 128;            // output features per CTA
 constexpr int kTileBytes = 16384;     // 128 rows x 64 bf16
-constexpr int kShortLoop = 16;        // K blocks
 
 __device__ int g_dense_fault = 0;
 
@@ -53,6 +52,56 @@ __device__ __forceinline__ void store_sum(const GemmParams& p, int row, int64_t 
   if (p.sink == DenseSink::kOperand) act_store1<BF16>(p.operand, row, (int)col, v);
   else if (BF16) static_cast<__nv_bfloat16*>(p.out)[(size_t)row * p.ldo + col] = __float2bfloat16_rn(v);
   else static_cast<float*>(p.out)[(size_t)row * p.ldo + col] = v;
+}
+
+// The sums of a 128 x BN tile, from tensor memory to where they go; a warp's lane = output feature, columns = activation rows.
+// `smem`: 1280 bytes per warp that nothing else uses at the time.
+template <int BN>
+__device__ __forceinline__ void store_tile(const GemmParams& p, unsigned char* smem, uint32_t tmem, int warp, int lane, int tile, int row0, int split, int batch) {
+        tc_fence_after();
+        const int64_t n = (int64_t)tile * kTile + warp * 32 + lane;
+        const bool live = n < p.n_valid;
+        const uint32_t base = tmem + ((uint32_t)(warp * 32) << 16);
+        float* dst = static_cast<float*>(p.out) + (size_t)split * p.split_stride + (size_t)row0 * p.ldo + n;
+        const int64_t col = (int64_t)batch * p.batch_cols + n;
+        const int nrows = min(p.rows - row0, BN);
+        // eight features of a row lie side by side, on a 16-byte boundary
+        const bool wide = p.sink != DenseSink::kPartials && ((p.n_valid | p.batch_cols | (p.sink == DenseSink::kRows ? p.ldo : 0)) & 7) == 0;
+  #pragma unroll 1
+        for (int c = 0; c < nrows; c += 16) {
+          uint32_t r[2][8];
+          tmem_ld8(base + (uint32_t)c, r[0]);
+          tmem_ld8(base + (uint32_t)c + 8, r[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (live && p.sink == DenseSink::kPartials) {
+  #pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (c + j < nrows) dst[(size_t)(c + j) * p.ldo] = __uint_as_float(r[j >> 3][j & 7]);
+          } else if (wide) {
+            // through the warp's corner of the first stage (every MMA has read it): 16 rows x 32 features, then 8 features
+            // per store
+            __nv_bfloat16* t = reinterpret_cast<__nv_bfloat16*>(smem) + warp * (16 * 40);
+  #pragma unroll
+            for (int j = 0; j < 16; ++j) t[j * 40 + lane] = __float2bfloat16_rn(activate(p.act, __uint_as_float(r[j >> 3][j & 7])));
+            __syncwarp();
+  #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int j = (lane >> 2) + h * 8, f = (lane & 3) * 8;
+              if (c + j < nrows && n - lane + f < p.n_valid) {
+                const uint4 v = *reinterpret_cast<const uint4*>(t + j * 40 + f);
+                const int64_t k = col - lane + f;
+                if (p.sink == DenseSink::kOperand)
+                  *reinterpret_cast<uint4*>(static_cast<unsigned char*>(p.operand.data) + image_offset(p.operand.mp, row0 + c + j, (int)k)) = v;
+                else *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out) + (size_t)(row0 + c + j) * p.ldo + k) = v;
+              }
+            }
+            __syncwarp();
+          } else if (live) {
+  #pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (c + j < nrows) store_sum<true>(p, row0 + c + j, col, __uint_as_float(r[j >> 3][j & 7]));
+          }
+        }
 }
 
 template <int BN, int STAGES>
@@ -141,58 +190,196 @@ __global__ void __launch_bounds__(192) dense_tc5_kernel(const GemmParams p) {
     if (lane == 0) ok = mbar_wait(&done, 0u, &s_abort, &g_dense_fault);
     __syncwarp();
     ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-    if (ok) {
-      tc_fence_after();
-      const int64_t n = (int64_t)blockIdx.y * kTile + warp * 32 + lane;
-      const bool live = n < p.n_valid;
-      const uint32_t base = tmem + ((uint32_t)(warp * 32) << 16);
-      float* dst = static_cast<float*>(p.out) + (size_t)split * p.split_stride + (size_t)row0 * p.ldo + n;
-      const int64_t col = (int64_t)batch * p.batch_cols + n;
-      const int nrows = min(p.rows - row0, BN);
-      // eight features of a row lie side by side, on a 16-byte boundary
-      const bool wide = p.sink != DenseSink::kPartials && ((p.n_valid | p.batch_cols | (p.sink == DenseSink::kRows ? p.ldo : 0)) & 7) == 0;
-#pragma unroll 1
-      for (int c = 0; c < nrows; c += 16) {
-        uint32_t r[2][8];
-        tmem_ld8(base + (uint32_t)c, r[0]);
-        tmem_ld8(base + (uint32_t)c + 8, r[1]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (live && p.sink == DenseSink::kPartials) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (c + j < nrows) dst[(size_t)(c + j) * p.ldo] = __uint_as_float(r[j >> 3][j & 7]);
-        } else if (wide) {
-          // through the warp's corner of the first stage (every MMA has read it): 16 rows x 32 features, then 8 features
-          // per store
-          __nv_bfloat16* t = reinterpret_cast<__nv_bfloat16*>(smem) + warp * (16 * 40);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) t[j * 40 + lane] = __float2bfloat16_rn(activate(p.act, __uint_as_float(r[j >> 3][j & 7])));
-          __syncwarp();
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int j = (lane >> 2) + h * 8, f = (lane & 3) * 8;
-            if (c + j < nrows && n - lane + f < p.n_valid) {
-              const uint4 v = *reinterpret_cast<const uint4*>(t + j * 40 + f);
-              const int64_t k = col - lane + f;
-              if (p.sink == DenseSink::kOperand)
-                *reinterpret_cast<uint4*>(static_cast<unsigned char*>(p.operand.data) + image_offset(p.operand.mp, row0 + c + j, (int)k)) = v;
-              else *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out) + (size_t)(row0 + c + j) * p.ldo + k) = v;
-            }
-          }
-          __syncwarp();
-        } else if (live) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (c + j < nrows) store_sum<true>(p, row0 + c + j, col, __uint_as_float(r[j >> 3][j & 7]));
-        }
-      }
-    }
+    if (ok) store_tile<BN>(p, smem, tmem, warp, lane, (int)blockIdx.y, row0, split, batch);
     tc_fence_before();
   }
   __syncthreads();
   if (warp == 5) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+  }
+}
+
+// Two CTAs of a cluster on 256 x 256 tiles (cta_group::2): each holds 128 of the weight rows and 128 of the activation
+// rows of a stage in its shared memory and a 128 x 256 half of the sums in its tensor memory; one thread of the first CTA
+// issues the MMAs for both.  The second CTA tells the first that its copies have landed by a remote arrival.  A stage is
+// 32 KB per CTA instead of 48, so six fit: the loads' latency, not their rate, bounds the loop (0.40 us a stage with four
+// stages of 48 KB, 0.35 with these; two CTAs per SM with two stages each: slower still).
+// The pairs are persistent and tensor memory holds two tiles' sums: what a tile costs besides its stages (about 11 us of
+// start and stores, a third of a launch of several waves) lies under the next tile's stages.
+constexpr int kPairStages = 6, kPairStage = 2 * kTileBytes;
+
+__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 ad, bd;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 ad, {%1, %3};\n\t"
+      "mov.b64 bd, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], ad, bd, %4, p;\n\t"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(acc)
+      : "memory");
+}
+// Arrives on the barrier at this offset in both CTAs once every MMA issued so far has finished.
+constexpr int kPairStaging = 4 * 16 * 40 * 2;   // store_tile's corner per warp
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void arrive_first(uint64_t* bar) {   // on the first CTA's barrier
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A tile of a pair: block of 256 rows (fastest: the blocks of a pair of weight tiles run side by side, so that its weights
+// leave HBM once), pair of weight tiles, split and matrix.
+struct PairTile {
+  int row0, tile, split, batch, kb0, nkb;
+  __device__ __forceinline__ PairTile(const GemmParams& p, int pairs, int rank, int t) {
+    const int blocks = p.mp / 256, z = t / (blocks * pairs);
+    row0 = t % blocks * 256;
+    tile = t / blocks % pairs * 2 + rank;
+    split = z % p.splits;
+    batch = z / p.splits;
+    kb0 = split * p.kb_per;
+    nkb = min(p.kb - kb0, p.kb_per);
+  }
+};
+
+__global__ void __launch_bounds__(192, 1) dense_pair_kernel(const GemmParams p, const int n_tiles, const int total) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full[kPairStages], peer[kPairStages], empty[kPairStages], sums_full[2], sums_empty[2], done;
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_abort;
+  constexpr int BN = 256;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int rank = (int)blockIdx.x & 1, first = (int)blockIdx.x >> 1, step = (int)gridDim.x >> 1, pairs = (n_tiles + 1) / 2;
+
+  if (tid == 0) {
+    s_abort = 0;
+    for (int s = 0; s < kPairStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&peer[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&sums_full[s], 1);
+      mbar_init(&sums_empty[s], 8);   // (the first CTA's) four warps of each CTA
+    }
+    mbar_init(&done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(2 * BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // both CTAs' barriers stand before anyone arrives on them
+  tc_fence_after();
+  grid_dep_launch();
+  const uint32_t tmem = s_tmem;
+
+  if (warp == 4) {
+    if (elect_one()) {   // ---- copies: this CTA's 128 weight rows and its 128 of the 256 activation rows ----
+      int i = 0;   // stages so far, of all tiles
+      bool ok = true;
+      for (int t = first; t < total && ok; t += step) {
+        const PairTile q(p, pairs, rank, t);
+        const int src_tile = q.tile < n_tiles ? q.tile : n_tiles - 1;   // an odd last tile has no partner: its rows are not stored
+        const unsigned char* wsrc = p.w + (size_t)q.batch * p.w_batch + ((size_t)src_tile * p.kb + q.kb0) * kTileBytes;
+        const unsigned char* xsrc = p.x + (size_t)q.batch * p.x_batch + (size_t)q.kb0 * ((size_t)p.mp * 128) + (size_t)(q.row0 + rank * 128) * 128;
+        int pre = 0;
+        if (i == 0) {   // the weights of the first stages depend on nothing
+          pre = q.nkb < kPairStages ? q.nkb : kPairStages;
+          for (int j = 0; j < pre; ++j) {
+            mbar_expect_tx(&full[j], kPairStage);
+            bulk_g2s(smem + (size_t)j * kPairStage, wsrc + (size_t)j * kTileBytes, kTileBytes, &full[j]);
+          }
+          grid_dep_wait();
+          for (int j = 0; j < pre; ++j)
+            bulk_g2s(smem + (size_t)j * kPairStage + kTileBytes, xsrc + (size_t)j * ((size_t)p.mp * 128), kTileBytes, &full[j]);
+          i = pre;
+        }
+        for (int j = pre; j < q.nkb; ++j, ++i) {
+          const int s = i % kPairStages;
+          if (i >= kPairStages) ok = mbar_wait(&empty[s], (uint32_t)(i / kPairStages - 1) & 1u, &s_abort, &g_dense_fault);
+          if (!ok) break;
+          mbar_expect_tx(&full[s], kPairStage);
+          bulk_g2s(smem + (size_t)s * kPairStage, wsrc + (size_t)j * kTileBytes, kTileBytes, &full[s]);
+          bulk_g2s(smem + (size_t)s * kPairStage + kTileBytes, xsrc + (size_t)j * ((size_t)p.mp * 128), kTileBytes, &full[s]);
+        }
+      }
+      // copies in flight must have landed before the CTA gives its shared memory back
+      for (int j = i > kPairStages ? i - kPairStages : 0; j < i; ++j) {
+        int no_abort = 0;
+        mbar_wait(&full[j % kPairStages], (uint32_t)(j / kPairStages) & 1u, &no_abort, &g_dense_fault);
+      }
+    }
+  } else if (warp == 5) {
+    if (elect_one()) {
+      // fp32 accumulator, bf16 x bf16, both K-major, N = 256, M = 256
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * kTile >> 4) << 24);
+      int i = 0, n = 0;   // stages and tiles so far
+      bool ok = true;
+      for (int t = first; t < total && ok; t += step, ++n) {
+        const PairTile q(p, pairs, rank, t);
+        const uint32_t d = tmem + (uint32_t)((n & 1) * BN);
+        if (rank == 0 && n >= 2) {   // both CTAs have stored what lies there
+          ok = mbar_wait(&sums_empty[n & 1], (uint32_t)(n / 2 - 1) & 1u, &s_abort, &g_dense_fault);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        for (int j = 0; j < q.nkb; ++j, ++i) {
+          const int s = i % kPairStages;
+          const uint32_t par = (uint32_t)(i / kPairStages) & 1u;
+          ok = mbar_wait(&full[s], par, &s_abort, &g_dense_fault);
+          if (!ok) break;
+          if (rank != 0) {
+            arrive_first(&peer[s]);
+            continue;
+          }
+          // ---- MMA issue for both CTAs ----
+          ok = mbar_wait(&peer[s], par, &s_abort, &g_dense_fault);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t a_lo = (smem_u32(smem + (size_t)s * kPairStage) >> 4) | (1u << 16);
+          const uint32_t b_lo = (smem_u32(smem + (size_t)s * kPairStage + kTileBytes) >> 4) | (1u << 16);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)   // 16 bf16 = 32 bytes of a row per MMA
+            mma_bf16_pair(d, a_lo + (uint32_t)(ks * 2), b_lo + (uint32_t)(ks * 2), idesc, (j | ks) != 0 ? 1u : 0u);
+          commit_pair(&empty[s]);
+        }
+        if (rank == 0 && ok) commit_pair(&sums_full[n & 1]);
+      }
+      if (rank == 0) commit_pair(&done);
+      int no_abort = 0;
+      mbar_wait(&done, 0u, &no_abort, &g_dense_fault);
+    }
+  } else {
+    int n = 0;
+    for (int t = first; t < total; t += step, ++n) {
+      const PairTile q(p, pairs, rank, t);
+      bool ok = true;
+      if (lane == 0) ok = mbar_wait(&sums_full[n & 1], (uint32_t)(n / 2) & 1u, &s_abort, &g_dense_fault);
+      __syncwarp();
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      if (!ok) break;
+      store_tile<BN>(p, smem + (size_t)kPairStages * kPairStage, tmem + (uint32_t)((n & 1) * BN), warp, lane, q.tile, q.row0, q.split, q.batch);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive_first(&sums_empty[n & 1]);
+    }
+  }
+  __syncthreads();
+  cluster_sync();   // neither CTA's memory goes away under the other
+  if (warp == 5) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
   }
 }
 
@@ -292,6 +479,12 @@ tb_status launch_tc5(const GemmParams& p, int n_tiles, unsigned nz, bool pdl, cu
                        smem, st, pdl, 1, p);
 }
 
+tb_status launch_pair(const GemmParams& p, int n_tiles, unsigned nz, bool pdl, cudaStream_t st) {
+  const int total = (n_tiles + 1) / 2 * (p.mp / 256) * (int)nz, slots = sm_count() / 2;
+  return launch_kernel(dense_pair_kernel, dim3((unsigned)(2 * (total < slots ? total : slots))), dim3(192),
+                       (size_t)kPairStages * kPairStage + kPairStaging + 1024, st, pdl, 2, p, n_tiles, total);
+}
+
 }  // namespace
 
 int dense_fault_flag() {
@@ -382,8 +575,10 @@ tb_status launch_dense_gemm(Precision prec, const DenseGemmArgs& a, cudaStream_t
     case 64: return launch_tc5<64, 4>(p, n_tiles, nz, a.pdl, st);
     case 128: return launch_tc5<128, 6>(p, n_tiles, nz, a.pdl, st);
     default:
-      // a short K loop is mostly epilogue: two CTAs per SM, one stores while the other computes
-      if (p.kb_per <= kShortLoop && (int64_t)(p.mp / 256) * n_tiles * nz > sm_count()) return launch_tc5<256, 2>(p, n_tiles, nz, a.pdl, st);
+      // Several waves, or a long K loop: pairs.  512 x 4096 x 21504: 78 against 104 us; 512 x 21504 x 4096 in two splits: 70 against
+      // 76; 512 x 896 x 21504: 39 against 48.  One wave of a short loop: 512 x 4096 x 4096 in two splits takes 24.3 alone and
+      // 25.9 in pairs, 512 x 4096 x 6144 34.6 and 35.6.
+      if (n_tiles >= 2 && ((int64_t)(p.mp / 256) * n_tiles * nz > sm_count() || p.kb_per >= 128)) return launch_pair(p, n_tiles, nz, a.pdl, st);
       return launch_tc5<256, 4>(p, n_tiles, nz, a.pdl, st);
   }
 }
