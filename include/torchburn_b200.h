@@ -208,9 +208,9 @@ void tb_set_gemv_tuning(int32_t product_mode, int32_t rows_per_warp, int32_t war
 void tb_set_stream_tuning(int32_t enabled, int32_t ctas_per_sm, int32_t ring_kb,
                           int32_t elements_per_lane, int32_t groups);
 /* The stateless products (tb_gemm_w4a32_grouped, tb_swiglu_gemv_w4a32, tb_linear_forward, ...) with two or more
- * activation rows need a workspace (digit form of x, partial sums of a K split).  The library keeps one block
- * per (device, stream), allocated at the first such call on the stream outside a graph capture and grown on
- * demand - the reference allocates its outputs per call too (src/quantization/packed_v2.rs:598-606).  This frees
+ * activation rows, and tb_fused_swiglu_mlp, need a workspace (digits or images of x, partial sums of a K split, hidden
+ * activations).  The library keeps blocks per (device, stream), allocated by calls outside a graph capture, one for each
+ * thread that calls at the same time, grown on demand, 2 GiB at most in all - the reference allocates its outputs per call too (src/quantization/packed_v2.rs:598-606).  This frees
  * all of them (after a device synchronize); later calls allocate again. */
 void tb_release_workspaces(void);
 /* 1 after a bounded device-side wait ran out in any kernel of this library on the current
@@ -262,7 +262,9 @@ tb_status tb_linear_device_ptrs(const tb_linear* lin, const uint8_t** qweight,
 
 /* fused_swiglu_mlp / fused_swiglu_mlp_batched: out = down(silu(gate(x)) * up(x)),
  * x [m, hidden] -> out [m, hidden].  src/ffi/quantization_ffi.rs:203-218, 517-532;
- * src/quantization/fused_ops.rs:138-424, 1267-1319. */
+ * src/quantization/fused_ops.rs:138-424, 1267-1319.  On device buffers the call is
+ * in the order of the stream, like tb_linear_forward; on host buffers it returns
+ * after the result is in `out`. */
 tb_status tb_fused_swiglu_mlp(tb_linear* gate, tb_linear* up, tb_linear* down, const float* x,
                               int64_t m, float* out, tb_space io_space, void* stream);
 
@@ -523,7 +525,9 @@ tb_status tb_decoder_step_batch(tb_decoder* dec, const int64_t* token_ids, const
  * *end_offset = start_offset + n; TB_ERR_ARG when it would pass max_seq_len.
  * A decoder built for one row steps token by token like the reference; one
  * built with max_batch > 1 takes max_batch positions of sequence 0 per
- * batched step (one pass over the weights for all of them). */
+ * batched step (one pass over the weights for all of them), and more than
+ * max_batch positions in portions of up to 512 rows, in memory that it holds for
+ * them (on one GPU; 0.2 GB at the 8B widths, without it in steps as before). */
 tb_status tb_decoder_prefill_tokens(tb_decoder* dec, const int64_t* tokens, int64_t n,
                                     int64_t start_offset, int64_t* end_offset);
 /* prefill, src/llm/decoder.rs:545-558: tokens at offsets 0..n-1, last logits out. */
