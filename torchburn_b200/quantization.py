@@ -75,6 +75,23 @@ def w4a32_grouped_linear(
     """
     x_orig_shape = x.shape
     K = x_orig_shape[-1]
+    # Operands that need no conversion or copy, on the current device: nothing but the call.  (One row of 4096 x 4096 is 7 us of
+    # kernel; the conversions that convert nothing, the device guard and the stream object below took 14 us of its 21.)
+    if (type(x) is torch.Tensor and x.is_cuda and x.dtype is torch.float32 and x.is_contiguous() and w_packed.dtype is torch.uint8
+            and w_packed.ndim == 2 and w_packed.is_contiguous() and scales.dtype is torch.float32 and scales.is_contiguous()
+            and (bias is None or (bias.dtype is torch.float32 and bias.is_contiguous()))):
+        index = x.get_device()
+        N, packed_k = w_packed.shape
+        M = x.numel() // K if K else 0
+        if (M > 0 and index == w_packed.get_device() == scales.get_device() == torch.cuda.current_device() and packed_k == (K + 1) // 2
+                and scales.shape == (N, (K + group_size - 1) // group_size)
+                and (bias is None or (bias.get_device() == index and bias.numel() == N))):
+            out = x.new_empty((*x_orig_shape[:-1], N))
+            status = lib().tb_gemm_w4a32_grouped(x.data_ptr(), w_packed.data_ptr(), scales.data_ptr(), None if bias is None else bias.data_ptr(),
+                                                 out.data_ptr(), M, N, K, group_size, torch._C._cuda_getCurrentRawStream(index))
+            if status:
+                check(status)
+            return out
     on_cpu = x.device.type != "cuda"
     dev = _require_cuda() if on_cpu else x.device
     x_2d = x.reshape(-1, K).contiguous().float().to(dev)
