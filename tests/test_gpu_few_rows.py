@@ -1,0 +1,85 @@
+"""Products of 2 to 8 activation rows (w4_rows_kernel).
+
+Bound of the products, per output, with A = sum |x| |w|: activations, codes and their products are exact; a 32-element block's
+sum is six accumulating instructions, of which the two with the large pieces may truncate at 2^-23 of at most A and the
+others at 2^-8 of that; adding the K / 32 blocks, the eight sums of the warps and the bias takes one fp32 rounding each
+(2^-24 A): below (2 * 2 * 1.1 + K / 32 + 10) * 2^-24 * A."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.fail("no CUDA device: GPU tests need a B200")
+    return torch
+
+
+@pytest.fixture(scope="module")
+def tb(torch):
+    import torchburn_b200 as tb
+
+    return tb
+
+
+def int4(torch, n, k, g, seed):
+    """(packed, scales, the weights in float64), on the GPU."""
+    gen = torch.Generator("cuda").manual_seed(seed)
+    w = torch.randn(n, k // g, g, device="cuda", generator=gen) * 0.02
+    s = (w.abs().amax(-1) / 7).clamp_min(1e-8)
+    c = (w / s[..., None]).round_().clamp_(-8, 7)
+    q = c.add(8).to(torch.uint8).reshape(n, k)
+    return (q[:, 0::2] | (q[:, 1::2] << 4)).contiguous(), s.contiguous(), (c.double() * s.double()[..., None]).reshape(n, k)
+
+
+@pytest.mark.parametrize("m,n,k,g,pair", [
+    (2, 1, 32, 32, 0), (8, 7, 32, 32, 1), (3, 17, 96, 32, 0),             # one block of K, one ragged tile
+    (5, 16 * 148, 256, 32, 0), (8, 16 * 148 + 1, 288, 32, 0),             # a tile per CTA, one more; a stage and an eighth
+    (4, 8 * 148 * 2 + 3, 512, 64, 1), (8, 14330, 896, 64, 0),             # unaligned rows of scales, copied in eights
+    (7, 4864, 896, 128, 1), (8, 1000, 1920, 128, 0),                      # and in fours; K that is no whole stage
+    (5, 14 * 16 * 148 + 5, 256, 32, 0), (8, 33000, 512, 64, 0),           # more tiles than a pass holds
+    (6, 6144, 4096, 32, 0), (8, 4096, 14336, 32, 0), (8, 14336, 4096, 32, 1), (5, 96, 20480, 64, 0),
+])
+def test_products_of_few_rows_match_float64(torch, tb, m, n, k, g, pair):
+    p, s, w = int4(torch, n, k, g, m + n + k)
+    p2, s2, w2 = int4(torch, n, k, g, m + n + k + 1)
+    gen = torch.Generator("cuda").manual_seed(m)
+    x = torch.randn(m, k, device="cuda", generator=gen) * 10 ** (6 * torch.rand(m, 1, device="cuda", generator=gen) - 3)
+    b = torch.randn(n, device="cuda", generator=gen)
+    tol = (4.4 + k / 32 + 10) * 2.0 ** -24
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        if pair:
+            y = torch.empty(m, n, device="cuda")
+            st = torch.cuda.current_stream().cuda_stream
+            assert tb.lib().tb_swiglu_gemv_w4a32(x.data_ptr(), p.data_ptr(), s.data_ptr(), b.data_ptr(), p2.data_ptr(), s2.data_ptr(), None, y.data_ptr(),
+                                                 m, n, k, g, st) == 0, tb.last_error()
+        else:
+            y = tb.w4a32_grouped_linear(x, p, s, b, g)
+        torch.cuda.synchronize()
+    ran = "w4_rows_kernel" in " ".join(e.key for e in prof.key_averages())
+    assert ran or m < 5, "five and more rows run on the streaming tensor-core kernel"
+    gate, bound = x.double() @ w.T + b, (x.double().abs() @ w.abs().T + b.abs()) * tol
+    if pair:
+        up, sig = x.double() @ w2.T, torch.sigmoid(gate)
+        # silu' <= 1.1, |silu(g)| <= |g|; four roundings of the epilogue
+        bound = 1.1 * bound * up.abs() + gate.abs() * (x.double().abs() @ w2.abs().T) * tol + 4 * 2.0 ** -23 * (gate * sig * up).abs() + bound * 1e-6
+        gate = gate * sig * up
+    assert bool(((y.double() - gate).abs() <= bound + 1e-30).all()), float(((y.double() - gate).abs() / bound).max())
+    if m < y.shape[0] + 1 and not pair:   # equal calls give equal bits
+        assert torch.equal(tb.w4a32_grouped_linear(x, p, s, b, g), y)
+    assert tb.lib().tb_device_fault_flag() == 0
+
+
+def test_few_rows_keep_infinities_to_their_row(torch, tb):
+    """A row with an infinity or a NaN leaves the other rows as they are."""
+    p, s, _ = int4(torch, 300, 512, 32, 1)
+    x = torch.randn(6, 512, device="cuda")
+    want = tb.w4a32_grouped_linear(x, p, s, None, 32)
+    x[2, 7], x[4, 100] = float("inf"), float("nan")
+    got = tb.w4a32_grouped_linear(x, p, s, None, 32)
+    keep = [0, 1, 3, 5]
+    assert torch.equal(got[keep], want[keep])
+    assert bool(torch.isnan(got[4]).all()) and not bool(torch.isfinite(got[2]).any())

@@ -23,7 +23,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "lib", "obj")
 LIB = os.path.join(HERE, "lib", "libtorchburn_b200.so")
 PROFILES = {"full": LIB, "dense": os.path.join(HERE, "lib", "libtorchburn_b200_dense.so")}
-INT4_SOURCES = ("w4_step.cu", "w4_stream.cu", "w4_gemv.cu", "w4_mma.cu", "w4_tc5.cu", "attention.cu", "attention_rows.cu")
+INT4_SOURCES = ("w4_step.cu", "w4_stream.cu", "w4_gemv.cu", "w4_mma.cu", "w4_rows.cu", "w4_tc5.cu", "attention.cu", "attention_rows.cu")
 INT4_ABSENT = "w4_absent.cpp"
 
 NVCC_FLAGS = [

@@ -123,7 +123,12 @@ void release_workspaces();   // gives back every block that no call holds
 // warps force the launch shape of the M = 1 kernels (0 = automatic).
 void set_gemv_tuning(int xmode, int rows_per_warp, int warps);
 
-// Tensor-core kernel for 2 <= M (w4_mma.cu).
+// Streaming tensor-core kernel for 2 to 8 rows (w4_rows.cu); `scratch` holds w4_rows_scratch_bytes.
+size_t w4_rows_scratch_bytes(int64_t k);
+bool w4_rows_supported(const GemvArgs& a);
+tb_status launch_w4_rows(const GemvArgs& a, void* scratch, cudaStream_t stream);
+int rows_fault_flag();
+// Integer tensor-core kernel for 9 and more rows (w4_mma.cu).
 size_t w4_mma_scratch_bytes(int m, int64_t k);
 tb_status launch_w4_mma(const GemvArgs& a, void* scratch, cudaStream_t stream);
 double w4_mma_cost(int64_t n, int64_t k, bool pair);   // microseconds of a call with 9 to 16 rows

@@ -12,6 +12,7 @@ tb_status launch_w4_gemv(const GemvArgs&, cudaStream_t) { return absent(); }
 int w4_gemv_launches(const GemvArgs&) { return 0; }
 void set_gemv_tuning(int, int, int) {}
 size_t w4_mma_scratch_bytes(int, int64_t) { return 0; }
+int rows_fault_flag() { return 0; }
 int tc5_fault_flag() { return 0; }
 void set_stream_tuning(int, int, int, int, int) {}
 int stream_fault_flag() { return 0; }

@@ -449,17 +449,17 @@ void set_gemv_tuning(int xmode, int rows_per_warp, int warps) {
 
 // Kernels one launch_w4_gemv call starts for these operands (the same choices as below).
 static bool few_rows_narrow(const GemvArgs& a) {
-  // Three or four rows of a narrow matrix: the CUDA-core kernel beats the tensor-core rows kernel, whose cost
-  // hardly depends on the row count below 8 (graph-timed, K = 4096: N = 4096 at 3 / 4 / 5 rows 11.7 / 13.9 /
-  // 16.0 us against 19.3; N = 6144 at 3 / 4 rows 18.2 / 21.4 against 23.0; the wide gate/up pair never).
+  // Three or four rows of a narrow matrix: the CUDA-core kernel beats the streaming tensor-core kernel, whose cost
+  // hardly depends on the row count (graph-timed over weights past L2: 4096 x 4096 at 3 / 4 rows 11.6 / 13.7 us against 12.0,
+  // 6144 x 4096 17.9 / 21.2 against 13.9, 1152 x 896 4.3 / 5.1 against 5.5; the wide gate/up pair never).
   // Every CTA of that kernel prepares all rows of x itself (with a fused RMSNorm: twice over them), so it is
   // kept to four rows, three with the norm.
-  return a.m >= 3 && a.m <= (a.norm_w ? 3 : 4) && a.w2 == nullptr && a.k <= 4096 && (int64_t)a.m * a.n <= 24576;
+  return a.m >= 3 && a.m <= (a.norm_w ? 3 : 4) && a.w2 == nullptr && a.k <= 4096 && (int64_t)a.m * a.n <= 12288;
 }
 int w4_gemv_launches(const GemvArgs& a) {
   if (w4_stream_supported(a)) return 1;
   if (a.m >= 2 && g_mma_enabled && !few_rows_narrow(a) && ((a.k / 2) % 16) == 0)
-    return w4_tc5_supported(a) ? w4_tc5_launches(a.m) : 2 * ((a.m + 63) / 64);   // per pass: the activation pre-pass + the product
+    return w4_rows_supported(a) ? 2 : w4_tc5_supported(a) ? w4_tc5_launches(a.m) : 2 * ((a.m + 63) / 64);   // per pass: the activation pre-pass + the product
   return (a.m + kMaxM - 1) / kMaxM;
 }
 
@@ -496,9 +496,11 @@ tb_status launch_w4_gemv(const GemvArgs& a, cudaStream_t stream) {
   if (a.x_ss8 || a.out_scaled || a.out_ss8)
     return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: the split RMSNorm needs the persistent M = 1 kernel for this shape");
   if (a.m >= 2 && g_mma_enabled && !few_rows_narrow(a) && ((a.k / 2) % 16) == 0) {
-    const bool tc5 = w4_tc5_supported(a);   // 17 and more rows, and 9 to 16 where it costs less: tcgen05
-    auto launch = [&](void* scratch) {   // both begin with the tickets of a K split
-      return tc5 ? launch_w4_tc5(a, static_cast<char*>(scratch) + 4096, static_cast<int*>(scratch), stream) : launch_w4_mma(a, scratch, stream);
+    const bool rows = w4_rows_supported(a);   // 2 to 8 rows
+    const bool tc5 = w4_tc5_supported(a);     // 17 and more rows, and 9 to 16 where it costs less: tcgen05
+    auto launch = [&](void* scratch) {   // begins with the tickets of a K split
+      return rows ? launch_w4_rows(a, static_cast<char*>(scratch) + 4096, stream) :
+             tc5 ? launch_w4_tc5(a, static_cast<char*>(scratch) + 4096, static_cast<int*>(scratch), stream) : launch_w4_mma(a, scratch, stream);
     };
     if (a.xq_scratch) return launch(a.xq_scratch);
     WorkspaceLease ws;
