@@ -54,10 +54,11 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 
-// Launch with optional programmatic stream serialization and a cluster of `cluster` CTAs along x.
+// Launch with optional programmatic stream serialization and a cluster of `cluster` CTAs along x.  (Static and dynamic shared memory
+// above 48 KB need the opt-in: asked for from 32 KB of dynamic memory on.)
 template <typename... KArgs, typename... Args>
 tb_status launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, int cluster, Args... args) {
-  if (smem > 48 * 1024) TB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 32 * 1024) TB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;

@@ -548,8 +548,10 @@ tb_status launch_window_parts(Precision p, const WindowAttnArgs& a, int splits, 
 }
 
 size_t window_attn_score_stride(int64_t max_visible) {
-  // the tensor-core form numbers keys per block of 64 queries: up to 63 more than one row sees
-  return (size_t)pad_to(max_visible + 64, 32);
+  // the tensor-core form numbers keys per block of 64 queries: up to 63 more than one row sees; whole tiles of 64 keys, then a
+  // reference per tile
+  const int64_t keys = pad_to(max_visible + 64, 64);
+  return (size_t)(keys + pad_to(keys / 64, 32));
 }
 
 tb_status launch_window_attention(Precision p, const WindowAttnArgs& a, cudaStream_t st, int* launches) {
