@@ -445,6 +445,12 @@ tb_status launch_m(const GemvParams& p, bool pdl, cudaStream_t stream) {
       w = g_force_warps > 0 ? g_force_warps : 8;
     } else if (EPI == 1) {
       r = ((int64_t)p.n >= (int64_t)sms * 64) ? 2 : 1;
+      // x staged by four warps: CTAs of eight wait longer for their slowest (4864 x 896, us a token of the 0.5B widths: one pair of rows
+      // a warp, eight warps 738, four 718; two pairs, four warps 711)
+      if (p.k <= 1024) {
+        w = 4;
+        if ((int64_t)p.n >= (int64_t)sms * 16) r = 2;
+      }
     } else {
       r = ((int64_t)p.n >= (int64_t)sms * 128) ? 4 : ((int64_t)p.n >= (int64_t)sms * 32 ? 2 : 1);
       if (r == 1) w = 4;
