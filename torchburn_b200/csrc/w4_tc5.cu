@@ -19,7 +19,11 @@
 // the thread that unpacks row r writes its codes with tcgen05.st straight from registers (A operand from tensor
 // memory), so the weights pass through shared memory only as packed nibbles.
 //
-//   unpacking    4 or 8 warps (thread = weight row) turn the nibbles in the ring into codes in tensor memory
+//   unpacking    4, 8 or 16 warps (thread = weight row) turn the nibbles in the ring into codes in tensor memory.  One warp
+//                takes ~1080 cycles for 64 elements of K (reading and unpacking 415, its waits for the stage and the
+//                unit ~440), a chain that no ring depth shortens; with few activation rows nothing else is as slow, so
+//                more warps take turns at the units.  16 rather than 8 at up to 32 rows: 42.2 -> 37.7 us for the pair
+//                of 16 x 4096 x 14336, 46.0 -> 43.9 for 32 rows.  From 96 columns on the epilogue needs the registers.
 //   epilogue     8 warps: two teams of 128 threads (thread = weight row, all activation rows) that take every
 //                other VISIT: the accumulators of up to four groups, 128 columns of tensor memory, handed over
 //                at once.  The fixed cost of a hand-over (commit, barrier, tcgen05.ld latency: ~400 cycles) was what
@@ -168,10 +172,13 @@ struct Shape {
   static constexpr int kVk = kGps * G;                     // K elements per visit: 32, 64 or 128
   static constexpr int kSteps = kVk / 16;                  // K16 steps per visit
   static constexpr int kVisitsPerStage = kVk >= kKC ? 1 : kKC / kVk;
-  static constexpr int kDW = kCols <= 96 ? 8 : 4;          // unpacking warps
+  static constexpr int kDW = NW == 2 && kCols <= 64 ? 16 : (kCols <= 96 ? 8 : 4);   // unpacking warps
+  // Teams of four of them: each for one weight tile (kTeamTile) or all of them, and for every kUnitStride-th unit.
+  static constexpr bool kTeamTile = NW == 2 && kDW >= 8;
+  static constexpr int kUnitStride = kDW / (kTeamTile ? 8 : 4);
   static constexpr int kThreads = (kDW + 12) * 32;
   // registers: (kDW + 4) warps give back to the 8 epilogue warps; the sum stays at what the block was launched with
-  static constexpr int kRegsLaunch = kDW == 8 ? 96 : 128, kRegsFew = kDW == 8 ? 64 : 56, kRegsMany = kDW == 8 ? 144 : 200;
+  static constexpr int kRegsLaunch = kDW == 16 ? 72 : (kDW == 8 ? 96 : 128), kRegsFew = kDW == 16 ? 48 : (kDW == 8 ? 64 : 56), kRegsMany = kDW == 16 ? 128 : (kDW == 8 ? 144 : 200);
   static_assert((kDW + 4) * kRegsFew + 8 * kRegsMany <= (kDW + 12) * kRegsLaunch, "register split");
   static constexpr int kStagesA = 128 / (32 * NW);
   static constexpr int kStagesB = MP <= 16 ? 16 : (MP <= 32 ? 8 : (MP <= 48 ? 5 : 4));   // up to 96 KB
@@ -206,13 +213,13 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
   if (tid == 0) {
     s_abort = 0;
     for (uint32_t s = 0; s < kRing; ++s) {
-      mbar_init(&full_a[s], NW == 2 && S::kDW == 8 ? 8 : 4);   // one lane of each unpacking warp of the stage
+      mbar_init(&full_a[s], S::kTeamTile ? 8 : 4);   // one lane of each unpacking warp of the stage
       mbar_init(&full_b[s], 1);
       mbar_init(&done[s], S::kVisitsPerStage);   // the MMAs that read the stage have finished: one commit per visit
     }
     for (int s = 0; s < S::kUnits; ++s) {
       mbar_init(&full_w[s], 1);
-      mbar_init(&empty_w[s], NW == 2 && S::kDW == 8 ? 8 : 4);   // one lane of each warp that reads the unit
+      mbar_init(&empty_w[s], S::kTeamTile ? 8 : 4);   // one lane of each warp that reads the unit
     }
     for (int s = 0; s < S::kScales; ++s) mbar_init(&empty_s[s], S::kGps == 4 ? 4 : 8);   // one team reads a unit's scales, or both
     for (int s = 0; s < kSlots; ++s) {
@@ -330,8 +337,8 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
   } else if (warp < S::kDW) {
     // ---------------- unpacking: thread = weight row ----------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kRegsFew));
-    // eight warps: a team per weight tile, or (one tile) teams that take every other unit of 128 elements
-    constexpr bool kTeamTile = S::kDW == 8 && NW == 2, kTeamUnit = S::kDW == 8 && NW == 1;
+    // eight or more warps: teams of four, each for one weight tile and, with 16 warps or one tile, every other unit of 128 elements
+    constexpr bool kTeamTile = S::kTeamTile;
     constexpr int kTiles = S::kDW == 4 ? NW : 1;       // weight tiles of one thread
     const int team = warp >> 2, row = tid & 127;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
@@ -339,10 +346,10 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
     // touches every bank once
     const uint32_t ring = smem_u32(smem + S::kOffNib) + (uint32_t)row * 64u;
     const uint32_t swz = (uint32_t)((row >> 1) & 3);
-    uint32_t u = kTeamUnit ? (uint32_t)team : 0u;   // the CTA's units run through all its tiles
+    uint32_t u = (uint32_t)(kTeamTile ? team >> 1 : (S::kDW == 4 ? 0 : team));   // the CTA's units run through all its tiles
     const uint32_t nu = (uint32_t)(my_tiles * nunits);
     bool ok = true;
-    for (; u < nu && ok; u += kTeamUnit ? 2 : 1) {
+    for (; u < nu && ok; u += (uint32_t)S::kUnitStride) {
       const uint32_t ws = u % S::kUnits;
       ok = mbar_wait_warp(&full_w[ws], (u / S::kUnits) & 1u, &s_abort);
       if (!ok) break;
@@ -352,24 +359,29 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
         const uint32_t a_col = lane_base + (c % SA) * (32u * NW);
 #pragma unroll
         for (int i = 0; i < kTiles; ++i) {
-          const int q = kTeamTile ? team : i;
+          const int q = kTeamTile ? team & 1 : i;
           const uint32_t src = ring + (ws * NW + (uint32_t)q) * kUnitBytes, col = a_col + (uint32_t)q * 32u;
-          uint32_t v[2][16];
+          // the codes are ready in registers before the stage is free (16 warps, 48 registers each: half of them)
+          constexpr int kHold = S::kDW == 16 ? 1 : 2;
 #pragma unroll
-          for (uint32_t e = 0; e < 2; ++e) {   // 32 elements = 16 columns per 16 bytes of nibbles
-            uint32_t wd[4];
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wd[0]), "=r"(wd[1]), "=r"(wd[2]), "=r"(wd[3]) : "r"(src + (((2 * h + e) ^ swz) * 16u)));
+          for (uint32_t e0 = 0; e0 < 2; e0 += kHold) {
+            uint32_t v[kHold][16];
 #pragma unroll
-            for (int w = 0; w < 4; ++w) unpack8(wd[w], &v[e][4 * w]);
+            for (uint32_t e = 0; e < kHold; ++e) {   // 32 elements = 16 columns per 16 bytes of nibbles
+              uint32_t wd[4];
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wd[0]), "=r"(wd[1]), "=r"(wd[2]), "=r"(wd[3]) : "r"(src + (((2 * h + e0 + e) ^ swz) * 16u)));
+#pragma unroll
+              for (int w = 0; w < 4; ++w) unpack8(wd[w], &v[e][4 * w]);
+            }
+            if (i == 0 && e0 == 0) {
+              if (c >= SA) ok = mbar_wait_warp(&done[(c - SA) % kRing], ((c - SA) / kRing) & 1u, &s_abort);
+              if (!ok) break;
+              tc_fence_after();
+            }
+#pragma unroll
+            for (uint32_t e = 0; e < kHold; ++e) tmem_st16(col + 16u * (e0 + e), v[e]);
           }
-          // the codes are ready in registers before the stage is free: from "free" to "full" it is only the store
-          if (i == 0) {
-            if (c >= SA) ok = mbar_wait_warp(&done[(c - SA) % kRing], ((c - SA) / kRing) & 1u, &s_abort);
-            if (!ok) break;
-            tc_fence_after();
-          }
-          tmem_st16(col, v[0]);
-          tmem_st16(col + 16u, v[1]);
+          if (!ok) break;
         }
         if (!ok) break;
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -460,7 +472,7 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
         const uint32_t slot = at6 >= kSlots ? at6 - kSlots : at6;
         const uint32_t d = lane_base + 128u + slot * 128u;
         constexpr int kN16 = S::kGps * S::kCols / 16;          // 16-column loads of the visit
-        constexpr int kBatch = S::kCols > 64 ? 2 : (kN16 < 4 ? kN16 : (kN16 % 4 == 0 ? 4 : 3));   // in flight at once
+        constexpr int kBatch = S::kCols > 32 && kN16 % 2 == 0 ? 2 : (S::kCols > 64 ? 2 : (kN16 < 4 ? kN16 : (kN16 % 4 == 0 ? 4 : 3)));   // in flight at once
         static_assert(kN16 % kBatch == 0, "loads per visit");
 #pragma unroll
         for (int b = 0; b < kN16 / kBatch; ++b) {
