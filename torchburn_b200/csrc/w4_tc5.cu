@@ -300,25 +300,38 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       bool ok = true;
       const int chunks = p.k / kKC;
       const uint32_t w_at = smem_u32(smem + S::kOffNib), s_at = smem_u32(smem + S::kOffScale);
-      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        const int mt = t % p.mtiles, kz = (t / p.mtiles) % p.ksplit;
-        const int n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW);
-        const unsigned char* src = p.xq + ((size_t)mt * chunks + (size_t)kz * nstages) * S::kBBytes;
-        for (int i = 0; i < nunits && ok; ++i, ++u) {
-          const uint32_t ws = u % S::kUnits, ss = u % S::kScales;
-          if (u >= S::kUnits) ok = mbar_wait_fast(&empty_w[ws], (u / S::kUnits - 1u) & 1u, &s_abort);
-          if (G == 32 && ok && u >= S::kScales) ok = mbar_wait_fast(&empty_s[ss], (u / S::kScales - 1u) & 1u, &s_abort);
-          if (!ok) break;
-          // the scales arrive with the codes: who has seen sums of the unit has seen its scales
-          mbar_expect_tx(&full_w[ws], NW * (kUnitBytes + (G == 32 ? kUnitScaleBytes : 0)));
+      auto weights = [&](uint32_t wu, int t, int i) {   // unit wu of the CTA: unit i of tile t
+        const uint32_t ws = wu % S::kUnits, ss = wu % S::kScales;
+        if (wu >= S::kUnits) ok = mbar_wait_fast(&empty_w[ws], (wu / S::kUnits - 1u) & 1u, &s_abort);
+        if (G == 32 && ok && wu >= S::kScales) ok = mbar_wait_fast(&empty_s[ss], (wu / S::kScales - 1u) & 1u, &s_abort);
+        if (!ok) return;
+        const int kz = (t / p.mtiles) % p.ksplit, n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW);
+        // the scales arrive with the codes: who has seen sums of the unit has seen its scales
+        mbar_expect_tx(&full_w[ws], NW * (kUnitBytes + (G == 32 ? kUnitScaleBytes : 0)));
+#pragma unroll
+        for (int q = 0; q < NW; ++q)
+          tma_box(w_at + (ws * NW + q) * kUnitBytes, &p.w[p.pair ? q : 0], kz * (p.kper >> 1) + i * 64, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
+        if constexpr (G == 32) {
 #pragma unroll
           for (int q = 0; q < NW; ++q)
-            tma_box(w_at + (ws * NW + q) * kUnitBytes, &p.w[p.pair ? q : 0], kz * (p.kper >> 1) + i * 64, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
-          if constexpr (G == 32) {
-#pragma unroll
-            for (int q = 0; q < NW; ++q)
-              tma_box(s_at + (ss * NW + q) * kUnitScaleBytes, &p.s[p.pair ? q : 0], kz * (p.kper / G) + i * 4, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
-          }
+            tma_box(s_at + (ss * NW + q) * kUnitScaleBytes, &p.s[p.pair ? q : 0], kz * (p.kper / G) + i * 4, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
+        }
+      };
+      // The first weights, a ring of them, do not depend on the pre-pass, which this kernel is launched beside (programmatic
+      // serialization); the images do.
+      static_assert(S::kScales >= S::kUnits, "scales of the first units");
+      uint32_t ahead = 0;
+      for (int t = blockIdx.x, i = 0; t < total && ahead < S::kUnits; ++ahead) {
+        weights(ahead, t, i);
+        if (++i == nunits) { i = 0; t += gridDim.x; }
+      }
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        const int mt = t % p.mtiles, kz = (t / p.mtiles) % p.ksplit;
+        const unsigned char* src = p.xq + ((size_t)mt * chunks + (size_t)kz * nstages) * S::kBBytes;
+        for (int i = 0; i < nunits && ok; ++i, ++u) {
+          if (u >= ahead) weights(u, t, i);
+          if (!ok) break;
           for (int h = 0; h < 2; ++h, ++c) {
             if (c >= SB) ok = mbar_wait_fast(&done[(c - SB) % kRing], ((c - SB) / kRing) & 1u, &s_abort);
             if (!ok) break;
@@ -331,6 +344,7 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       if (!ok) {
         int no_abort = 0;
         for (uint32_t i = c > SB ? c - SB : 0; i < c; ++i) mbar_wait_fast(&full_b[i % kRing], (i / kRing) & 1u, &no_abort);
+        if (u < ahead) u = ahead;
         for (uint32_t i = u > S::kUnits ? u - S::kUnits : 0; i < u; ++i) mbar_wait_fast(&full_w[i % S::kUnits], (i / S::kUnits) & 1u, &no_abort);
       }
     }
@@ -626,6 +640,7 @@ template <int NI>
 __global__ void __launch_bounds__(kPrepThreads) tc5_prep_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
                                                                 unsigned char* __restrict__ xq, int m, int mp, int k) {
   __shared__ float s_ss[kPrepThreads / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the product may set up and fetch weights; its images wait for this grid's end
   const int row = blockIdx.x, tid = threadIdx.x, step = (int)blockDim.x * 8;
   const bool live = row < m;
   const float* xr = x + (size_t)(live ? row : 0) * k;
@@ -823,8 +838,21 @@ tb_status launch_w4_tc5(const GemvArgs& a, void* scratch, int* tickets, cudaStre
     TB_CUDA_TRY(cudaFuncSetAttribute(v.kern[gi], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem[gi]));
     const int64_t tiles = (int64_t)plan.mtiles * plan.ntiles * plan.ksplit;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    v.kern[gi]<<<grid, v.threads[gi], v.smem[gi], stream>>>(p);
-    TB_CUDA_TRY(cudaGetLastError());
+    // Beside the pre-pass (which itself starts when all in front of it is complete): the tensor memory, the barriers and the first
+    // ring of weights are ready when the images are.  The MLP of 16 rows at 4096 / 14336: 71.1 -> 66.2 us; 333 rows gain nothing.
+    // (Weights that ran ahead of the images all the way, not only by the first ring, cost 27 -> 40 us at 16 x 14336 x 4096: the
+    // copying thread's wait for a unit held back images that others waited for.)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)v.threads[gi]);
+    cfg.dynamicSmemBytes = v.smem[gi];
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    TB_CUDA_TRY(cudaLaunchKernelEx(&cfg, v.kern[gi], p));
   }
   return TB_OK;
 }
