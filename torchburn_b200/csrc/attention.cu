@@ -37,6 +37,8 @@ constexpr int kRG = kWR / 4;           // groups of 4 rows per warp and stage (2
 constexpr int kMaxGq = 8;              // q heads per kv head
 constexpr int kMaxStages = 8;
 constexpr int kChunkRows = 512;        // positions whose scores are held in shared memory at a time
+constexpr int kChunkRows3 = 256;       // with three CTAs per SM
+constexpr int chunk_rows(int ctas) { return ctas == 3 ? kChunkRows3 : kChunkRows; }
 constexpr size_t kCounterBytes = 16384;  // 4096 tickets: (sequence, kv head) pairs of a launch
 constexpr int kMaxParts = 48;          // shares of a sequence: more cost more in the merge than they save
 constexpr int kSeqCap = 32768;         // src/llm/decoder.rs:1180
@@ -129,13 +131,13 @@ __device__ __forceinline__ float rope_elem(const float* x, const float* c, const
   return __fadd_rn(__fmul_rn(x[i], c[i]), __fmul_rn(x[i - half], s[i]));
 }
 
-// Shared memory (floats): q_s [gq][D] | kv_new [2][D] | S [kChunkRows + 1][GQM] | region.  The
+// Shared memory (floats): q_s [gq][D] | kv_new [2][D] | S [chunk + 1][GQM] | region.  The
 // region is the ring (stages * 32 * D) while rows stream in; afterwards it holds w_acc
 // [kCW][gq][D] for the combine and, in the CTA that merges, wts [gq][nc] | ml [gq] | a tile of
 // partials.  Every part starts on a 16-byte boundary (float4 accesses).
 __host__ __device__ inline size_t up4(size_t v) { return (v + 3) & ~(size_t)3; }
-__host__ __device__ inline size_t attn_fixed_floats(int D, int gq, int gqm) {
-  return up4((size_t)gq * D) + 2 * (size_t)D + up4((size_t)(kChunkRows + 1) * gqm);
+__host__ __device__ inline size_t attn_fixed_floats(int D, int gq, int gqm, int chunk) {
+  return up4((size_t)gq * D) + 2 * (size_t)D + up4((size_t)(chunk + 1) * gqm);
 }
 inline size_t attn_region_floats(int D, int gq, int nc, int stages) {
   const size_t ring = (size_t)stages * kStageRows * D;
@@ -353,7 +355,7 @@ __device__ __forceinline__ Share plan_share(const AttnParams& p, int x, int lane
 }
 
 // One CTA = one share of the positions of one (sequence, kv head).  The share is walked in
-// chunks of at most kChunkRows positions; for every chunk the producer lane streams the K
+// chunks of at most 512 (256) positions; for every chunk the producer lane streams the K
 // rows and then the V rows through the ring (32 rows per stage).  The consumer warps score the
 // K stages as they land (8 rows of a stage per warp) into S, the CTA then takes the exact
 // maximum and the exponentials of the chunk (a two-pass softmax inside the chunk; the running
@@ -361,12 +363,14 @@ __device__ __forceinline__ Share plan_share(const AttnParams& p, int x, int lane
 // they land.  No softmax dependency sits inside either streaming loop.
 // Two CTAs per SM is what the grid is sized for; telling the compiler so costs nothing (159 registers)
 // and measured 1% on the whole step.  With a bound of one CTA it takes 187 registers and the step is 8% slower.
-#ifndef TB_ATTN_MIN_CTAS
-#define TB_ATTN_MIN_CTAS 2
-#endif
-#define TB_ATTN_BOUNDS __launch_bounds__(kThreads, TB_ATTN_MIN_CTAS)
-template <int D, int GQM>
-__global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
+// A batch that is walked in several rounds of CTAs has three per SM (128 registers, four ring stages instead of six,
+// half the chunk): a stage's scores are a chain of ~1000 cycles in a warp, and a CTA that starts or merges leaves its
+// neighbours the memory.  32 sequences of 128 to 4096 positions, 8 kv heads of 128: 115 -> 108 us a layer.  One round
+// gains nothing (8 sequences: 34 us either way), one sequence loses (more shares to merge), and with eight q heads per kv
+// head or narrower heads 128 registers are not enough or not measured: those keep two.
+template <int D, int GQM, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS) attn_decode_kernel(const AttnParams p) {
+  constexpr int kChunk = chunk_rows(CTAS);
   constexpr int F4 = D / 32;
   constexpr int CPR = D / 4;
   constexpr bool QREG = GQM * F4 <= 16 && kCW == 4;
@@ -385,8 +389,8 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
   const int gq = p.gq;
   float* q_s = smem;
   float* kv_new = q_s + up4((size_t)gq * D);
-  float* S = kv_new + 2 * D;                             // [(kChunkRows + 1)][GQM]
-  float* region = S + up4((size_t)(kChunkRows + 1) * GQM);
+  float* S = kv_new + 2 * D;                             // [(kChunk + 1)][GQM]
+  float* region = S + up4((size_t)(kChunk + 1) * GQM);
 
   const int kvh = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -429,7 +433,7 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
   // row is the last one of its range; it is taken from shared memory, not from the cache.
   const bool has_new = active && off >= t0 && off < t0 + rows;
   const int ring_rows = rows - (has_new ? 1 : 0);
-  const int nchunks = active ? max(1, (ring_rows + kChunkRows - 1) / kChunkRows) : 0;
+  const int nchunks = active ? max(1, (ring_rows + kChunk - 1) / kChunk) : 0;
   const int cache_seq = p.shared_cache ? 0 : b;
   float* kc = p.k_cache + ((int64_t)cache_seq * p.num_kv_heads + kvh) * p.max_seq_len * D;
   float* vc = p.v_cache + ((int64_t)cache_seq * p.num_kv_heads + kvh) * p.max_seq_len * D;
@@ -441,8 +445,8 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
       int i = 0;
       bool lost = false;
       for (int c = 0; c < nchunks && !lost; ++c) {
-        const int cr0 = c * kChunkRows;
-        const int crn = min(kChunkRows, ring_rows - cr0);
+        const int cr0 = c * kChunk;
+        const int crn = min(kChunk, ring_rows - cr0);
         const int nt = (crn + kStageRows - 1) / kStageRows;
         for (int pass = 0; pass < 2 && !lost; ++pass) {
           const float* src = (pass == 0 ? kc : vc) + (int64_t)(t0 + cr0) * D;
@@ -547,8 +551,8 @@ __global__ void TB_ATTN_BOUNDS attn_decode_kernel(const AttnParams p) {
     int it = 0;  // stages consumed so far (same order as the producer's)
 #pragma unroll 1
     for (int c = 0; c < nchunks; ++c) {
-      const int cr0 = c * kChunkRows;
-      const int crn = min(kChunkRows, ring_rows - cr0);
+      const int cr0 = c * kChunk;
+      const int crn = min(kChunk, ring_rows - cr0);
       const int nt = (crn + kStageRows - 1) / kStageRows;
       const bool new_here = has_new && c == nchunks - 1;
       if (c > 0) consumer_barrier();  // the previous chunk's weights in S have been used
@@ -793,6 +797,7 @@ struct AttnLayout {
   int grid;       // CTAs per kv head
   int nc;         // most of them that share a sequence
   int stages;
+  int ctas;       // per SM
   size_t part_o, part_ml;
 };
 
@@ -806,8 +811,12 @@ AttnLayout attn_layout(int batch, int num_heads, int num_kv_heads, int head_dim,
   AttnLayout L;
   const int64_t cap = max_seq_len < kSeqCap ? max_seq_len : kSeqCap;
   // Ring depth: 96 KB of stages for head_dim 128 (two CTAs per SM), fewer bytes for narrower heads.
-  const int cps = g_ctas_per_sm > 0 ? g_ctas_per_sm : 2;
-  L.stages = head_dim == 128 ? 6 : 8;
+  int cps = g_ctas_per_sm > 0 ? g_ctas_per_sm : 2;
+  L.ctas = 2;
+  if (g_ctas_per_sm == 0 && g_chunk_override == 0 && head_dim == 128 && num_heads <= 4 * num_kv_heads &&
+      4ll * batch * num_kv_heads > (int64_t)cps * sm_count())
+    L.ctas = cps = 3;   // several rounds (below)
+  L.stages = head_dim == 128 ? (L.ctas == 3 ? 4 : 6) : 8;
   if (cps == 1 && L.stages < 8) L.stages = 8;
   if (g_ring_stages > 0) L.stages = g_ring_stages;
   if (L.stages > kMaxStages) L.stages = kMaxStages;
@@ -869,22 +878,29 @@ size_t attention_counters_offset(int batch, int num_heads, int num_kv_heads, int
   return 0;
 }
 
-template <int D, int GQM>
+template <int D, int GQM, int CTAS>
 static tb_status launch_attn(const AttnParams& p, const cudaLaunchConfig_t& cfg) {
   if (cfg.dynamicSmemBytes > 32 * 1024)
-    TB_CUDA_TRY(cudaFuncSetAttribute(attn_decode_kernel<D, GQM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TB_CUDA_TRY(cudaFuncSetAttribute(attn_decode_kernel<D, GQM, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)cfg.dynamicSmemBytes));
-  TB_CUDA_TRY(cudaLaunchKernelEx(&cfg, attn_decode_kernel<D, GQM>, p));
+  TB_CUDA_TRY(cudaLaunchKernelEx(&cfg, attn_decode_kernel<D, GQM, CTAS>, p));
   return TB_OK;
 }
 
 template <int D>
-static tb_status launch_attn_d(const AttnParams& p, const cudaLaunchConfig_t& cfg, int gqm) {
+static tb_status launch_attn_d(const AttnParams& p, const cudaLaunchConfig_t& cfg, int gqm, int ctas) {
+  if constexpr (D == 128) {
+    if (ctas == 3) {
+      if (gqm == 1) return launch_attn<D, 1, 3>(p, cfg);
+      if (gqm == 2) return launch_attn<D, 2, 3>(p, cfg);
+      return launch_attn<D, 4, 3>(p, cfg);
+    }
+  }
   switch (gqm) {
-    case 1: return launch_attn<D, 1>(p, cfg);
-    case 2: return launch_attn<D, 2>(p, cfg);
-    case 4: return launch_attn<D, 4>(p, cfg);
-    default: return launch_attn<D, 8>(p, cfg);
+    case 1: return launch_attn<D, 1, 2>(p, cfg);
+    case 2: return launch_attn<D, 2, 2>(p, cfg);
+    case 4: return launch_attn<D, 4, 2>(p, cfg);
+    default: return launch_attn<D, 8, 2>(p, cfg);
   }
 }
 
@@ -953,9 +969,9 @@ tb_status launch_attention_decode(const AttnArgs& a, cudaStream_t stream) {
   p.qkv_rot_out = a.q_rot_out;
   p.num_heads = a.num_heads; p.num_kv_heads = a.num_kv_heads; p.gq = gq;
   p.fixed_per = L.fixed_per; p.batch = a.batch; p.nc = L.nc; p.stages = L.stages;
-  // two CTAs per SM when the ring can be cut to make room (wide heads with many q heads per kv head)
+  // two (three) CTAs per SM when the ring can be cut to make room (wide heads with many q heads per kv head)
   int stages = L.stages;
-  while (stages > 3 && 2 * (sizeof(float) * (attn_fixed_floats(D, gq, gqm) + attn_region_floats(D, gq, L.nc, stages)) + 2048) > 227 * 1024)
+  while (stages > 3 && L.ctas * (sizeof(float) * (attn_fixed_floats(D, gq, gqm, chunk_rows(L.ctas)) + attn_region_floats(D, gq, L.nc, stages)) + 2048) > 227 * 1024)
     --stages;
   p.stages = stages;
   const size_t region = attn_region_floats(D, gq, L.nc, stages);
@@ -966,7 +982,7 @@ tb_status launch_attention_decode(const AttnArgs& a, cudaStream_t stream) {
   p.scale = 1.0f / sqrtf((float)a.head_dim);
   p.tl = timeline_next_block();
 
-  const size_t smem = sizeof(float) * (attn_fixed_floats(D, gq, gqm) + region);
+  const size_t smem = sizeof(float) * (attn_fixed_floats(D, gq, gqm, chunk_rows(L.ctas)) + region);
   if (smem > 200 * 1024) return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: attention needs %zu bytes of shared memory", smem);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)L.grid, (unsigned)a.num_kv_heads);
@@ -982,9 +998,9 @@ tb_status launch_attention_decode(const AttnArgs& a, cudaStream_t stream) {
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  if (D == 128) return launch_attn_d<128>(p, cfg, gqm);
-  if (D == 64) return launch_attn_d<64>(p, cfg, gqm);
-  return launch_attn_d<32>(p, cfg, gqm);
+  if (D == 128) return launch_attn_d<128>(p, cfg, gqm, L.ctas);
+  if (D == 64) return launch_attn_d<64>(p, cfg, gqm, L.ctas);
+  return launch_attn_d<32>(p, cfg, gqm, L.ctas);
 }
 
 // ---------------------------------------------------------------------------
