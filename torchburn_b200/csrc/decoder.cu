@@ -170,7 +170,7 @@ tb_status enqueue_step(tb_decoder* d, int b, bool debug, cudaEvent_t before_lm_h
   }
   // Narrow models' QKV and output projections too: their kernels (w4_gemv) are short, and so is what they prefetch (0.5B
   // widths, one sequence behind 1024 positions: 800 us a token without, 775 with; 8B widths, whose kernels are others: 600 against 688).
-  const int pm = d->pdl_mask | (b == 1 && d->H < 2048 ? 5 : 0);
+  const int pm = d->pdl_mask | (b == 1 && d->tp == 1 && d->H < 2048 ? 5 : 0);
   int launches = 0;
   if (d->fused_step && b == 1 && !debug && before_lm_head == nullptr) {
     // embedding (+ the first norm's weights and sums of squares), then every layer and lm_head in one kernel
