@@ -35,8 +35,8 @@
 //                cp.async, every 16 bytes of a warp's 32 rows are 32 different lines: the shared-memory pipe was
 //                busy with them half of the time and every read of the ring waited ~500 cycles behind them.)
 //
-// CTAs are persistent: every role walks the CTA's list of tiles by itself, so a tile's prologue and epilogue lie
-// under its neighbours' streaming.  Every wait is bounded.  No cluster features, no multicast.
+// CTAs are persistent: every role walks the CTA's list of tiles, or its range of the units of K of all tiles, by itself, so a
+// tile's prologue and epilogue lie under its neighbours' streaming.  Every wait is bounded.  No cluster features, no multicast.
 #include <cuda_bf16.h>
 
 #include "tb_common.cuh"
@@ -59,7 +59,7 @@ constexpr int kSlots = 3;       // accumulator slots of 128 columns; the first 1
 // teams) may wait for a chunk while one up to ten chunks older is still open, and a wait on a barrier two phases ahead
 // would pass at once.
 constexpr uint32_t kRing = 16;
-constexpr int kMaxSplit = 8;    // CTAs that share a tile's K
+constexpr int kMaxSplit = 8;    // most CTAs that share a tile's K
 constexpr int kMaxRows = 512;   // activation rows per launch (bounds the workspace)
 constexpr int kMinRows = 9;     // below: the integer mma.sync kernel
 constexpr int kSureRows = 17;   // from here on always this one, in between the one that costs less (w4_mma_cost)
@@ -73,12 +73,13 @@ struct Tc5Params {
   const float* bias[2];
   const float* resid;
   float* out;
-  float* parts;              // ksplit > 1: sums [tile of rows and weight rows][part][column][128 weight rows]
+  float* parts;              // ranges: sums [CTA][its first tile, its last one][column][128 weight rows]
   int* tickets;              // [tile]: parts that have arrived; zero, and left zero
   const unsigned char* xq;   // [activation tile][64-element chunk of K][piece][MP rows x 128 B], swizzled
   int m;                     // activation rows
   int n, k, ng;
-  int mtiles, ntiles, ksplit, kper;   // tiles of activation rows and of weight rows, CTAs that share a tile's K, K elements of each
+  int mtiles, ntiles;        // tiles of activation rows and of weight rows
+  int per, more;             // ranges: units of K (of all tiles, one after another) of a CTA, the first `more` CTAs take one more; per 0: whole tiles in turn
   int pair;                  // the second weight tile is the up matrix
 };
 
@@ -201,17 +202,31 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_a[kRing], full_b[kRing], done[kRing], full_w[8], empty_w[8], empty_s[8], acc_full[2 * kSlots], acc_empty[kSlots], drained[kSlots];
   __shared__ uint32_t s_tmem;
-  __shared__ int s_abort, s_ticket;
+  __shared__ int s_abort, s_ticket, s_first, s_parts[2], s_tile, s_unit, s_visits;
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int total = p.mtiles * p.ksplit * p.ntiles;
-  const int my_tiles = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int nstages = p.kper / kKC, nunits = p.kper / kUnit, nvisits = p.kper / S::kVk;   // of one tile
+  // The CTA's units of K, numbered from 0, are units g0 ... of its own list of tiles (t0, t0 + ts, ...): a range of all tiles' units,
+  // which may begin and end inside a tile, or whole tiles in turn.
+  const int nunits = p.k / kUnit;   // of one tile
+  const int bx = (int)blockIdx.x, tiles = p.mtiles * p.ntiles;
+  const int g0 = p.per ? bx * p.per + min(bx, p.more) : 0;
+  const int my_units = p.per ? p.per + (bx < p.more ? 1 : 0) : (tiles - bx + (int)gridDim.x - 1) / (int)gridDim.x * nunits;
+  const int t0 = p.per ? 0 : bx, ts = p.per ? 1 : (int)gridDim.x;
   constexpr uint32_t SA = S::kStagesA, SB = S::kStagesB;
 
+  if (p.per && (tid == 32 || tid == 64)) {   // the CTAs that share the CTA's first and its last tile
+    auto cta_of = [&](int unit) {
+      const int wide = p.more * (p.per + 1);
+      return unit < wide ? unit / (p.per + 1) : p.more + (unit - wide) / p.per;
+    };
+    const int t = (tid == 32 ? g0 : g0 + my_units - 1) / nunits, c0 = cta_of(t * nunits);
+    s_parts[tid == 32 ? 0 : 1] = cta_of(t * nunits + nunits - 1) - c0 + 1;
+    if (tid == 32) s_first = c0;
+  }
   if (tid == 0) {
     s_abort = 0;
+    s_tile = t0 + g0 / nunits * ts; s_unit = g0 % nunits; s_visits = my_units * (kUnit / S::kVk);   // where the epilogue begins and ends
     for (uint32_t s = 0; s < kRing; ++s) {
       mbar_init(&full_a[s], S::kTeamTile ? 8 : 4);   // one lane of each unpacking warp of the stage
       mbar_init(&full_b[s], 1);
@@ -250,7 +265,7 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MP >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
       const uint32_t b_lo0 = (smem_u32(smem) >> 4) | (1u << 16);
       const uint32_t d_base = tmem + 128u + me * 128u;
-      const uint32_t nv = (uint32_t)(my_tiles * nvisits);
+      const uint32_t nv = (uint32_t)(my_units * (kUnit / S::kVk));
       bool ok = true;
       uint32_t turn = 0;   // visits of this slot so far
       for (uint32_t v = me; v < nv; v += kSlots, ++turn) {
@@ -298,47 +313,45 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       // ---------------- copies ----------------
       uint32_t c = 0, u = 0;
       bool ok = true;
-      const int chunks = p.k / kKC;
       const uint32_t w_at = smem_u32(smem + S::kOffNib), s_at = smem_u32(smem + S::kOffScale);
       auto weights = [&](uint32_t wu, int t, int i) {   // unit wu of the CTA: unit i of tile t
         const uint32_t ws = wu % S::kUnits, ss = wu % S::kScales;
         if (wu >= S::kUnits) ok = mbar_wait_fast(&empty_w[ws], (wu / S::kUnits - 1u) & 1u, &s_abort);
         if (G == 32 && ok && wu >= S::kScales) ok = mbar_wait_fast(&empty_s[ss], (wu / S::kScales - 1u) & 1u, &s_abort);
         if (!ok) return;
-        const int kz = (t / p.mtiles) % p.ksplit, n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW);
+        const int n0 = t / p.mtiles * (p.pair ? kTileN : kTileN * NW);
         // the scales arrive with the codes: who has seen sums of the unit has seen its scales
         mbar_expect_tx(&full_w[ws], NW * (kUnitBytes + (G == 32 ? kUnitScaleBytes : 0)));
 #pragma unroll
         for (int q = 0; q < NW; ++q)
-          tma_box(w_at + (ws * NW + q) * kUnitBytes, &p.w[p.pair ? q : 0], kz * (p.kper >> 1) + i * 64, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
+          tma_box(w_at + (ws * NW + q) * kUnitBytes, &p.w[p.pair ? q : 0], i * 64, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
         if constexpr (G == 32) {
 #pragma unroll
           for (int q = 0; q < NW; ++q)
-            tma_box(s_at + (ss * NW + q) * kUnitScaleBytes, &p.s[p.pair ? q : 0], kz * (p.kper / G) + i * 4, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
+            tma_box(s_at + (ss * NW + q) * kUnitScaleBytes, &p.s[p.pair ? q : 0], i * 4, n0 + (p.pair ? 0 : q * kTileN), smem_u32(&full_w[ws]));
         }
       };
       // The first weights, a ring of them, do not depend on the pre-pass, which this kernel is launched beside (programmatic
       // serialization); the images do.
       static_assert(S::kScales >= S::kUnits, "scales of the first units");
       uint32_t ahead = 0;
-      for (int t = blockIdx.x, i = 0; t < total && ahead < S::kUnits; ++ahead) {
+      const int tf = t0 + g0 / nunits * ts, i0 = g0 % nunits;   // where the CTA begins
+      for (int t = tf, i = i0; ahead < (uint32_t)my_units && ahead < S::kUnits; ++ahead) {
         weights(ahead, t, i);
-        if (++i == nunits) { i = 0; t += gridDim.x; }
+        if (++i == nunits) { i = 0; t += ts; }
       }
       asm volatile("griddepcontrol.wait;" ::: "memory");
-      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        const int mt = t % p.mtiles, kz = (t / p.mtiles) % p.ksplit;
-        const unsigned char* src = p.xq + ((size_t)mt * chunks + (size_t)kz * nstages) * S::kBBytes;
-        for (int i = 0; i < nunits && ok; ++i, ++u) {
-          if (u >= ahead) weights(u, t, i);
+      for (int t = tf, i = i0; u < (uint32_t)my_units && ok; ++u) {
+        if (u >= ahead) weights(u, t, i);
+        if (!ok) break;
+        const unsigned char* src = p.xq + ((size_t)(t % p.mtiles) * nunits + i) * (2 * S::kBBytes);
+        for (int h = 0; h < 2; ++h, ++c) {
+          if (c >= SB) ok = mbar_wait_fast(&done[(c - SB) % kRing], ((c - SB) / kRing) & 1u, &s_abort);
           if (!ok) break;
-          for (int h = 0; h < 2; ++h, ++c) {
-            if (c >= SB) ok = mbar_wait_fast(&done[(c - SB) % kRing], ((c - SB) / kRing) & 1u, &s_abort);
-            if (!ok) break;
-            mbar_expect_tx(&full_b[c % kRing], S::kBBytes);
-            bulk_g2s(smem + (size_t)(c % SB) * S::kBBytes, src + (size_t)(2 * i + h) * S::kBBytes, S::kBBytes, &full_b[c % kRing]);
-          }
+          mbar_expect_tx(&full_b[c % kRing], S::kBBytes);
+          bulk_g2s(smem + (size_t)(c % SB) * S::kBBytes, src + h * S::kBBytes, S::kBBytes, &full_b[c % kRing]);
         }
+        if (++i == nunits) { i = 0; t += ts; }
       }
       // copies in flight must have landed before the CTA gives its shared memory back (all have, unless a wait was given up)
       if (!ok) {
@@ -361,7 +374,7 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
     const uint32_t ring = smem_u32(smem + S::kOffNib) + (uint32_t)row * 64u;
     const uint32_t swz = (uint32_t)((row >> 1) & 3);
     uint32_t u = (uint32_t)(kTeamTile ? team >> 1 : (S::kDW == 4 ? 0 : team));   // the CTA's units run through all its tiles
-    const uint32_t nu = (uint32_t)(my_tiles * nunits);
+    const uint32_t nu = (uint32_t)my_units;
     bool ok = true;
     for (; u < nu && ok; u += (uint32_t)S::kUnitStride) {
       const uint32_t ws = u % S::kUnits;
@@ -415,51 +428,52 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
     float* ex = reinterpret_cast<float*>(smem + S::kOffEx);
     // 32-element groups: the scales lie in their ring, four a row and unit.  Larger groups: the rows' scales need not start on
     // 16 bytes, so every thread copies its own with cp.async: tile, visit within it, ring slot
-    int ft = blockIdx.x, fv = team;
+    int ft = t0 + g0 / nunits * ts, fv = g0 % nunits * (kUnit / S::kVk) + team;
     uint32_t fs = 0;
     const float* fp[NW];
     auto open_tile = [&](int t) {
-      const int n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW), kz = (t / p.mtiles) % p.ksplit;
+      const int n0 = t / p.mtiles * (p.pair ? kTileN : kTileN * NW);
 #pragma unroll
       for (int q = 0; q < NW; ++q) {
         const int j = n0 + (p.pair ? 0 : q * kTileN) + row;
-        fp[q] = t < total && j < p.n ? (p.pair && q ? p.scales[1] : p.scales[0]) + (size_t)j * p.ng + (size_t)kz * (p.kper / G) : nullptr;
+        fp[q] = j < p.n ? (p.pair && q ? p.scales[1] : p.scales[0]) + (size_t)j * p.ng : nullptr;   // (past the last tile: none)
       }
     };
     open_tile(ft);
     auto fetch = [&]() {
-      while (ft < total && fv >= nvisits) {
-        fv -= nvisits;
-        ft += gridDim.x;
+      while (fv >= p.k / S::kVk) {   // (a few visits past the CTA's last one are fetched, too, and not used)
+        fv -= p.k / S::kVk;
+        ft += p.per ? 1 : (int)gridDim.x;
         open_tile(ft);
       }
-      if (ft < total) {
 #pragma unroll
-        for (int q = 0; q < NW; ++q)
-          if (fp[q] != nullptr)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(sring + fs * (256u * S::kScaleBytes) + (uint32_t)(q * S::kGps * 4)),
-                         "l"(fp[q] + (size_t)fv * S::kGps), "n"(S::kGps * 4)
-                         : "memory");
-        fv += 2;
-      }
+      for (int q = 0; q < NW; ++q)
+        if (fp[q] != nullptr)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(sring + fs * (256u * S::kScaleBytes) + (uint32_t)(q * S::kGps * 4)),
+                       "l"(fp[q] + (size_t)fv * S::kGps), "n"(S::kGps * 4)
+                       : "memory");
+      fv += 2;
       fs = fs + 1 == S::kScales ? 0 : fs + 1;
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if constexpr (G != 32)
 #pragma unroll 1
       for (int i = 0; i < S::kScales - 1; ++i) fetch();
-    uint32_t v = (uint32_t)team, tile_end = 0, rs = 0, at6 = (uint32_t)team, par6 = 0;   // at6: v modulo 6, par6: its round's parity
+    uint32_t v = (uint32_t)team, rs = 0, at6 = (uint32_t)team, par6 = 0;   // at6: v modulo 6, par6: its round's parity
     int read_s = -1;
     bool ok = true;
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-      tile_end += (uint32_t)nvisits;
-      const int mt = t % p.mtiles, kz = (t / p.mtiles) % p.ksplit;
-      const int n0 = (t / (p.mtiles * p.ksplit)) * (p.pair ? kTileN : kTileN * NW);
+    // What only a tile's ends need is read again there: registers are short between them.
+    volatile int* const again = &s_unit;
+    volatile int* const visits = &s_visits;
+    int tile_end = -*again * (kUnit / S::kVk);
+    for (int t = s_tile; tile_end < *visits; t += p.per ? 1 : (int)gridDim.x) {
+      tile_end += p.k / S::kVk;
+      const uint32_t stop = (uint32_t)min(tile_end, *visits);
       float acc[S::kCols];
 #pragma unroll
       for (int i = 0; i < S::kCols; ++i) acc[i] = 0.f;
-      if (p.ksplit > 1 && et == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.tickets + (t / (p.mtiles * p.ksplit) * p.mtiles + mt)));
-      for (; v < tile_end && ok; v += 2) {
+      if (p.per && et == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.tickets + t));
+      for (; v < stop && ok; v += 2) {
         if constexpr (G != 32) {
           asm volatile("cp.async.wait_group %0;" ::"n"(S::kScales - 2) : "memory");
           __syncwarp();
@@ -483,6 +497,9 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
           else if constexpr (S::kGps == 2) asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(sc[q][0]), "=f"(sc[q][S::kGps - 1]) : "r"(a));
           else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc[q][0]) : "r"(a));
         }
+        // Into the slot that the visit before has read.  Here, and not behind the arithmetic, it leaves the registers to the sums: the
+        // pair of 200 rows 4096 -> 14336 with groups of 64 158 -> 153 us.
+        if constexpr (G != 32) fetch();
         const uint32_t slot = at6 >= kSlots ? at6 - kSlots : at6;
         const uint32_t d = lane_base + 128u + slot * 128u;
         constexpr int kN16 = S::kGps * S::kCols / 16;          // 16-column loads of the visit
@@ -511,12 +528,12 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
           if (S::kGps > 1 || (v & 2u)) read_s = (int)(v / kPerUnit % S::kScales);   // this team's last look at the unit's scales
         } else {
           rs = rs + 1 == S::kScales ? 0 : rs + 1;
-          fetch();
           __syncwarp();
         }
         at6 += 2;
         if (at6 >= 2 * kSlots) { at6 -= 2 * kSlots; par6 ^= 1u; }
       }
+      const int mt = t % p.mtiles, n0 = t / p.mtiles * (p.pair ? kTileN : kTileN * NW);
       // ---- the teams' sums: each finishes half of the activation rows ----
       constexpr int kHalf = MP / 2;
       epilogue_barrier();   // the last tile's exchange has been read
@@ -530,27 +547,58 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       for (int q = 0; q < NW; ++q)
 #pragma unroll
         for (int i = 0; i < kHalf; ++i) mine[(q * kHalf + i) * 128] += team ? acc[q * MP + kHalf + i] : acc[q * MP + i];
-      if (p.ksplit > 1) {
+      const int i0 = t == s_tile ? *again : 0;   // the CTA's first unit of the tile
+      if (i0 || tile_end > *visits) {
         // Parts of K: every CTA writes its sums, the last one to arrive adds all of them in the order of the parts, the same
         // order whichever it is, so that equal calls give equal bits.  Sixteen bytes a thread, in short loops: the tail's code
         // comes from memory after every other kernel (a sum per thread and column, unrolled: 2 us more a launch).
-        const int tile = t / (p.mtiles * p.ksplit) * p.mtiles + mt;
+        // The CTAs of the tile follow one another; it is the last tile of the first of them and the first tile of the others.
         constexpr int kPart = S::kCols * 128;   // floats
-        float4* part = reinterpret_cast<float4*>(p.parts + (size_t)tile * p.ksplit * kPart) + et;
+        const int c0 = i0 ? s_first : bx, nparts = s_parts[i0 ? 0 : 1];
+        const float4* rest = reinterpret_cast<const float4*>(p.parts + (size_t)(2 * c0) * kPart) + et;   // part z at 2 z * kPart floats, the first one kPart further
         const bool wide = (p.n & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.resid) | reinterpret_cast<uintptr_t>(p.bias[0])) & 15) == 0;
         epilogue_barrier();   // the teams' sums are complete
+        {
+          float4* part = reinterpret_cast<float4*>(p.parts + (size_t)(2 * bx + (i0 ? 0 : 1)) * kPart) + et;
 #pragma unroll 4
-        for (int i = 0; i < kPart / 4; i += 256) part[kz * (kPart / 4) + i] = reinterpret_cast<const float4*>(ex)[i + et];
+          for (int i = 0; i < kPart / 4; i += 256) part[i] = reinterpret_cast<const float4*>(ex)[i + et];
+        }
         epilogue_barrier();
         if (et == 0) {   // one fence on either side of the ticket, for all threads that the barriers order with it
           __threadfence();
-          const int ticket = atomicAdd(p.tickets + tile, 1);
+          const int ticket = atomicAdd(p.tickets + t, 1);
           __threadfence();
-          if (ticket == p.ksplit - 1) p.tickets[tile] = 0;   // for the next launch
+          if (ticket == nparts - 1) p.tickets[t] = 0;   // for the next launch
           s_ticket = ticket;
         }
         epilogue_barrier();
-        if (s_ticket != p.ksplit - 1 || !ok) continue;
+        if (s_ticket != nparts - 1 || !ok) continue;
+        auto sum_of = [&](int at) {   // at: in float4, behind this thread's first
+          float4 v[kMaxSplit];
+#pragma unroll
+          for (int z = 0; z < kMaxSplit; ++z) v[z] = z < nparts ? __ldcg(rest + (2 * z + (z == 0 ? 1 : 0)) * (kPart / 4) + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int z = 1; z < kMaxSplit; ++z) { v[0].x += v[z].x; v[0].y += v[z].y; v[0].z += v[z].z; v[0].w += v[z].w; }
+          return v[0];
+        };
+        if (NW == 2 && p.pair) {
+#pragma unroll 1
+          for (int i = 0; i < kPart / 8; i += 256) {   // four features of one activation row a thread
+            const int c = (i + et) >> 5, half = c / kHalf;   // column of the gate sums; in either half as many of the up sums follow
+            const int mrow = mt * MP + (half ? 0 : kHalf) + c % kHalf, j = n0 + (et & 31) * 4;
+            if (mrow >= p.m || j >= p.n) continue;
+            const float4 g4 = sum_of(i + half * kHalf * 32), u4 = sum_of(i + (half + 1) * kHalf * 32);
+            const float ga[4] = {g4.x, g4.y, g4.z, g4.w}, up[4] = {u4.x, u4.y, u4.z, u4.w};
+            float* dst = p.out + (size_t)mrow * p.n + j;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (j + e < p.n) {
+                const float a = ga[e] + (p.bias[0] ? p.bias[0][j + e] : 0.f), b = up[e] + (p.bias[1] ? p.bias[1][j + e] : 0.f);
+                dst[e] = (a / (1.0f + expf(-a))) * b;   // src/llm/decoder.rs:1319-1322
+              }
+          }
+          continue;
+        }
 #pragma unroll 1
         for (int i = 0; i < kPart / 4; i += 256) {   // four features of one activation row a thread
           const int c = (i + et) >> 5, q = c / kHalf % NW;
@@ -558,20 +606,16 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
           const int j = n0 + q * kTileN + (et & 31) * 4;
           if (mrow >= p.m || j >= p.n) continue;
           const size_t at = (size_t)mrow * p.n + j;
-          float4 v[kMaxSplit];
-#pragma unroll
-          for (int z = 0; z < kMaxSplit; ++z) v[z] = z < p.ksplit ? __ldcg(part + z * (kPart / 4) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
           float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), add = bias;
           if (wide) {
             if (p.bias[0]) bias = *reinterpret_cast<const float4*>(p.bias[0] + j);
             if (p.resid) add = *reinterpret_cast<const float4*>(p.resid + at);
           }
-#pragma unroll
-          for (int z = 1; z < kMaxSplit; ++z) { v[0].x += v[z].x; v[0].y += v[z].y; v[0].z += v[z].z; v[0].w += v[z].w; }
+          const float4 v = sum_of(i);
           if (wide) {
-            *reinterpret_cast<float4*>(p.out + at) = make_float4(v[0].x + bias.x + add.x, v[0].y + bias.y + add.y, v[0].z + bias.z + add.z, v[0].w + bias.w + add.w);
+            *reinterpret_cast<float4*>(p.out + at) = make_float4(v.x + bias.x + add.x, v.y + bias.y + add.y, v.z + bias.z + add.z, v.w + bias.w + add.w);
           } else {
-            const float o[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+            const float o[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               if (j + e < p.n) p.out[at + e] = o[e] + (p.bias[0] ? p.bias[0][j + e] : 0.f) + (p.resid ? p.resid[at + e] : 0.f);
@@ -733,43 +777,74 @@ constexpr Variant variant() {
 const Variant kVariants[] = {variant<16, 1>(), variant<32, 1>(), variant<48, 1>(), variant<64, 1>(),
                              variant<16, 2>(), variant<32, 2>(), variant<48, 2>(), variant<64, 2>()};
 
-// What a launch costs, in microseconds, pre-pass included, fitted to sweeps of every variant and split over 9 to 333 rows and the
-// projections of the 8B and 0.5B widths (rms 8%; the plan it picks is within 1% of the best one on average, 17% at worst): a
-// stage of 64 elements takes 0.24 + 0.0023 MP (one weight tile) or 0.43 + 0.0044 MP (two) with 32-element groups - the
-// roles' instruction chains, not HBM or the tensor pipe (0.44 at 64 x 2) - and about 0.85 of that with larger ones; a tile's
-// end 0.05 per accumulator column; a split of K two block-wide exchanges through memory and 0.024 per column and part, which
-// the last CTA reads.
+// Whole tiles in turn leave SMs idle when they do not fill the last wave: 112 CTAs of 148 for a gate/up pair of 14336 features or for
+// 4096 features and 333 rows.  A range of units of K for every CTA, which may begin and end inside a tile, leaves none, but
+// the ends cost an exchange through memory: an end 2.2 + 0.022 per accumulator column, and what the last CTA of a tile reads.
+// Measured, whole tiles (or equal parts) / ranges over all SMs: 333 x 14336 -> 4096 153 / 127 us, the pair of 200 rows 4096 -> 14336
+// 180 / 166, of 100 rows 105 / 99, of 16 rows 39.0 / 35.8; but 333 x 4096 -> 6144 53 / 63 and small matrices 11 / 14.
+// The cost of a launch in microseconds, pre-pass included, fitted to 399 plans of 26 calls (every variant, 16 to 333 rows, the
+// projections of the 8B and 0.5B widths; near the best plan rms 3%; the plan it picks is 0.5% from the best on average, 3%
+// at worst): a stage of 64 elements takes what kStage says - the roles' instruction chains, not HBM or the tensor pipe -,
+// a tile's end 0.057 per accumulator column.
 constexpr int kPadRows = 64;   // padding of the last tile: less than the largest tile
 constexpr int kTickets = 1024;
-struct Plan { const Variant* v; int mtiles, ntiles, ksplit; double cost; };
-double plan_cost(const Variant& v, int m, int64_t n, int64_t k, int g, bool pair, int ks, int sms, Plan* plan) {
-  const int rows = pair ? kTileN : kTileN * v.nw;
-  plan->v = &v; plan->ksplit = ks;
-  plan->mtiles = (m + v.mp - 1) / v.mp;
-  plan->ntiles = (int)((n + rows - 1) / rows);
-  const int64_t tiles = (int64_t)plan->mtiles * plan->ntiles * ks;
-  const int64_t waves = (tiles + sms - 1) / sms;
-  const double stage = (v.nw == 2 ? 0.43 + 0.0044 * v.mp : 0.24 + 0.0023 * v.mp) * (g > 32 ? 0.85 : 1.0);
-  const double cols = v.mp * v.nw;
-  return (double)waves * ((double)(k / ks / kKC) * stage + 0.05 * cols + (ks > 1 ? 3.0 + 0.024 * cols * ks : 0.0)) + 5.0;
+constexpr double kStage[2][4] = {{0.300, 0.314, 0.363, 0.393}, {0.49, 0.546, 0.649, 0.660}};   // one or two weight tiles, 16 to 64 rows
+struct Plan { const Variant* v; int mtiles, ntiles, grid, per, more; double cost; };   // per, more: Tc5Params
+double plan_cost(const Plan& p, int64_t k, int g) {
+  const double stage = kStage[p.v->nw - 1][p.v->mp / 16 - 1] * (g > 32 ? 0.95 : 1.0), cols = p.v->mp * p.v->nw;
+  const int64_t tiles = (int64_t)p.mtiles * p.ntiles, ku = k / kUnit;
+  const double prep = 3.5 + 0.19e-3 * (double)k;
+  if (p.per == 0) return (double)((tiles + p.grid - 1) / p.grid) * ((double)(k / kKC) * stage + 0.057 * cols) + prep;
+  const int units = p.per + (p.more ? 1 : 0);
+  const double share = (double)units / (double)ku;                                                    // of a tile, or tiles, a CTA
+  const double ends = share >= 1.0 ? share + 1.0 : (p.more == 0 && ku % units == 0 ? 1.0 : 1.0 + share);   // tiles that a CTA ends or leaves
+  const double shared = ends < 2.0 ? ends : 2.0, parts = share >= 1.0 ? 2.0 : (double)p.grid / (double)tiles;
+  return units * (kUnit / kKC) * stage + ends * 0.057 * cols + shared * (2.2 + 0.022 * cols + 0.0026 * cols * parts) + prep;
 }
-// Parts of a split of K: 32768 columns of partial sums per row (4096 x 14336 in 8 parts), 40 MB at most (301 rows of it in 7).
+// At 9 to 16 rows, the choice between this kernel and the integer one: whole tiles or equal parts of K, as they were measured against
+// each other (w4_mma_cost).  A launch of ranges may take less; calls that it would move are left where they are.
+double few_rows_cost(int m, int64_t n, int64_t k, int g, bool pair) {
+  double best = 1e30;
+  for (int nw = pair ? 2 : 1; nw <= 2; ++nw)
+    for (int mp = 16; mp <= 64; mp += 16)
+      for (int ks = 1; ks <= kMaxSplit; ++ks) {
+        if (ks > 1 && (pair || (k / kUnit) % ks != 0)) continue;
+        const int rows = pair ? kTileN : kTileN * nw;
+        const int64_t tiles = (int64_t)((m + mp - 1) / mp) * ((n + rows - 1) / rows) * ks;
+        const double stage = (nw == 2 ? 0.43 + 0.0044 * mp : 0.24 + 0.0023 * mp) * (g > 32 ? 0.85 : 1.0), cols = mp * nw;
+        const double c = (double)((tiles + sm_count() - 1) / sm_count()) * ((double)(k / ks / kKC) * stage + 0.05 * cols + (ks > 1 ? 3.0 + 0.024 * cols * ks : 0.0)) + 5.0;
+        if (c < best) best = c;
+      }
+  return best;
+}
+// Parts of K: 32768 columns of partial sums per row (4096 x 14336 in 8 parts), 40 MB at most.
 size_t part_bytes(int m) {
   const size_t rows = (size_t)(m < kMaxRows ? m : kMaxRows) + kPadRows;
   return (rows < 320 ? rows : 320) * 32768 * sizeof(float);
 }
-size_t part_bytes_of(const Plan& p) { return (size_t)p.mtiles * p.ntiles * p.ksplit * p.v->mp * p.v->nw * kTileN * sizeof(float); }
 Plan choose_plan(int m, int64_t n, int64_t k, int g, bool pair) {
   const int sms = sm_count();
-  Plan best{}, cur{};
-  double best_cost = 1e30;
+  Plan best{};
+  best.cost = 1e30;
   for (const Variant& v : kVariants) {
     if (pair && v.nw != 2) continue;
-    for (int ks = 1; ks <= kMaxSplit; ++ks) {
-      if (ks > 1 && (pair || (k / kUnit) % ks != 0)) continue;   // (the SwiGLU of a split would want both matrices' parts)
-      const double c = plan_cost(v, m, n, k, g, pair, ks, sms, &cur);
-      if (ks > 1 && (cur.mtiles * cur.ntiles > kTickets || part_bytes_of(cur) > part_bytes(m))) continue;
-      if (c < best_cost) { best_cost = c; best = cur; best.cost = c; }
+    const int rows = pair ? kTileN : kTileN * v.nw;
+    Plan p{&v, (m + v.mp - 1) / v.mp, (int)((n + rows - 1) / rows), 0, 0, 0, 0.0};
+    const int64_t tiles = (int64_t)p.mtiles * p.ntiles, ku = k / kUnit;
+    p.grid = (int)(tiles < sms ? tiles : sms);
+    p.cost = plan_cost(p, k, g);
+    if (p.cost < best.cost) best = p;
+    if (tiles > kTickets) continue;
+    // Ranges of units: one CTA per SM, or as many as leave every tile the same number of parts
+    for (int parts = 0; parts <= kMaxSplit; ++parts) {
+      const int64_t grid = parts ? tiles * parts : sms;
+      if (parts == 1 || grid > sms || grid > tiles * ku) continue;
+      if (2 * (size_t)grid * v.mp * v.nw * kTileN * sizeof(float) > part_bytes(m)) continue;
+      p.grid = (int)grid; p.per = (int)(tiles * ku / grid); p.more = (int)(tiles * ku % grid);
+      if (p.more == 0 && p.per % ku == 0) continue;   // whole tiles
+      if ((p.more == 0 && ku % p.per == 0 ? ku / p.per : (ku - 2) / p.per + 2) > kMaxSplit) continue;
+      p.cost = plan_cost(p, k, g);
+      if (p.cost < best.cost) best = p;
     }
   }
   return best;
@@ -786,7 +861,7 @@ int tc5_fault_flag() {
   return v;
 }
 
-// Images, then the parts of a split of K.
+// Images, then the parts of K.
 size_t w4_tc5_scratch_bytes(int m, int64_t k) {
   const int rows = (m < kMaxRows ? m : kMaxRows) + kPadRows;
   return image_bytes(rows, (k + kKC - 1) / kKC * kKC) + part_bytes(m);
@@ -798,7 +873,7 @@ bool w4_tc5_supported(const GemvArgs& a) {
   if (a.x_ss8 || a.out_scaled || a.out_ss8 || a.x_normed_out) return false;
   if ((reinterpret_cast<uintptr_t>(a.w) & 15) || (a.w2 && (reinterpret_cast<uintptr_t>(a.w2) & 15))) return false;
   if ((reinterpret_cast<uintptr_t>(a.scales) & 15) || (a.w2 && (reinterpret_cast<uintptr_t>(a.scales2) & 15))) return false;   // boxes and copies of up to 16 bytes
-  return a.m >= kSureRows || choose_plan(a.m, a.n, a.k, a.g, a.w2 != nullptr).cost < w4_mma_cost(a.n, a.k, a.w2 != nullptr);
+  return a.m >= kSureRows || few_rows_cost(a.m, a.n, a.k, a.g, a.w2 != nullptr) < w4_mma_cost(a.n, a.k, a.w2 != nullptr);
 }
 
 // Launches of one call: kMaxRows rows at a time, the pre-pass and the product.
@@ -822,7 +897,7 @@ tb_status launch_w4_tc5(const GemvArgs& a, void* scratch, int* tickets, cudaStre
     p.parts = reinterpret_cast<float*>(xq + image_bytes(plan.mtiles * v.mp, a.k));
     p.tickets = tickets;
     p.m = mc; p.n = (int)a.n; p.k = (int)a.k; p.ng = (int)(a.k / a.g);
-    p.mtiles = plan.mtiles; p.ntiles = plan.ntiles; p.ksplit = plan.ksplit; p.kper = (int)(a.k / plan.ksplit);
+    p.mtiles = plan.mtiles; p.ntiles = plan.ntiles; p.per = plan.per; p.more = plan.more;
     p.pair = pair ? 1 : 0;
     for (int q = 0; q < (pair ? 2 : 1); ++q) {
       if (!tma_matrix_map(&p.w[q], CU_TENSOR_MAP_DATA_TYPE_UINT8, q ? a.w2 : a.w, a.k / 2, a.n, a.k / 2, 64, kTileN, CU_TENSOR_MAP_SWIZZLE_64B) ||
@@ -836,14 +911,12 @@ tb_status launch_w4_tc5(const GemvArgs& a, void* scratch, int* tickets, cudaStre
     prep<<<(unsigned)(plan.mtiles * v.mp), threads, 0, stream>>>(a.x + (size_t)m0 * a.k, a.norm_w, a.eps, xq, mc, v.mp, (int)a.k);
     TB_CUDA_TRY(cudaGetLastError());
     TB_CUDA_TRY(cudaFuncSetAttribute(v.kern[gi], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem[gi]));
-    const int64_t tiles = (int64_t)plan.mtiles * plan.ntiles * plan.ksplit;
-    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     // Beside the pre-pass (which itself starts when all in front of it is complete): the tensor memory, the barriers and the first
     // ring of weights are ready when the images are.  The MLP of 16 rows at 4096 / 14336: 71.1 -> 66.2 us; 333 rows gain nothing.
     // (Weights that ran ahead of the images all the way, not only by the first ring, cost 27 -> 40 us at 16 x 14336 x 4096: the
     // copying thread's wait for a unit held back images that others waited for.)
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = dim3((unsigned)plan.grid);
     cfg.blockDim = dim3((unsigned)v.threads[gi]);
     cfg.dynamicSmemBytes = v.smem[gi];
     cfg.stream = stream;
