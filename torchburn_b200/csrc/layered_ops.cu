@@ -125,31 +125,64 @@ __global__ void __launch_bounds__(kThreads) residual_norm_kernel(const GlueArgs 
     if (!(tok >= 0 && tok < a.vocab && pos >= 0 && pos < a.max_pos)) pos = -1;
     if (tid == 0) a.r.pos[r] = pos;
   }
+  // Four pieces of the row at a time, all their loads in flight before the first of them is used, and the residual's first ones in
+  // front of the block sum: a row is two passes of one or two trips to memory (512 rows of 4096: 9.3 us with a trip
+  // per piece, 7.7 so).
   float inv = 1.f;
   float ss[1] = {0.f};
-  for (int e = 0, i = tid; i < xs4; ++e, i += kThreads) {
-    float4 v = f4(0.f);
+  for (int e0 = 0; e0 < e4; e0 += 4) {
+    float4 v[4];
     if (!emb) {
-      v = sum_partials(a.y, r, i * 4);
-      if (a.y_bias) v = add4(v, ld4(a.y_bias + i * 4));
-    } else if (pos >= 0) {
-      v = embed4(a, tok, pos, i * 4);
+      const float* p = a.y.y + (size_t)r * a.y.ldy;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = (e0 + u) * kThreads + tid < xs4 ? ld4(p + ((e0 + u) * kThreads + tid) * 4) : f4(0.f);
+      for (int z = 1; z < a.y.splits; ++z) {
+        float4 t[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) t[u] = (e0 + u) * kThreads + tid < xs4 ? ld4(p + (size_t)z * a.y.split_stride + ((e0 + u) * kThreads + tid) * 4) : f4(0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = add4(v[u], t[u]);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = pos >= 0 && (e0 + u) * kThreads + tid < xs4 ? embed4(a, tok, pos, ((e0 + u) * kThreads + tid) * 4) : f4(0.f);
     }
-    s_dyn[e * kThreads + tid] = v;
-    ss[0] += dot4(v);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = (e0 + u) * kThreads + tid;
+      if (i >= xs4) break;
+      if (!emb && a.y_bias) v[u] = add4(v[u], ld4(a.y_bias + i * 4));
+      s_dyn[i] = v[u];
+      ss[0] += dot4(v[u]);
+    }
   }
+  float4 xv[4], pw[4];
+  auto fetch = [&](int e0) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = (e0 + u) * kThreads + tid;
+      xv[u] = !emb && i < xs4 ? ld4(a.x_in + (size_t)r * a.xs + i * 4) : f4(0.f);
+      pw[u] = a.post_w && i < xs4 ? ld4(a.post_w + i * 4) : f4(0.f);
+    }
+  };
+  fetch(0);
   if (a.post_w) {
     cluster_sum<1>(s_sum, 0, 1, 0, ss);
     inv = 1.0f / sqrtf(ss[0] / (float)a.width + a.eps);
   }
   ss[0] = 0.f;
-  for (int e = 0, i = tid; i < xs4; ++e, i += kThreads) {
-    const float4 y = s_dyn[e * kThreads + tid];
-    float4 v = emb ? f4(0.f) : ld4(a.x_in + (size_t)r * a.xs + i * 4);
-    v = a.post_w ? fma4(scale4(y, inv), ld4(a.post_w + i * 4), v) : add4(v, y);
-    ss[0] += dot4(v);
-    *reinterpret_cast<float4*>(a.x_out + (size_t)r * a.xs + i * 4) = v;
-    if (a.snapshot) *reinterpret_cast<float4*>(a.snapshot + (size_t)r * a.xs + i * 4) = v;
+  for (int e0 = 0; e0 < e4; e0 += 4) {
+    if (e0) fetch(e0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = (e0 + u) * kThreads + tid;
+      if (i >= xs4) break;
+      const float4 y = s_dyn[i];
+      const float4 v = a.post_w ? fma4(scale4(y, inv), pw[u], xv[u]) : add4(xv[u], y);
+      ss[0] += dot4(v);
+      *reinterpret_cast<float4*>(a.x_out + (size_t)r * a.xs + i * 4) = v;
+      if (a.snapshot) *reinterpret_cast<float4*>(a.snapshot + (size_t)r * a.xs + i * 4) = v;
+    }
   }
   cluster_sum<1>(s_sum, 0, 1, 0, ss);
   if (tid == 0) a.rstd[r] = 1.0f / sqrtf(ss[0] / (float)a.width + a.eps);
@@ -183,6 +216,60 @@ __global__ void __launch_bounds__(kThreads) norm_conv_kernel(const GlueArgs a) {
   }
   if (pos < 0) o = f4(0.f);
   act_store4<BF16>(a.out, orow, i * 4, o);
+}
+
+// The same for at most four taps: four rows a block, whose inputs, with the three rows in front of them, are loaded once and all at
+// the same time.  A row a block took its taps one after the other, each two dependent trips to memory behind the row before it
+// (512 rows of 4096, four taps: 10.2 us; 6.6 so, two or eight rows a block the same).  grid (rows / 4, columns / 1024)
+constexpr int kConvRows = 4, kConvTaps = 4;
+template <bool BF16>
+__global__ void __launch_bounds__(kThreads, 3) norm_conv_rows_kernel(const GlueArgs a) {
+  constexpr int N = kConvRows + kConvTaps - 1;
+  const int r0 = a.row0 + (int)blockIdx.x * kConvRows, i = (int)blockIdx.y * kThreads + threadIdx.x;
+  const int taps = a.conv_w != nullptr ? a.taps : 1, first = kConvTaps - taps;   // rows from `first` on are needed
+  grid_dep_launch();
+  if (i >= (a.xs >> 2)) return;
+  const float4 pw = ld4(a.pre_w + i * 4);
+  float4 w[kConvTaps];
+#pragma unroll
+  for (int j = 0; j < kConvTaps; ++j) w[j] = a.conv_w != nullptr && j < taps ? ld4(a.conv_w + (size_t)(taps - 1 - j) * a.xs + i * 4) : f4(0.f);
+  grid_dep_wait();
+  int pos[N], slot[N];
+  float rs[N];
+  float4 h[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {   // row r0 - 3 + k
+    const int q = r0 - (kConvTaps - 1) + k;
+    const bool in = k >= first && q >= 0 && q < a.r.rows;
+    pos[k] = in ? a.r.pos[q] : -1;
+    slot[k] = in ? a.r.slots[q] : -1;
+    rs[k] = in ? a.rstd[q] : 0.f;
+    h[k] = in ? ld4(a.x_out + (size_t)q * a.xs + i * 4) : f4(0.f);
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) h[k] = mul4(scale4(h[k], rs[k]), pw);
+#pragma unroll
+  for (int m = 0; m < kConvRows; ++m) {
+    constexpr int kAt = kConvTaps - 1;
+    const int r = r0 + m, at = m + kAt, p = pos[at];
+    if (r >= a.r.rows) break;
+    if (a.write_state && p >= 0) *reinterpret_cast<float4*>(a.conv_state + ((size_t)slot[at] * a.ring + (p & (a.ring - 1))) * a.xs + i * 4) = h[at];
+    const int orow = a.row_map != nullptr ? a.row_map[r] : r;
+    if (a.out.data == nullptr || orow < 0) continue;
+    float4 o = h[at];
+    if (a.conv_w != nullptr) {
+#pragma unroll
+      for (int j = 0; j < kConvTaps; ++j) {
+        if (j >= taps || j > p) break;
+        float4 hp = h[at - j];
+        if (j > 0 && !(r - j >= 0 && slot[at - j] == slot[at] && pos[at - j] == p - j))
+          hp = ld4(a.conv_state + ((size_t)slot[at] * a.ring + ((p - j) & (a.ring - 1))) * a.xs + i * 4);
+        o = fma4(w[j], hp, o);
+      }
+    }
+    if (p < 0) o = f4(0.f);
+    act_store4<BF16>(a.out, orow, i * 4, o);
+  }
 }
 
 // grid: (rows / rows_per * csize); rows_per consecutive rows per cluster, after up to taps - 1 rows of the same
@@ -722,6 +809,11 @@ tb_status launch_glue(Precision p, const GlueArgs& a, cudaStream_t st) {
     if (a.taps > 32 || e4 > 50) return fail(TB_ERR_UNSUPPORTED, "TB_UNSUPPORTED: hidden size %d with %d taps", a.width, a.taps);
     if (a.row0 == 0)
       TB_TRY(launch_kernel(residual_norm_kernel, dim3((unsigned)n), dim3(kThreads), (size_t)e4 * kThreads * sizeof(float4), st, a.pdl, 1, a, e4));
+    if (n >= 256 && (a.conv_w == nullptr || a.taps <= kConvTaps)) {   // fewer rows leave SMs without a block of four
+      const dim3 grid((unsigned)((n + kConvRows - 1) / kConvRows), (unsigned)e4);
+      return p == Precision::kBf16 ? launch_kernel(norm_conv_rows_kernel<true>, grid, dim3(kThreads), 0, st, a.pdl, 1, a)
+                                   : launch_kernel(norm_conv_rows_kernel<false>, grid, dim3(kThreads), 0, st, a.pdl, 1, a);
+    }
     const dim3 grid((unsigned)n, (unsigned)e4);
     return p == Precision::kBf16 ? launch_kernel(norm_conv_kernel<true>, grid, dim3(kThreads), 0, st, a.pdl, 1, a)
                                  : launch_kernel(norm_conv_kernel<false>, grid, dim3(kThreads), 0, st, a.pdl, 1, a);
