@@ -237,6 +237,11 @@ typedef struct tb_linear tb_linear;
 tb_status tb_linear_create(tb_linear** out, const uint8_t* qweight, const float* scales,
                            const float* bias, int64_t out_features, int64_t in_features,
                            int32_t group_size, tb_space weight_space);
+/* The same over DEVICE memory of the caller's: nothing is copied, every call reads what the memory then holds, and it has to stay
+ * until the last of them is done on its stream.  tb_linear_destroy frees the handle alone. */
+tb_status tb_linear_view(tb_linear** out, const uint8_t* qweight, const float* scales,
+                         const float* bias, int64_t out_features, int64_t in_features,
+                         int32_t group_size);
 void tb_linear_destroy(tb_linear* lin);
 
 /* The interleaved "v2" weight layout (src/quantization/packed_v2.rs:26-143,

@@ -228,6 +228,7 @@ extern "C" {
     pub fn tb_release_workspaces();
     pub fn tb_device_fault_flag() -> i32;
     pub fn tb_linear_create(out: *mut *mut tb_linear, qweight: *const u8, scales: *const f32, bias: *const f32, out_features: i64, in_features: i64, group_size: i32, weight_space: tb_space) -> tb_status;
+    pub fn tb_linear_view(out: *mut *mut tb_linear, qweight: *const u8, scales: *const f32, bias: *const f32, out_features: i64, in_features: i64, group_size: i32) -> tb_status;
     pub fn tb_linear_destroy(lin: *mut tb_linear);
     pub fn tb_f32_to_f16(value: f32) -> u16;
     pub fn tb_f16_to_f32(bits: u16) -> f32;

@@ -108,6 +108,7 @@ SIGNATURES = {
     "tb_release_workspaces": (None, []),
     "tb_device_fault_flag": (_i32, []),
     "tb_linear_create": (_i32, [_PP, _p, _p, _p, _i64, _i64, _i32, _i32]),
+    "tb_linear_view": (_i32, [_PP, _p, _p, _p, _i64, _i64, _i32]),
     "tb_f32_to_f16": (C.c_uint16, [_f32]),
     "tb_f16_to_f32": (_f32, [C.c_uint16]),
     "tb_pack_v1_to_v2": (_i32, [_p, _p, _i64, _i64, _p]),

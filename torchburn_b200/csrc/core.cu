@@ -82,6 +82,7 @@ struct tb_linear {
   int64_t n = 0, k = 0;
   int g = 0;
   int device = 0;
+  bool owner = true;   // false: the weights are the caller's (tb_linear_view)
   // pinned + device staging for host callers, grown on demand
   float *h_x = nullptr, *h_out = nullptr, *d_x = nullptr, *d_out = nullptr;
   int64_t stage_m = 0;
@@ -287,9 +288,27 @@ tb_status tb_linear_create(tb_linear** out, const uint8_t* qweight, const float*
   return TB_OK;
 }
 
+tb_status tb_linear_view(tb_linear** out, const uint8_t* qweight, const float* scales, const float* bias,
+                         int64_t out_features, int64_t in_features, int32_t group_size) {
+  if (!out) return fail(TB_ERR_ARG, "tb_linear_view: null out");
+  *out = nullptr;
+  if (!qweight || !scales) return fail(TB_ERR_ARG, "tb_linear_view: null weight");
+  TB_TRY(check_linear_shape(out_features, in_features, group_size));
+  tb_linear* lin = new (std::nothrow) tb_linear();
+  if (!lin) return fail(TB_ERR_OOM, "tb_linear_view: host allocation failed");
+  lin->n = out_features; lin->k = in_features; lin->g = group_size;
+  cudaGetDevice(&lin->device);
+  lin->owner = false;
+  lin->qweight = const_cast<uint8_t*>(qweight);
+  lin->scales = const_cast<float*>(scales);
+  lin->bias = const_cast<float*>(bias);
+  *out = lin;
+  return TB_OK;
+}
+
 void tb_linear_destroy(tb_linear* lin) {
   if (!lin) return;
-  cudaFree(lin->qweight); cudaFree(lin->scales); cudaFree(lin->bias);
+  if (lin->owner) { cudaFree(lin->qweight); cudaFree(lin->scales); cudaFree(lin->bias); }
   cudaFreeHost(lin->h_x); cudaFreeHost(lin->h_out); cudaFree(lin->d_x); cudaFree(lin->d_out);
   delete lin;
 }

@@ -219,22 +219,25 @@ class QuantizedLinear(nn.Module):
 
 
 class _LinearHandle:
-    """tb_linear over a module's (or raw tensors') weights; uploads once."""
+    """tb_linear over a module's weights: the module's own device memory (a view), or a copy of it on the device."""
 
-    def __init__(self, qweight, scales, bias, group_size):
-        qweight = qweight.contiguous()
-        scales = scales.contiguous().float()
-        bias = bias.detach().contiguous().float() if bias is not None else None
+    def __init__(self, qweight, scales, bias, group_size, view=False):
         n, k = qweight.shape[0], qweight.shape[1] * 2
-        space = TB_DEVICE if qweight.device.type == "cuda" else TB_HOST
-        if space == TB_DEVICE:
-            scales = scales.to(qweight.device)
-            bias = bias.to(qweight.device) if bias is not None else None
         h = C.c_void_p()
-        check(lib().tb_linear_create(C.byref(h), qweight.data_ptr(), scales.data_ptr(),
-                                     bias.data_ptr() if bias is not None else None, n, k, group_size, space))
+        if view:
+            check(lib().tb_linear_view(C.byref(h), qweight.data_ptr(), scales.data_ptr(), bias.data_ptr() if bias is not None else None, n, k, group_size))
+        else:
+            qweight = qweight.contiguous()
+            scales = scales.contiguous().float()
+            bias = bias.detach().contiguous().float() if bias is not None else None
+            space = TB_DEVICE if qweight.device.type == "cuda" else TB_HOST
+            if space == TB_DEVICE:
+                scales = scales.to(qweight.device)
+                bias = bias.to(qweight.device) if bias is not None else None
+            check(lib().tb_linear_create(C.byref(h), qweight.data_ptr(), scales.data_ptr(),
+                                         bias.data_ptr() if bias is not None else None, n, k, group_size, space))
         self.h = h
-        self.n, self.k = n, k
+        self.n, self.k, self.view = n, k, view
 
     def __del__(self):
         if getattr(self, "h", None):
@@ -242,13 +245,40 @@ class _LinearHandle:
             self.h = None
 
 
+def _readable(q, s, b, group_size) -> bool:
+    """Whether the kernels can read these weights where they are: whole, of the right types, on the current device."""
+    if not (q.is_cuda and q.ndim == 2 and q.dtype is torch.uint8 and s.dtype is torch.float32 and q.is_contiguous() and s.is_contiguous()):
+        return False
+    n, index = q.shape[0], q.get_device()
+    return (index == s.get_device() == torch.cuda.current_device() and s.numel() * group_size == n * q.shape[1] * 2
+            and q.data_ptr() % 16 == 0 and s.data_ptr() % 16 == 0
+            and (b is None or (b.dtype is torch.float32 and b.is_contiguous() and b.get_device() == index and b.numel() == n)))
+
+
 def _handle_of(m) -> _LinearHandle:
-    key = (m.qweight.data_ptr(), m.qweight._version, m.scales.data_ptr(), m.scales._version)
+    """The handle of a module's weights, as they are now.  A view reads the module's memory at every call; a copy (weights on the host, on
+    another device, of another type) is made again when one of the tensors is another one or has been written to."""
+    q, s, b = m.qweight, m.scales, m.bias
     cached = getattr(m, "_tb_handle", None)
+    if _readable(q, s, b, m.group_size):
+        key, held = (q.data_ptr(), s.data_ptr(), None if b is None else b.data_ptr(), q.shape, m.group_size), None
+    else:
+        held = (q, s) if b is None else (q, s, b)   # held, so that no other tensor takes an address or id of these
+        key = (m.group_size, *((id(t), t.data_ptr(), object() if t.is_inference() else t._version) for t in held))   # (an inference tensor has no version: copied anew)
     if cached is None or cached[0] != key:
-        cached = (key, _LinearHandle(m.qweight, m.scales, m.bias, m.group_size))
+        cached = (key, _LinearHandle(q, s, b, m.group_size, view=held is None), held)
         object.__setattr__(m, "_tb_handle", cached)
     return cached[1]
+
+
+def _used_on(stream: int, *modules) -> None:
+    """Weights that are read where they are, on a stream of the caller's: their memory is not given to others before that is done."""
+    if stream:
+        now = torch.cuda.current_stream()
+        for m in modules:
+            for t in (m.qweight, m.scales, m.bias):
+                if t is not None and t.is_cuda:
+                    t.record_stream(now)
 
 
 def _io(x: torch.Tensor):
@@ -268,7 +298,9 @@ def fused_swiglu_mlp(x: torch.Tensor, gate_proj, up_proj, down_proj) -> torch.Te
     assert hidden == g.k
     out = torch.empty(list(xf.shape[:-1]) + [d.n], dtype=torch.float32, device=xf.device)
     with torch.cuda.device(dev):
-        check(lib().tb_fused_swiglu_mlp(g.h, u.h, d.h, xf.data_ptr(), m, out.data_ptr(), space, _stream_ptr(dev)))
+        stream = _stream_ptr(dev)
+        _used_on(stream, gate_proj, up_proj, down_proj)
+        check(lib().tb_fused_swiglu_mlp(g.h, u.h, d.h, xf.data_ptr(), m, out.data_ptr(), space, stream))
     return out
 
 
