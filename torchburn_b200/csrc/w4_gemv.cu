@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(WARPS * 32) w4_gemv_kernel(const GemvParams p)
           }
         }
         float amax = abs_max<8>(xv);
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         uint32_t dig[6];
         float sx;
         int S, s8hi, s8lo;

@@ -89,7 +89,7 @@ __device__ __forceinline__ float idot32(const uint4 wv, const uint32_t (&xq)[24]
 }
 
 // Quantises NE consecutive elements of a 32-element block whose maximum magnitude is
-// `amax` (NE = 32: the whole block; 16: one half, the maximum taken over both halves):
+// `amax` (NaN if one of them is; NE = 32: the whole block; 16: one half, the maximum taken over both halves):
 // digits + sx + S = sum(q) of these elements (the -8 offset of the codes contributes -8 * S).
 template <int NE>
 __device__ __forceinline__ void quantize_part_int(const float (&v)[NE], float amax, uint32_t (&dig)[NE / 8 * 6],
@@ -122,11 +122,19 @@ __device__ __forceinline__ void quantize_part_int(const float (&v)[NE], float am
       }
 }
 
+// The larger of two numbers, NaN if either is (fmaxf would drop it, and with it what the caller multiplies by).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return m;
+}
+
+// The largest magnitude; NaN if one of them is.
 template <int NE>
 __device__ __forceinline__ float abs_max(const float (&v)[NE]) {
   float amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < NE; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  for (int i = 0; i < NE; ++i) amax = max_nan(amax, fabsf(v[i]));
   return amax;
 }
 

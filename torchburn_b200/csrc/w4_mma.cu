@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_x_kernel(const float* 
     }
   }
   float amax = abs_max<8>(v);
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
   uint32_t dig[6];
   float sx;
   int sum;

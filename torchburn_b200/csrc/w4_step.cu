@@ -575,7 +575,7 @@ __device__ __forceinline__ uint32_t gemv_phase(const StepPhase& d, const StepPar
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       const float4 t4 = xs[c ^ sw];
-      amax = fmaxf(fmaxf(amax, fmaxf(fabsf(t4.x), fabsf(t4.y))), fmaxf(fabsf(t4.z), fabsf(t4.w)));
+      amax = max_nan(max_nan(amax, max_nan(fabsf(t4.x), fabsf(t4.y))), max_nan(fabsf(t4.z), fabsf(t4.w)));
     }
     int S = 0;
 #pragma unroll

@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(512) w4_stream_kernel(const StreamParams p) {
       }
     }
     float amax = abs_max<EPL>(v);
-    if (EPL == 16) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));  // the block's other half
+    if (EPL == 16) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));  // the block's other half
     int S;
     quantize_part_int<EPL>(v, amax, dig, sx, S);
     split_offset(S, s8hi, s8lo);
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(512) w4_stream_rows_kernel(const RowsParams p)
         }
       }
       float amax = abs_max<EPL>(v);
-      if (EPL == 16) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+      if (EPL == 16) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
       int S;
       quantize_part_int<EPL>(v, amax, dig[m], sx[m], S);
       split_offset(S, s8hi[m], s8lo[m]);
