@@ -79,3 +79,40 @@ def test_few_rows_keep_infinities_to_their_row(torch, tb):
     keep = [0, 1, 3, 5]
     assert torch.equal(got[keep], want[keep])
     assert bool(torch.isnan(got[4]).all()) and not bool(torch.isfinite(got[2]).any())
+
+
+@pytest.mark.parametrize("pair", [0, 1])
+@pytest.mark.parametrize("m,n,k,g", [(2, 700, 896, 32), (3, 6000, 1024, 64), (4, 4097, 512, 128), (5, 96, 8192, 32), (8, 5003, 4096, 32), (8, 600, 14336, 32), (6, 9600, 256, 32)])
+def test_the_integer_kernel_stays_selectable(torch, tb, m, n, k, g, pair):
+    """tb_set_gemv_tuning(3, ...) takes these products to the integer kernel: other bits than the default's, within the bound of
+    its arithmetic (the streaming kernel's for the sums, and half a step of 2^-22 of a block's maximum for each of its elements)."""
+    a, b = int4(torch, n, k, g, 1), int4(torch, n, k, g, 2)
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator("cuda").manual_seed(m + k))
+    st = torch.cuda.current_stream().cuda_stream
+
+    def run():
+        y = torch.full((m, n), float("nan"), device="cuda")
+        rc = tb.lib().tb_swiglu_gemv_w4a32(x.data_ptr(), a[0].data_ptr(), a[1].data_ptr(), None, b[0].data_ptr(), b[1].data_ptr(), None, y.data_ptr(), m, n, k, g, st) if pair else \
+            tb.lib().tb_gemm_w4a32_grouped(x.data_ptr(), a[0].data_ptr(), a[1].data_ptr(), None, y.data_ptr(), m, n, k, g, st)
+        assert rc == 0, tb.last_error()
+        return y
+    streamed = run()
+    try:
+        tb.lib().tb_set_gemv_tuning(3, 0, 0)
+        integer = run()
+    finally:
+        tb.lib().tb_set_gemv_tuning(1, 0, 0)
+    assert not torch.equal(integer, streamed)
+    top = x.double().abs().reshape(m, k // 32, 32).amax(-1, keepdim=True).expand(m, k // 32, 32).reshape(m, k)
+
+    def sums(w):
+        d = (4.4 + k / 32 + 10) * 2.0 ** -24 * (x.double().abs() @ w.abs().T)
+        return x.double() @ w.T, d + 2.0 ** -23 * (top @ w.abs().T)
+    (want, d), (up, du) = sums(a[2]), sums(b[2])
+    if pair:
+        silu = torch.nn.functional.silu(want)
+        d = 1.1 * d * (up.abs() + du) + silu.abs() * du + 4 * 2.0 ** -23 * (silu * up).abs()
+        want = silu * up
+    for y in (streamed, integer):
+        assert bool(((y.double() - want).abs() <= d + 1e-30).all())
+    assert tb.lib().tb_device_fault_flag() == 0

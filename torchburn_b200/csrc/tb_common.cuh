@@ -126,6 +126,7 @@ void set_gemv_tuning(int xmode, int rows_per_warp, int warps);
 // Streaming tensor-core kernel for 2 to 8 rows (w4_rows.cu); `scratch` holds w4_rows_scratch_bytes.
 size_t w4_rows_scratch_bytes(int64_t k);
 bool w4_rows_supported(const GemvArgs& a);
+void set_rows_enabled(int enabled);
 tb_status launch_w4_rows(const GemvArgs& a, void* scratch, cudaStream_t stream);
 int rows_fault_flag();
 // Integer tensor-core kernel for 9 and more rows (w4_mma.cu).

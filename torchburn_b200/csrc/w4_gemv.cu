@@ -499,6 +499,7 @@ tb_status launch_epi(int m, const GemvParams& p, bool pdl, cudaStream_t stream) 
 void set_gemv_tuning(int xmode, int rows_per_warp, int warps) {
   g_mma_enabled = xmode == 2 ? 0 : 1;  // 2: integer products on CUDA cores for every M
   set_tc5_enabled(xmode == 3 ? 0 : 1);  // 3: the mma.sync integer kernel for every M
+  set_rows_enabled(xmode == 3 ? 0 : 1);
   g_xmode = xmode != 0 ? 1 : 0;
   g_force_r = rows_per_warp;
   g_force_warps = warps;

@@ -55,6 +55,7 @@ constexpr size_t kSmemMax = 226 * 1024;
 constexpr int kMaxRowsM = 8;
 
 __device__ int g_rows_fault = 0;
+int g_rows_enabled = 1;
 
 struct RowsParams {
   CUtensorMap w[2];          // [n, k / 2] bytes, boxes of 128 x 16 rows (a pair: x 8 rows)
@@ -403,6 +404,8 @@ Plan choose_plan(int64_t n, int g, bool pair) {
 
 }  // namespace
 
+void set_rows_enabled(int enabled) { g_rows_enabled = enabled; }
+
 int rows_fault_flag() {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, g_rows_fault, sizeof(int)) != cudaSuccess) return -1;
@@ -412,7 +415,7 @@ int rows_fault_flag() {
 size_t w4_rows_scratch_bytes(int64_t k) { return (size_t)padded_blocks(k) * kImageBytes; }
 
 bool w4_rows_supported(const GemvArgs& a) {
-  return a.m >= 2 && a.m <= kMaxRowsM && a.k % 32 == 0 && tma_encoder() &&
+  return g_rows_enabled && a.m >= 2 && a.m <= kMaxRowsM && a.k % 32 == 0 && tma_encoder() &&
          !((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.w2) | reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.norm_w)) & 15);
 }
 

@@ -61,7 +61,7 @@ constexpr int kSlots = 3;       // accumulator slots of 128 columns; the first 1
 constexpr uint32_t kRing = 16;
 constexpr int kMaxSplit = 8;    // most CTAs that share a tile's K
 constexpr int kMaxRows = 512;   // activation rows per launch (bounds the workspace)
-constexpr int kMinRows = 9;     // below: the integer mma.sync kernel
+constexpr int kMinRows = 9;     // below: the streaming kernel (w4_rows.cu)
 constexpr int kSureRows = 17;   // from here on always this one, in between the one that costs less (w4_mma_cost)
 
 __device__ int g_tc5_fault = 0;
