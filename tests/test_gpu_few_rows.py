@@ -50,13 +50,16 @@ def test_products_of_few_rows_match_float64(torch, tb, m, n, k, g, pair):
     x = torch.randn(m, k, device="cuda", generator=gen) * 10 ** (6 * torch.rand(m, 1, device="cuda", generator=gen) - 3)
     b = torch.randn(n, device="cuda", generator=gen)
     tol = (4.4 + k / 32 + 10) * 2.0 ** -24
-    if pair:
+    st = torch.cuda.current_stream().cuda_stream
+
+    def run():
+        if not pair:
+            return tb.w4a32_grouped_linear(x, p, s, b, g)
         y = torch.empty(m, n, device="cuda")
-        st = torch.cuda.current_stream().cuda_stream
         assert tb.lib().tb_swiglu_gemv_w4a32(x.data_ptr(), p.data_ptr(), s.data_ptr(), b.data_ptr(), p2.data_ptr(), s2.data_ptr(), None, y.data_ptr(),
                                              m, n, k, g, st) == 0, tb.last_error()
-    else:
-        y = tb.w4a32_grouped_linear(x, p, s, b, g)
+        return y
+    y = run()
     gate, bound = x.double() @ w.T + b, (x.double().abs() @ w.abs().T + b.abs()) * tol
     if pair:
         up, sig = x.double() @ w2.T, torch.sigmoid(gate)
@@ -64,8 +67,7 @@ def test_products_of_few_rows_match_float64(torch, tb, m, n, k, g, pair):
         bound = 1.1 * bound * up.abs() + gate.abs() * (x.double().abs() @ w2.abs().T) * tol + 4 * 2.0 ** -23 * (gate * sig * up).abs() + bound * 1e-6
         gate = gate * sig * up
     assert bool(((y.double() - gate).abs() <= bound + 1e-30).all()), float(((y.double() - gate).abs() / bound).max())
-    if m < y.shape[0] + 1 and not pair:   # equal calls give equal bits
-        assert torch.equal(tb.w4a32_grouped_linear(x, p, s, b, g), y)
+    assert torch.equal(run(), y)   # equal calls give equal bits
     assert tb.lib().tb_device_fault_flag() == 0
 
 
@@ -116,3 +118,51 @@ def test_the_integer_kernel_stays_selectable(torch, tb, m, n, k, g, pair):
     for y in (streamed, integer):
         assert bool(((y.double() - want).abs() <= d + 1e-30).all())
     assert tb.lib().tb_device_fault_flag() == 0
+
+
+@pytest.mark.parametrize("m,k", [(5, 256), (8, 4608)])
+def test_rows_at_both_ends_of_fp32(torch, tb, m, k):
+    """Zeros, numbers of 1e-35 and 1e33 beside ordinary rows, a denormal."""
+    n, g = 96, 32
+    p, s, w = int4(torch, n, k, g, 5)
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator("cuda").manual_seed(6))
+    x[0] = 0
+    x[1] *= 1e-35
+    x[2] *= 1e33
+    x[3] = 0
+    x[3, k - 50] = 2.5e-39
+    got, want = tb.w4a32_grouped_linear(x, p, s, None, g), x.double() @ w.T
+    bound = (4.4 + k / 32 + 10) * 2.0 ** -24 * (x.double().abs() @ w.abs().T)
+    assert not got[0].any()
+    for i in (1, 2, 4, m - 1):
+        # a piece below the smallest normal number may come out as zero: k of them, 2^-126 each, times codes of up to 8 and a scale
+        assert bool(((got[i].double() - want[i]).abs() <= bound[i] + k * 2.0 ** -126 * 8 * float(s.max())).all()), i
+    assert float((got[3].double() - want[3]).abs().max()) < 2e-39   # denormal sums may come out as zeros
+
+
+@pytest.mark.parametrize("rows", [2, 3, 5, 8])
+@pytest.mark.parametrize("hidden,heads,kv,dim,inter", [(896, 14, 7, 64, 640), (4608, 72, 36, 64, 256)])
+def test_the_norm_in_front_of_few_rows(torch, tb, rows, hidden, heads, kv, dim, inter):
+    """A decoder of one layer at position 0, where attention gives every head its key head's value, against float64.  The pre-pass takes the norm
+    of a row in one block of the grid and, beyond 4096, in several.  1e-5: the layers' fp32 sums of random terms, a few 1e-7 each."""
+    def norm(i):
+        return torch.randn(hidden, device="cuda", generator=torch.Generator("cuda").manual_seed(i)) * 0.1 + 1
+    vocab, q = 300, heads * dim
+    qkv, o = int4(torch, q + 2 * kv * dim, hidden, 32, 1), int4(torch, hidden, q, 32, 2)
+    gate, up, down, head = int4(torch, inter, hidden, 32, 3), int4(torch, inter, hidden, 32, 4), int4(torch, hidden, inter, 32, 5), int4(torch, vocab, hidden, 32, 6)
+    embed = torch.randn(vocab, hidden, device="cuda", generator=torch.Generator("cuda").manual_seed(7))
+    n1, n2, n3 = norm(8), norm(9), norm(10)
+    dec = tb.B200QwenDecoder(embed, [[n1, *qkv[:2], *o[:2], n2, *gate[:2], *up[:2], *down[:2], None]], n3, *head[:2], 1, hidden, inter, heads, kv, dim, 32,
+                             1e-6, 16, 10000.0, max_batch=8)
+    ids = [(37 * i + 5) % vocab for i in range(rows)]
+    got = torch.as_tensor(dec.step_batch(ids, [0] * rows)).cuda().double()
+
+    def rms(x, w):
+        return x / (x.square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double()
+    x = embed[ids].double()
+    v = (rms(x, n1) @ qkv[2].T)[:, q + kv * dim:].view(rows, kv, 1, dim).expand(rows, kv, heads // kv, dim).reshape(rows, q)
+    x = x + v @ o[2].T
+    h = rms(x, n2)
+    x = x + (torch.nn.functional.silu(h @ gate[2].T) * (h @ up[2].T)) @ down[2].T
+    want = rms(x, n3) @ head[2].T
+    assert float((got - want).norm() / want.norm()) < 1e-5

@@ -458,14 +458,15 @@ def test_tcgen05_batched_product_matches_oracle(torch, tb, oracle, n, k, g, m, b
     (520, 7168, 128, 2, False, True),      # 128-element groups, pair
     (96, 8192, 32, 2, True, True),         # fewer rounds than CTAs
     (4096, 4096, 32, 3, True, False),      # three and four rows of a narrow matrix: the CUDA-core kernel
-    (6144, 4096, 32, 4, False, False),
+    (3072, 4096, 32, 4, False, False),
+    (6144, 4096, 32, 4, False, False),     # past its largest output: the streaming tensor-core kernel
 ])
 def test_two_rows_take_the_persistent_kernel_and_match_oracle(torch, tb, oracle, n, k, g, m, bias, pair):
     """Two activation rows take a variant of the persistent streaming kernel of the M = 1 path: a lane keeps
     the digits of its block of K for both rows and multiplies each weight word with both (one pass over the
     weights).  Against the oracle, against the kernel that runs with the streaming kernel switched off, and
-    against the float64 bound of the single-row kernel.  Three and four rows of a narrow matrix run on the
-    CUDA-core kernel (same checks; the switch changes nothing for them)."""
+    against the float64 bound of the single-row kernel.  Three and four rows run on the CUDA-core or the
+    streaming tensor-core kernel (same checks; the switch changes nothing for them)."""
     L = tb.lib()
     rng = np.random.default_rng(n + 7 * k + m)
     p, s = _quantized(torch, tb, n, k, g, n + k + m, std=0.05)
