@@ -115,7 +115,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 // EPI: 0 = plain (+bias, +resid), 1 = SwiGLU of two matrices sharing x.
 // M activation rows, R weight rows per warp, WARPS warps per CTA,
 // XMODE: 0 = fp32 products, 1 = integer products (see above).
-template <int M, int R, int WARPS, int EPI, bool NORM, int XMODE>
+// ONCE: one row that is staged in one go, a thread taking eight elements of it, from the loads to the digits, so that x is read
+// once, and four threads share a block.  (A thread per block reads it twice, 28 threads of 256 busy at K = 896, in a chain of some 400
+// instructions.)  A form of its own: the registers of both stagings in one kernel cost a CTA per SM (4864 x 896 3.4 -> 4.1 us, apart 3.1).
+template <int M, int R, int WARPS, int EPI, bool NORM, int XMODE, bool ONCE>
 __global__ void __launch_bounds__(WARPS * 32) w4_gemv_kernel(const GemvParams p) {
   constexpr int NW = (EPI == 1) ? 2 : 1;
   constexpr int XV = XMODE == 1 ? 7 : 8;  // 16-byte vectors of staged x per block
@@ -158,19 +161,16 @@ __global__ void __launch_bounds__(WARPS * 32) w4_gemv_kernel(const GemvParams p)
   // The weights do not depend on the previous kernel: start streaming them
   // before waiting for it (programmatic dependent launch).
   load_tile(0, wv, sc);
-  // One row that is staged in one go: a thread takes eight elements of it, from the loads to the digits, so that x is read once, and
-  // four threads share a block.  (A thread per block read it twice, 28 threads of 256 busy at K = 896, in a chain of some 400
-  // instructions: 775 against 702 us a token of the 0.5B widths, two such kernels a layer with the norm and one without.)  The norm's weights do not depend on the kernel in front either.
-  const bool once = XMODE == 1 && M == 1 && p.kc >= p.k && p.k <= WARPS * 32 * 8;
+  // The norm's weights do not depend on the kernel in front either.
   const int k8 = threadIdx.x * 8;
   float xv[8], nv[8];
-  if (once && NORM && k8 < p.k) {
+  if (ONCE && NORM && k8 < p.k) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(p.norm_w + k8)), b = __ldg(reinterpret_cast<const float4*>(p.norm_w + k8) + 1);
     nv[0] = a.x; nv[1] = a.y; nv[2] = a.z; nv[3] = a.w; nv[4] = b.x; nv[5] = b.y; nv[6] = b.z; nv[7] = b.w;
   }
   pdl_wait();
   pdl_launch_dependents();
-  if (once) {
+  if (ONCE) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     if (k8 < p.k) {
       a = *reinterpret_cast<const float4*>(p.x + k8);
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(WARPS * 32) w4_gemv_kernel(const GemvParams p)
 #pragma unroll
     for (int m = 0; m < M; ++m) {
       float ss = 0.f;
-      if (once) {
+      if (ONCE) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) ss = fmaf(xv[i], xv[i], ss);
       } else {
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(WARPS * 32) w4_gemv_kernel(const GemvParams p)
             xs4[m * kc4 + blk * 8 + (j ^ (blk & 7))] = v;
           }
         }
-      } else if (once) {
+      } else if (ONCE) {
         if (NORM && k8 < p.k) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) xv[i] = (xv[i] * inv_rms[0]) * nv[i];
@@ -406,9 +406,9 @@ int g_xmode = 1;
 int g_mma_enabled = 1;
 int g_force_r = 0, g_force_warps = 0;
 
-template <int M, int R, int WARPS, int EPI, bool NORM, int XMODE>
-tb_status launch_cfg(const GemvParams& p, bool pdl, cudaStream_t stream) {
-  auto kern = w4_gemv_kernel<M, R, WARPS, EPI, NORM, XMODE>;
+template <int M, int R, int WARPS, int EPI, bool NORM, int XMODE, bool ONCE>
+tb_status launch_form(const GemvParams& p, bool pdl, cudaStream_t stream) {
+  auto kern = w4_gemv_kernel<M, R, WARPS, EPI, NORM, XMODE, ONCE>;
   const size_t smem = XMODE == 1 ? (size_t)M * 7 * (p.kc >> 5) * sizeof(uint4) : (size_t)M * p.kc * sizeof(float);
   static thread_local size_t configured[64] = {0};
   int dev = 0;
@@ -431,6 +431,19 @@ tb_status launch_cfg(const GemvParams& p, bool pdl, cudaStream_t stream) {
   cfg.numAttrs = pdl ? 1 : 0;
   TB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
   return TB_OK;
+}
+
+// One row in one go where a CTA has the threads for it, unless the matrix is narrow and long: then CTAs come by the dozen per SM, one
+// staging lies under its neighbours' streaming, and the general form issues less.  General / in one go, us a call over weights past L2:
+// single matrices 2304 x 768 3.1 / 2.5, 16000 x 1024 6.8 / 5.6, 128256 x 2016 50.8 / 48.1, but 24000 x 512 6.6 / 6.9, 151936 x 896 33.0 / 34.2;
+// pairs 4864 x 896 4.7 / 4.6, 128256 x 2016 102.7 / 94.2, but 16000 x 512 8.2 / 8.8, 151936 x 896 61.2 / 65.3.
+template <int M, int R, int WARPS, int EPI, bool NORM, int XMODE>
+tb_status launch_cfg(const GemvParams& p, bool pdl, cudaStream_t stream) {
+  if constexpr (M == 1 && XMODE == 1) {
+    const bool many = p.k <= 1024 && (EPI == 1 ? (int64_t)p.n >= (int64_t)sm_count() * 96 : R == 4);
+    if (p.kc >= p.k && p.k <= WARPS * 32 * 8 && !many) return launch_form<M, R, WARPS, EPI, NORM, XMODE, true>(p, pdl, stream);
+  }
+  return launch_form<M, R, WARPS, EPI, NORM, XMODE, false>(p, pdl, stream);
 }
 
 template <int M, int EPI, bool NORM, int XMODE>
