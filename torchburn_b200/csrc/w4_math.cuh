@@ -122,20 +122,17 @@ __device__ __forceinline__ void quantize_part_int(const float (&v)[NE], float am
       }
 }
 
-// The larger of two numbers, NaN if either is (fmaxf would drop it, and with it what the caller multiplies by).
-__device__ __forceinline__ float max_nan(float a, float b) {
-  float m;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
-  return m;
-}
+// The larger of two magnitudes, NaN if either is (fmaxf would drop it, and with it what the caller multiplies by).  On their bits, which
+// sort like the numbers, Inf and NaN above them: max.NaN.f32 in its place cost 6% of a product of one row (64000 x 1280 24.4 / 23.0 us).
+__device__ __forceinline__ float max_nan(float a, float b) { return __uint_as_float(max(__float_as_uint(a), __float_as_uint(b))); }
 
 // The largest magnitude; NaN if one of them is.
 template <int NE>
 __device__ __forceinline__ float abs_max(const float (&v)[NE]) {
-  float amax = 0.f;
+  uint32_t amax = 0;
 #pragma unroll
-  for (int i = 0; i < NE; ++i) amax = max_nan(amax, fabsf(v[i]));
-  return amax;
+  for (int i = 0; i < NE; ++i) amax = max(amax, __float_as_uint(v[i]) & 0x7FFFFFFFu);
+  return __uint_as_float(amax);
 }
 
 }  // namespace tb
