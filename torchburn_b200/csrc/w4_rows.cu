@@ -229,6 +229,9 @@ __global__ void __launch_bounds__(kThreads, 1) w4_rows_kernel(const __grid_const
     };
     for (; it < first; ++it, next()) weights(pass, kc, it);
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Behind the own wait, so that completion stays transitive along a chain.  The attention of a step is launched early behind its QKV
+    // product: two sequences of width 1024 347 -> 335 us a step, four of width 2048 543 -> 526.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (int i = 0, c = kfirst; i < first; ++i) {
       images(c, i);
       if (++c == nk) c = 0;
