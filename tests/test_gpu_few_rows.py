@@ -1,9 +1,10 @@
-"""Products of 2 to 8 activation rows (w4_rows_kernel).
+"""Products of 2 to 8 activation rows (w4_rows_kernel, and the integer kernel where that takes less).
 
 Bound of the products, per output, with A = sum |x| |w|: activations, codes and their products are exact; a 32-element block's
 sum is six accumulating instructions, of which the two with the large pieces may truncate at 2^-23 of at most A and the
 others at 2^-8 of that; adding the K / 32 blocks, the eight sums of the warps and the bias takes one fp32 rounding each
-(2^-24 A): below (2 * 2 * 1.1 + K / 32 + 10) * 2^-24 * A."""
+(2^-24 A): below (2 * 2 * 1.1 + K / 32 + 10) * 2^-24 * A.  The integer kernel rounds every element to a multiple of 2^-22 of its block's
+maximum, half of that at most: 2^-23 * sum over blocks of max |x| sum |w| more."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -35,14 +36,19 @@ def int4(torch, n, k, g, seed):
     return (q[:, 0::2] | (q[:, 1::2] << 4)).contiguous(), s.contiguous(), (c.double() * s.double()[..., None]).reshape(n, k)
 
 
+INTEGER = [(5, 16 * 148, 256, 32, 0), (5, 14 * 16 * 148 + 5, 256, 32, 0), (8, 33000, 512, 64, 0), (5, 96, 20480, 64, 0), (3, 700, 8192, 64, 0), (8, 8960, 1536, 32, 1),
+           (2, 18944, 896, 32, 1), (5, 18944, 1536, 32, 0), (6, 13824, 1024, 128, 1), (4, 24576, 1024, 32, 1)]
+
+
 @pytest.mark.parametrize("m,n,k,g,pair", [
     (2, 1, 32, 32, 0), (8, 7, 32, 32, 1), (3, 17, 96, 32, 0),             # one block of K, one ragged tile
-    (5, 16 * 148, 256, 32, 0), (8, 16 * 148 + 1, 288, 32, 0),             # a tile per CTA, one more; a stage and an eighth
+    (8, 16 * 148 + 1, 288, 32, 0), (5, 16 * 148, 288, 32, 0),             # a tile per CTA, one more; a stage and an eighth
     (4, 8 * 148 * 2 + 3, 512, 64, 1), (8, 14330, 896, 64, 0),             # unaligned rows of scales, copied in eights
     (7, 4864, 896, 128, 1), (8, 1000, 1920, 128, 0),                      # and in fours; K that is no whole stage
-    (5, 14 * 16 * 148 + 5, 256, 32, 0), (8, 33000, 512, 64, 0),           # more tiles than a pass holds
-    (6, 6144, 4096, 32, 0), (8, 4096, 14336, 32, 0), (8, 14336, 4096, 32, 1), (5, 96, 20480, 64, 0),
-])
+    (5, 14 * 16 * 148 + 5, 288, 32, 0), (8, 33000, 768, 64, 0),           # more tiles than a pass holds, and as many
+    (6, 6144, 4096, 32, 0), (8, 4096, 14336, 32, 0), (8, 14336, 4096, 32, 1),
+    (8, 8960, 1504, 32, 1), (5, 2400, 8192, 32, 0), (7, 5000, 512, 32, 0), (2, 8288, 1024, 32, 1),   # beside the integer kernel's sizes
+    *INTEGER])
 def test_products_of_few_rows_match_float64(torch, tb, m, n, k, g, pair):
     p, s, w = int4(torch, n, k, g, m + n + k)
     p2, s2, w2 = int4(torch, n, k, g, m + n + k + 1)
@@ -60,21 +66,33 @@ def test_products_of_few_rows_match_float64(torch, tb, m, n, k, g, pair):
                                              m, n, k, g, st) == 0, tb.last_error()
         return y
     y = run()
-    gate, bound = x.double() @ w.T + b, (x.double().abs() @ w.abs().T + b.abs()) * tol
+    try:
+        tb.lib().tb_set_gemv_tuning(3, 0, 0)
+        integer = torch.equal(run(), y)
+    finally:
+        tb.lib().tb_set_gemv_tuning(1, 0, 0)
+    if n > 17:   # (one narrow case is the CUDA-core kernel's in either mode, too few outputs differ in others)
+        assert integer == ((m, n, k, g, pair) in INTEGER)
+    top = x.double().abs().reshape(m, k // 32, 32).amax(-1, keepdim=True).expand(m, k // 32, 32).reshape(m, k)
+
+    def more(w):
+        return 2.0 ** -23 * (top @ w.abs().T) if integer else 0.0
+    gate, bound = x.double() @ w.T + b, (x.double().abs() @ w.abs().T + b.abs()) * tol + more(w)
     if pair:
         up, sig = x.double() @ w2.T, torch.sigmoid(gate)
         # silu' <= 1.1, |silu(g)| <= |g|; four roundings of the epilogue
-        bound = 1.1 * bound * up.abs() + gate.abs() * (x.double().abs() @ w2.abs().T) * tol + 4 * 2.0 ** -23 * (gate * sig * up).abs() + bound * 1e-6
+        bound = 1.1 * bound * up.abs() + gate.abs() * ((x.double().abs() @ w2.abs().T) * tol + more(w2)) + 4 * 2.0 ** -23 * (gate * sig * up).abs() + bound * 1e-6
         gate = gate * sig * up
     assert bool(((y.double() - gate).abs() <= bound + 1e-30).all()), float(((y.double() - gate).abs() / bound).max())
     assert torch.equal(run(), y)   # equal calls give equal bits
     assert tb.lib().tb_device_fault_flag() == 0
 
 
-def test_few_rows_keep_infinities_to_their_row(torch, tb):
+@pytest.mark.parametrize("k", [512, 896])   # the integer kernel, the streaming one
+def test_few_rows_keep_infinities_to_their_row(torch, tb, k):
     """A row with an infinity or a NaN leaves the other rows as they are."""
-    p, s, _ = int4(torch, 300, 512, 32, 1)
-    x = torch.randn(6, 512, device="cuda")
+    p, s, _ = int4(torch, 300, k, 32, 1)
+    x = torch.randn(6, k, device="cuda")
     want = tb.w4a32_grouped_linear(x, p, s, None, 32)
     x[2, 7], x[4, 100] = float("inf"), float("nan")
     got = tb.w4a32_grouped_linear(x, p, s, None, 32)
@@ -84,7 +102,7 @@ def test_few_rows_keep_infinities_to_their_row(torch, tb):
 
 
 @pytest.mark.parametrize("pair", [0, 1])
-@pytest.mark.parametrize("m,n,k,g", [(2, 700, 896, 32), (3, 6000, 1024, 64), (4, 4097, 512, 128), (5, 96, 8192, 32), (8, 5003, 4096, 32), (8, 600, 14336, 32), (6, 9600, 256, 32)])
+@pytest.mark.parametrize("m,n,k,g", [(2, 700, 896, 32), (3, 6000, 1024, 64), (4, 4097, 640, 128), (5, 96, 4096, 32), (8, 5003, 4096, 32), (8, 600, 7168, 32), (6, 9600, 288, 32)])
 def test_the_integer_kernel_stays_selectable(torch, tb, m, n, k, g, pair):
     """tb_set_gemv_tuning(3, ...) takes these products to the integer kernel: other bits than the default's, within the bound of
     its arithmetic (the streaming kernel's for the sums, and half a step of 2^-22 of a block's maximum for each of its elements)."""
@@ -120,7 +138,7 @@ def test_the_integer_kernel_stays_selectable(torch, tb, m, n, k, g, pair):
     assert tb.lib().tb_device_fault_flag() == 0
 
 
-@pytest.mark.parametrize("m,k", [(5, 256), (8, 4608)])
+@pytest.mark.parametrize("m,k", [(5, 288), (8, 4608)])
 def test_rows_at_both_ends_of_fp32(torch, tb, m, k):
     """Zeros, numbers of 1e-35 and 1e33 beside ordinary rows, a denormal."""
     n, g = 96, 32

@@ -1,6 +1,6 @@
 // Grouped INT4 W4A32 products for several activation rows (up to 64 per pass) on the
-// tensor cores, with exact integer arithmetic: 9 to 16 rows of small matrices, and whatever the
-// streaming kernel for 2 to 8 rows (w4_rows.cu) and the tcgen05 kernel do not take.
+// tensor cores, with exact integer arithmetic: 9 to 16 rows of small matrices, the sizes at which it beats the
+// streaming kernel for 2 to 8 rows (w4_rows.cu), and whatever that one and the tcgen05 kernel do not take.
 //
 // Replaces gemm_w4a32_grouped (src/quantization/gemv.rs:1690-1725: M independent GEMVs) and
 // fused_swiglu_mlp_batched (src/quantization/fused_ops.rs:1267-1319) for M > 1.
@@ -374,7 +374,7 @@ template <int MT, int EPI, int KC>
 tb_status launch_rows_mt(const MmaParams& p, cudaStream_t stream) {
   // rows per CTA so that the grid is about one CTA per SM or more; narrow matrices split K over warps
   const int per_sm = p.n / sm_count();
-  // Up to 16 activation rows (MT = 2), graph-timed on the Llama-3-8B shapes at 16 rows: CTAs of 64 weight
+  // Up to 16 activation rows (MT <= 2), graph-timed on the Llama-3-8B shapes at 16 rows: CTAs of 64 weight
   // rows with 8 warps (4 side by side, K of a stage split in two) against CTAs of 32 rows with 4 warps: gate/up
   // pair 61.9 us against 71.8; the K = 14336 projection 44.0 against 49.4.  Only where 64-row CTAs still cover every
   // SM: the narrow projections and the shards of a tensor-parallel rank stay with 32-row CTAs of 8 warps.
@@ -391,6 +391,7 @@ tb_status launch_rows_mt(const MmaParams& p, cudaStream_t stream) {
 
 template <int EPI>
 tb_status launch_rows_epi(const MmaParams& p, cudaStream_t stream) {
+  if (p.mt_total <= 1) return launch_rows_mt<1, EPI, 8>(p, stream);
   if (p.mt_total <= 2) return launch_rows_mt<2, EPI, 8>(p, stream);
   if (p.mt_total <= 4) return launch_rows_mt<4, EPI, 4>(p, stream);
   return launch_rows_mt<8, EPI, 4>(p, stream);

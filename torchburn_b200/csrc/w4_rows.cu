@@ -405,6 +405,24 @@ Plan choose_plan(int64_t n, int g, bool pair) {
   return p;
 }
 
+// Where the integer kernel (w4_mma.cu) takes less.  Tiles: of the CTA with most of them, and per pass.  Measured with 32-element groups
+// at 8 rows over 28 x 13 sizes (2 to 8 rows cost the same), us, integer / this kernel:
+//   one tile a CTA and a long K, which it splits over four CTAs: 1024 x 8192 13.2 / 15.2, 2048 x 11008 17.7 / 19.0, 1024 x 14336 16.3 / 22.6;
+//   next to no K, this kernel's start alone: 256 x 512 4.0 / 4.8, 2560 x 512 4.8 / 5.1, but 8960 x 512 6.7 / 6.4;
+//   eight tiles a pass, the first count with stages of 256: pairs 8960 x 1536 13.1 / 15.1, 18944 x 4096 39.5 / 48.3, 9472 x 8960 48.8 / 51.1, single
+//   18944 x 1536 13.8 / 14.4 (from K = 2048 on even); seven tiles, 14336 x 4096: 28.3 / 21.6;
+//   many tiles of short rows, in pairs: 13824 x 1024 13.9 / 14.5, 24576 x 2048 31.6 / 32.9 (x 3072 44.1 / 44.4).
+// Its reads want rows of 128 bytes: at K = 896 it is 1.2 to 1.5 times as slow as this kernel, but for 18944 pairs (16.1 / 18.2).
+bool integer_takes_less(const GemvArgs& a) {
+  const bool pair = a.w2 != nullptr, whole = a.k % 256 == 0;
+  const Plan p = choose_plan(a.n, a.g, pair);
+  const int most = (p.tiles + sm_count() - 1) / sm_count();
+  const bool eight = p.pass_tiles == kWarpTiles + 1, one_pass = most <= kMaxTiles;
+  if (pair) return eight ? whole || !one_pass : whole && a.k <= (one_pass ? (most >= 12 ? 1024 : 0) : 2048);
+  if (most == 1 && a.k >= 8192) return true;
+  return whole && (a.k <= 512 ? most <= 2 || most >= 6 : eight && a.k >= 1024 && a.k < 2048);
+}
+
 }  // namespace
 
 void set_rows_enabled(int enabled) { g_rows_enabled = enabled; }
@@ -419,7 +437,8 @@ size_t w4_rows_scratch_bytes(int64_t k) { return (size_t)padded_blocks(k) * kIma
 
 bool w4_rows_supported(const GemvArgs& a) {
   return g_rows_enabled && a.m >= 2 && a.m <= kMaxRowsM && a.k % 32 == 0 && tma_encoder() &&
-         !((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.w2) | reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.norm_w)) & 15);
+         !((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.w2) | reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.norm_w)) & 15) &&
+         !integer_takes_less(a);
 }
 
 tb_status launch_w4_rows(const GemvArgs& a, void* scratch, cudaStream_t stream) {
