@@ -314,12 +314,11 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       uint32_t c = 0, u = 0;
       bool ok = true;
       const uint32_t w_at = smem_u32(smem + S::kOffNib), s_at = smem_u32(smem + S::kOffScale);
-      auto weights = [&](uint32_t wu, int t, int i) {   // unit wu of the CTA: unit i of tile t
+      auto weights = [&](uint32_t wu, int n0, int i) {   // unit wu of the CTA: unit i of the tile at weight row n0
         const uint32_t ws = wu % S::kUnits, ss = wu % S::kScales;
         if (wu >= S::kUnits) ok = mbar_wait_fast(&empty_w[ws], (wu / S::kUnits - 1u) & 1u, &s_abort);
         if (G == 32 && ok && wu >= S::kScales) ok = mbar_wait_fast(&empty_s[ss], (wu / S::kScales - 1u) & 1u, &s_abort);
         if (!ok) return;
-        const int n0 = t / p.mtiles * (p.pair ? kTileN : kTileN * NW);
         // the scales arrive with the codes: who has seen sums of the unit has seen its scales
         mbar_expect_tx(&full_w[ws], NW * (kUnitBytes + (G == 32 ? kUnitScaleBytes : 0)));
 #pragma unroll
@@ -336,22 +335,32 @@ __global__ void __launch_bounds__(Shape<MP, NW, G>::kThreads, 1) w4_tc5_kernel(c
       static_assert(S::kScales >= S::kUnits, "scales of the first units");
       uint32_t ahead = 0;
       const int tf = t0 + g0 / nunits * ts, i0 = g0 % nunits;   // where the CTA begins
-      for (int t = tf, i = i0; ahead < (uint32_t)my_units && ahead < S::kUnits; ++ahead) {
-        weights(ahead, t, i);
-        if (++i == nunits) { i = 0; t += ts; }
+      // What a tile decides is computed at its start: two divisions per unit in this thread were what bounded one weight tile of up to 64 rows
+      // (17 x 4096 x 14336 30.5 -> 26.4 us, 24 x 896 x 151936 57.4 -> 48.9, 301 x 4864 x 896 23.5 -> 20.6).
+      const int row_step = p.pair ? kTileN : kTileN * NW;
+      for (int t = tf, i = i0, n0 = tf / p.mtiles * row_step; ahead < (uint32_t)my_units && ahead < S::kUnits; ++ahead) {
+        weights(ahead, n0, i);
+        if (++i == nunits) { i = 0; t += ts; n0 = t / p.mtiles * row_step; }
       }
       asm volatile("griddepcontrol.wait;" ::: "memory");
+      int n0 = tf / p.mtiles * row_step;
+      const unsigned char* src = p.xq + ((size_t)(tf % p.mtiles) * nunits + i0) * (2 * S::kBBytes);
       for (int t = tf, i = i0; u < (uint32_t)my_units && ok; ++u) {
-        if (u >= ahead) weights(u, t, i);
+        if (u >= ahead) weights(u, n0, i);
         if (!ok) break;
-        const unsigned char* src = p.xq + ((size_t)(t % p.mtiles) * nunits + i) * (2 * S::kBBytes);
         for (int h = 0; h < 2; ++h, ++c) {
           if (c >= SB) ok = mbar_wait_fast(&done[(c - SB) % kRing], ((c - SB) / kRing) & 1u, &s_abort);
           if (!ok) break;
           mbar_expect_tx(&full_b[c % kRing], S::kBBytes);
-          bulk_g2s(smem + (size_t)(c % SB) * S::kBBytes, src + h * S::kBBytes, S::kBBytes, &full_b[c % kRing]);
+          bulk_g2s(smem + (size_t)(c % SB) * S::kBBytes, src, S::kBBytes, &full_b[c % kRing]);
+          src += S::kBBytes;
         }
-        if (++i == nunits) { i = 0; t += ts; }
+        if (++i == nunits) {
+          i = 0;
+          t += ts;
+          n0 = t / p.mtiles * row_step;
+          src = p.xq + (size_t)(t % p.mtiles) * nunits * (2 * S::kBBytes);
+        }
       }
       // copies in flight must have landed before the CTA gives its shared memory back (all have, unless a wait was given up)
       if (!ok) {
