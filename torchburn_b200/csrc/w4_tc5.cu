@@ -788,27 +788,30 @@ const Variant kVariants[] = {variant<16, 1>(), variant<32, 1>(), variant<48, 1>(
 
 // Whole tiles in turn leave SMs idle when they do not fill the last wave: 112 CTAs of 148 for a gate/up pair of 14336 features or for
 // 4096 features and 333 rows.  A range of units of K for every CTA, which may begin and end inside a tile, leaves none, but
-// the ends cost an exchange through memory: an end 2.2 + 0.022 per accumulator column, and what the last CTA of a tile reads.
-// Measured, whole tiles (or equal parts) / ranges over all SMs: 333 x 14336 -> 4096 153 / 127 us, the pair of 200 rows 4096 -> 14336
-// 180 / 166, of 100 rows 105 / 99, of 16 rows 39.0 / 35.8; but 333 x 4096 -> 6144 53 / 63 and small matrices 11 / 14.
-// The cost of a launch in microseconds, pre-pass included, fitted to 399 plans of 26 calls (every variant, 16 to 333 rows, the
-// projections of the 8B and 0.5B widths; near the best plan rms 3%; the plan it picks is 0.5% from the best on average, 3%
-// at worst): a stage of 64 elements takes what kStage says - the roles' instruction chains, not HBM or the tensor pipe -,
-// a tile's end 0.057 per accumulator column.
+// the ends cost an exchange through memory: an end 1.6 + 0.017 per accumulator column, and what the last CTA of a tile reads.
+// Measured, whole tiles (or equal parts) / ranges over all SMs, groups of 32: 333 x 14336 -> 4096 153 / 128 us, 200 x 4096 -> 14336 94 / 90, the pair of
+// 200 rows 4096 -> 14336 186 / 166, of 100 rows 105 / 97, of 16 rows 35.9 / 33.8; but 333 x 4096 -> 6144 55 / 64, 200 x 4096 -> 4096 32 / 36.
+// The cost of a launch in microseconds, pre-pass included, chosen so that the plan it picks is near the best one of 624 calls (4796 plans
+// of every variant, 16 to 512 rows, 26 matrices of 1024 to 28672 rows, groups of 32 to 128): 0.4% from it on average, 9% at worst; the constants before the
+// copying thread lost its divisions picked plans 1.7% from the best on average and 15% at worst on a part of them.  A stage of 64 elements takes what kStage
+// says - the roles' instruction chains, not HBM or the tensor pipe -, a tile's end 0.051 per accumulator column.
 constexpr int kPadRows = 64;   // padding of the last tile: less than the largest tile
 constexpr int kTickets = 1024;
-constexpr double kStage[2][4] = {{0.300, 0.314, 0.363, 0.393}, {0.49, 0.546, 0.649, 0.660}};   // one or two weight tiles, 16 to 64 rows
+constexpr double kStage[2][4] = {{0.288, 0.281, 0.341, 0.393}, {0.451, 0.479, 0.709, 0.712}};   // one or two weight tiles, 16 to 64 rows
+constexpr double kLarge[2][2][4] = {{{0.90, 0.90, 0.915, 0.911}, {1.104, 1.093, 0.898, 0.894}},   // of that with groups of 64
+                                    {{0.90, 0.893, 0.883, 0.887}, {1.025, 1.059, 0.757, 0.852}}};   // and of 128
 struct Plan { const Variant* v; int mtiles, ntiles, grid, per, more; double cost; };   // per, more: Tc5Params
 double plan_cost(const Plan& p, int64_t k, int g) {
-  const double stage = kStage[p.v->nw - 1][p.v->mp / 16 - 1] * (g > 32 ? 0.95 : 1.0), cols = p.v->mp * p.v->nw;
+  const int nw = p.v->nw - 1, mp = p.v->mp / 16 - 1;
+  const double stage = kStage[nw][mp] * (g > 32 ? kLarge[g / 128][nw][mp] : 1.0), cols = p.v->mp * p.v->nw;
   const int64_t tiles = (int64_t)p.mtiles * p.ntiles, ku = k / kUnit;
-  const double prep = 3.5 + 0.19e-3 * (double)k;
-  if (p.per == 0) return (double)((tiles + p.grid - 1) / p.grid) * ((double)(k / kKC) * stage + 0.057 * cols) + prep;
+  const double prep = 3.3 + 0.12e-3 * (double)k;
+  if (p.per == 0) return (double)((tiles + p.grid - 1) / p.grid) * ((double)(k / kKC) * stage + 0.051 * cols) + prep;
   const int units = p.per + (p.more ? 1 : 0);
   const double share = (double)units / (double)ku;                                                    // of a tile, or tiles, a CTA
   const double ends = share >= 1.0 ? share + 1.0 : (p.more == 0 && ku % units == 0 ? 1.0 : 1.0 + share);   // tiles that a CTA ends or leaves
   const double shared = ends < 2.0 ? ends : 2.0, parts = share >= 1.0 ? 2.0 : (double)p.grid / (double)tiles;
-  return units * (kUnit / kKC) * stage + ends * 0.057 * cols + shared * (2.2 + 0.022 * cols + 0.0026 * cols * parts) + prep;
+  return units * (kUnit / kKC) * stage + ends * 0.051 * cols + shared * (1.64 + 0.0171 * cols + 0.0067 * cols * parts) + prep;
 }
 // At 9 to 16 rows, the choice between this kernel and the integer one: whole tiles or equal parts of K, as they were measured against
 // each other (w4_mma_cost).  A launch of ranges may take less; calls that it would move are left where they are.
