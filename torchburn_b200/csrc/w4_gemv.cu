@@ -262,9 +262,10 @@ __global__ void __launch_bounds__(WARPS * 32) w4_gemv_kernel(const GemvParams p)
             reinterpret_cast<float4*>(p.x_normed_out + k8)[1] = make_float4(xv[4], xv[5], xv[6], xv[7]);
           }
         }
-        float amax = abs_max<8>(xv);
-        amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        constexpr bool kBits = R == 4;
+        float amax = abs_max<8, kBits>(xv);
+        amax = max_nan<kBits>(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = max_nan<kBits>(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         uint32_t dig[6];
         float sx;
         int S, s8hi, s8lo;
