@@ -247,12 +247,12 @@ class _LinearHandle:
 
 def _readable(q, s, b, group_size) -> bool:
     """Whether the kernels can read these weights where they are: whole, of the right types, on the current device."""
-    if not (q.is_cuda and q.ndim == 2 and q.dtype is torch.uint8 and s.dtype is torch.float32 and q.is_contiguous() and s.is_contiguous()):
+    if not (q.is_cuda and q.dtype is torch.uint8 and s.dtype is torch.float32 and q.ndim == 2 and q.is_contiguous() and s.is_contiguous()):
         return False
-    n, index = q.shape[0], q.get_device()
-    return (index == s.get_device() == torch.cuda.current_device() and s.numel() * group_size == n * q.shape[1] * 2
-            and q.data_ptr() % 16 == 0 and s.data_ptr() % 16 == 0
-            and (b is None or (b.dtype is torch.float32 and b.is_contiguous() and b.get_device() == index and b.numel() == n)))
+    index = q.get_device()
+    return (index == s.get_device() == torch._C._cuda_getDevice() and s.numel() * group_size == q.numel() * 2
+            and not (q.data_ptr() | s.data_ptr()) & 15
+            and (b is None or (b.dtype is torch.float32 and b.is_contiguous() and b.get_device() == index and b.numel() == q.shape[0])))
 
 
 def _handle_of(m) -> _LinearHandle:
@@ -293,10 +293,15 @@ def fused_swiglu_mlp(x: torch.Tensor, gate_proj, up_proj, down_proj) -> torch.Te
     for modules carrying qweight/scales/bias/group_size; x (..., hidden) -> (..., hidden_out)."""
     xf, space, dev = _io(x)
     hidden = xf.shape[-1]
-    m = _flattened_rows(xf.shape)
     g, u, d = _handle_of(gate_proj), _handle_of(up_proj), _handle_of(down_proj)
     assert hidden == g.k
-    out = torch.empty(list(xf.shape[:-1]) + [d.n], dtype=torch.float32, device=xf.device)
+    m = _flattened_rows(xf.shape)
+    out = torch.empty((*xf.shape[:-1], d.n), dtype=torch.float32, device=xf.device)
+    if dev.index == torch._C._cuda_getDevice():   # (the guard and the stream object are longer than the look at the weights)
+        stream = torch._C._cuda_getCurrentRawStream(dev.index)
+        _used_on(stream, gate_proj, up_proj, down_proj)
+        check(lib().tb_fused_swiglu_mlp(g.h, u.h, d.h, xf.data_ptr(), m, out.data_ptr(), space, stream))
+        return out
     with torch.cuda.device(dev):
         stream = _stream_ptr(dev)
         _used_on(stream, gate_proj, up_proj, down_proj)
