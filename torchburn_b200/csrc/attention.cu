@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) attn_decode_kernel(const AttnP
 }
 
 int g_chunk_override = 0;
-int g_ctas_per_sm = 0;   // 0 = automatic (2)
+int g_ctas_per_sm = 0;   // 0 = automatic (2, for large batches 3: attn_layout)
 int g_ring_stages = 0;   // 0 = automatic
 
 struct AttnLayout {

@@ -168,8 +168,9 @@ tb_status enqueue_step(tb_decoder* d, int b, bool debug, cudaEvent_t before_lm_h
     d->debug_rows = b;
     return layered_enqueue(d->lay, s, st, &d->launches_per_step);
   }
-  // Narrow models' QKV and output projections too: their kernels (w4_gemv) are short, and so is what they prefetch (0.5B
-  // widths, one sequence behind 1024 positions: 800 us a token without, 775 with; 8B widths, whose kernels are others: 600 against 688).
+  // Narrow models' QKV and output projections too: their kernels are short, and so is what they prefetch.  One sequence behind 1024
+  // positions, eight layers, us a token without / with: width 512 169.6 / 163.5, 768 190.9 / 185.5, 896 225.5 / 219.7, 1024 191.4 / 186.3, 1536 361.0 / 353.0,
+  // 1792 325.3 / 319.0.  2048 (302 / 290) and 2560 (413 / 399) would gain as well, 4096 loses (600 / 688); the line is at the widths of w4_gemv.
   const int pm = d->pdl_mask | (b == 1 && d->tp == 1 && d->H < 2048 ? 5 : 0);
   int launches = 0;
   if (d->fused_step && b == 1 && !debug && before_lm_head == nullptr) {

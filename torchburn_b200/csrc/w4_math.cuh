@@ -1,5 +1,7 @@
-// Integer arithmetic shared by the grouped-INT4 kernels.
+// Arithmetic shared by the grouped-INT4 kernels.
 #pragma once
+#include <cuda_bf16.h>
+
 #include <cstdint>
 
 namespace tb {
@@ -140,6 +142,19 @@ __device__ __forceinline__ float abs_max(const float (&v)[NE]) {
 #pragma unroll
   for (int i = 0; i < NE; ++i) amax = max_nan<kBits>(amax, fabsf(v[i]));
   return amax;
+}
+
+// 8 nibbles -> four bf16 pairs holding the codes (nibble - 8) of elements (0,4) (1,5) (2,6) (3,7): 0x4300 | nibble is the
+// bf16 number 128 + nibble, and 136 is subtracted exactly.  The activation images use the same order of K inside every
+// 8 elements.
+__device__ __forceinline__ void unpack8(uint32_t word, uint32_t* out4) {
+  const uint32_t off = 0x43084308u;   // 136
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t a = ((word >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&off));
+    out4[i] = *reinterpret_cast<const uint32_t*>(&v);
+  }
 }
 
 }  // namespace tb

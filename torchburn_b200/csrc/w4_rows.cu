@@ -36,6 +36,7 @@
 #include "tb_common.cuh"
 #include "tc5.cuh"
 #include "tma_map.cuh"
+#include "w4_math.cuh"
 
 namespace tb {
 
@@ -74,17 +75,6 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// 8 nibbles -> four bf16 pairs holding the codes (nibble - 8) of elements (0,4) (1,5) (2,6) (3,7): 0x4300 | nibble is the bf16
-// number 128 + nibble.  The images use the same order.
-__device__ __forceinline__ void unpack8(uint32_t word, uint32_t (&o)[4]) {
-  const uint32_t off = 0x43084308u;   // 136
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t a = ((word >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
-    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&off));
-    o[i] = *reinterpret_cast<const uint32_t*>(&v);
-  }
 }
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kWarps * 32) : "memory"); }
 // kBytes (16, 8 or 4) to shared memory, of which the first `live` from memory and zeros behind them.

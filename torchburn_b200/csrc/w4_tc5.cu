@@ -42,6 +42,7 @@
 #include "tb_common.cuh"
 #include "tc5.cuh"
 #include "tma_map.cuh"
+#include "w4_math.cuh"
 
 namespace tb {
 
@@ -147,19 +148,6 @@ __device__ __forceinline__ void fma2(float& a0, float& a1, uint32_t x0, uint32_t
       "fma.rn.f32x2 a, x, s, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
       : "+f"(a0), "+f"(a1)
       : "r"(x0), "r"(x1), "f"(s));
-}
-
-// 8 nibbles -> four bf16 pairs holding the codes (nibble - 8) of elements (0,4) (1,5) (2,6) (3,7): 0x4300 | nibble is the
-// bf16 number 128 + nibble, and 136 is subtracted exactly.  The activation images use the same order of K inside every
-// 8 elements.
-__device__ __forceinline__ void unpack8(uint32_t word, uint32_t* out4) {
-  const uint32_t off = 0x43084308u;   // 136
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t a = ((word >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
-    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&off));
-    out4[i] = *reinterpret_cast<const uint32_t*>(&v);
-  }
 }
 
 constexpr int floor_pow2(int v) { return v >= 4 ? 4 : (v >= 2 ? 2 : 1); }
@@ -813,8 +801,9 @@ double plan_cost(const Plan& p, int64_t k, int g) {
   const double shared = ends < 2.0 ? ends : 2.0, parts = share >= 1.0 ? 2.0 : (double)p.grid / (double)tiles;
   return units * (kUnit / kKC) * stage + ends * 0.051 * cols + shared * (1.64 + 0.0171 * cols + 0.0067 * cols * parts) + prep;
 }
-// At 9 to 16 rows, the choice between this kernel and the integer one: whole tiles or equal parts of K, as they were measured against
-// each other (w4_mma_cost).  A launch of ranges may take less; calls that it would move are left where they are.
+// At 9 to 16 rows, the choice between this kernel and the integer one: what this kernel cost with whole tiles or equal parts of K, eight
+// unpacking warps and its pre-pass in front, as the two were measured against each other (w4_mma_cost).  It costs less now, so that calls near the
+// line are left where they were and not where they take least: the pair of 16 rows 4096 -> 1792 takes 23.8 us on the integer kernel, of 17 rows 16.3 here.
 double few_rows_cost(int m, int64_t n, int64_t k, int g, bool pair) {
   double best = 1e30;
   for (int nw = pair ? 2 : 1; nw <= 2; ++nw)
