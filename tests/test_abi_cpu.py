@@ -85,6 +85,7 @@ def test_argument_errors_without_gpu(tb):
     assert L.tb_gemv_w4a32_grouped(buf, wb, buf, None, buf, 4, 80, 32, None) == 2  # k % g != 0
     h = C.c_void_p()
     assert L.tb_linear_create(C.byref(h), wb, buf, None, 0, 64, 32, 0) == 2
+    assert L.tb_linear_view(C.byref(h), wb, buf, None, 4, 80, 32) == 2 and L.tb_linear_view(C.byref(h), None, buf, None, 4, 64, 32) == 1
     assert L.tb_decoder_create(C.byref(h), None, None, None, None, None, None, 0) == 1
     assert L.tb_decoder_kv_len(None) == 0
     assert L.tb_decoder_is_device_lost(None) == 0

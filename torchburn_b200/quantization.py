@@ -299,13 +299,13 @@ def fused_swiglu_mlp(x: torch.Tensor, gate_proj, up_proj, down_proj) -> torch.Te
     out = torch.empty((*xf.shape[:-1], d.n), dtype=torch.float32, device=xf.device)
     if dev.index == torch._C._cuda_getDevice():   # (the guard and the stream object are longer than the look at the weights)
         stream = torch._C._cuda_getCurrentRawStream(dev.index)
-        _used_on(stream, gate_proj, up_proj, down_proj)
         check(lib().tb_fused_swiglu_mlp(g.h, u.h, d.h, xf.data_ptr(), m, out.data_ptr(), space, stream))
+        _used_on(stream, gate_proj, up_proj, down_proj)
         return out
     with torch.cuda.device(dev):
         stream = _stream_ptr(dev)
-        _used_on(stream, gate_proj, up_proj, down_proj)
         check(lib().tb_fused_swiglu_mlp(g.h, u.h, d.h, xf.data_ptr(), m, out.data_ptr(), space, stream))
+        _used_on(stream, gate_proj, up_proj, down_proj)
     return out
 
 
